@@ -31,7 +31,6 @@ static int check_ws(void *ws, size_t have, size_t need, const char *who) {
 }
 
 #define HB_PLAN_ARGS(p) (p)->g->d, prec, nmaps, (p)->lmax, (p)->mmax
-static const float4 *ck_of(const hb_plan *p, int prec) { return prec == 32 ? p->ck : nullptr; }
 
 static int map2alm_impl(const hb_plan *p, int nmaps, const void *maps, const double *w, void *alm, void *ws,
                         size_t wsb, int flags, cudaStream_t st, int prec, const char *who) {
@@ -41,7 +40,7 @@ static int map2alm_impl(const hb_plan *p, int nmaps, const void *maps, const dou
     if ((rc = check_ws(ws, wsb, fm_bytes(p, prec, nmaps), who))) return rc;
     const GeomDev &d = p->g->d;
     if ((rc = launch_ring_analysis(d, prec, nmaps, maps, d.npix, w, ws, p->mmax, flags, false, false, st))) return rc;
-    return launch_leg_analysis(HB_PLAN_ARGS(p), ws, alm, st, ck_of(p, prec), p->blk_ofs);
+    return launch_leg_analysis(p, prec, nmaps, ws, alm, st);
 }
 
 static int alm2map_impl(const hb_plan *p, int nmaps, const void *alm, void *maps, void *ws, size_t wsb, int flags,
@@ -51,7 +50,7 @@ static int alm2map_impl(const hb_plan *p, int nmaps, const void *alm, void *maps
     if (!maps || !alm) return fail(HB_ERR_INVALID, std::string(who) + ": null data pointer");
     if ((rc = check_ws(ws, wsb, fm_bytes(p, prec, nmaps), who))) return rc;
     const GeomDev &d = p->g->d;
-    if ((rc = launch_leg_synthesis(HB_PLAN_ARGS(p), alm, ws, st, ck_of(p, prec), p->blk_ofs))) return rc;
+    if ((rc = launch_leg_synthesis(p, prec, nmaps, alm, ws, st))) return rc;
     return launch_ring_synthesis(d, prec, nmaps, ws, p->mmax, maps, d.npix, nullptr, false, true, flags, st);
 }
 
@@ -66,7 +65,7 @@ static int alm2map_adj_impl(const hb_plan *p, int nmaps, const void *maps, void 
     if ((rc = launch_ring_analysis(d, prec, nmaps, maps, d.npix, nullptr, ws, p->mmax, flags & ~HB_F_NOFOLD, true,
                                    true, st)))
         return rc;
-    return launch_leg_analysis(HB_PLAN_ARGS(p), ws, alm, st, ck_of(p, prec), p->blk_ofs);
+    return launch_leg_analysis(p, prec, nmaps, ws, alm, st);
 }
 
 // transpose of map2alm: Legendre synthesis, then ring synthesis with c_m = 1 and pixel weights
@@ -78,7 +77,7 @@ static int map2alm_adj_impl(const hb_plan *p, int nmaps, const void *alm, const 
     if (flags & HB_F_NOFOLD) return fail(HB_ERR_UNSUPPORTED, std::string(who) + ": HB_F_NOFOLD has no adjoint here");
     if ((rc = check_ws(ws, wsb, fm_bytes(p, prec, nmaps), who))) return rc;
     const GeomDev &d = p->g->d;
-    if ((rc = launch_leg_synthesis(HB_PLAN_ARGS(p), alm, ws, st, ck_of(p, prec), p->blk_ofs))) return rc;
+    if ((rc = launch_leg_synthesis(p, prec, nmaps, alm, ws, st))) return rc;
     return launch_ring_synthesis(d, prec, nmaps, ws, p->mmax, maps, d.npix, w, true, false, flags, st);
 }
 
@@ -298,7 +297,7 @@ int hb_legendre_analysis_ms(const hb_plan *p, int prec, int nmaps, int nm, const
         return fail(HB_ERR_INVALID, "hb_legendre_analysis_ms: bad args");
     int rc = check_plan(p, nmaps, prec, false, "hb_legendre_analysis_ms");
     if (rc) return rc;
-    return launch_leg_analysis(HB_PLAN_ARGS(p), F, alm, ST(s), ck_of(p, prec), p->blk_ofs, nm, mlist);
+    return launch_leg_analysis(p, prec, nmaps, F, alm, ST(s), nm, mlist);
 }
 int hb_legendre_synthesis_ms(const hb_plan *p, int prec, int nmaps, int nm, const int32_t *mlist, const void *alm,
                              void *G, hb_stream_t s) {
@@ -306,19 +305,19 @@ int hb_legendre_synthesis_ms(const hb_plan *p, int prec, int nmaps, int nm, cons
         return fail(HB_ERR_INVALID, "hb_legendre_synthesis_ms: bad args");
     int rc = check_plan(p, nmaps, prec, false, "hb_legendre_synthesis_ms");
     if (rc) return rc;
-    return launch_leg_synthesis(HB_PLAN_ARGS(p), alm, G, ST(s), ck_of(p, prec), p->blk_ofs, nm, mlist);
+    return launch_leg_synthesis(p, prec, nmaps, alm, G, ST(s), nm, mlist);
 }
 int hb_legendre_analysis(const hb_plan *p, int prec, int nmaps, const void *F, void *alm, hb_stream_t s) {
     if ((prec != 32 && prec != 64) || !F || !alm) return fail(HB_ERR_INVALID, "hb_legendre_analysis: bad args");
     int rc = check_plan(p, nmaps, prec, false, "hb_legendre_analysis");
     if (rc) return rc;
-    return launch_leg_analysis(HB_PLAN_ARGS(p), F, alm, ST(s), ck_of(p, prec), p->blk_ofs);
+    return launch_leg_analysis(p, prec, nmaps, F, alm, ST(s));
 }
 int hb_legendre_synthesis(const hb_plan *p, int prec, int nmaps, const void *alm, void *G, hb_stream_t s) {
     if ((prec != 32 && prec != 64) || !G || !alm) return fail(HB_ERR_INVALID, "hb_legendre_synthesis: bad args");
     int rc = check_plan(p, nmaps, prec, false, "hb_legendre_synthesis");
     if (rc) return rc;
-    return launch_leg_synthesis(HB_PLAN_ARGS(p), alm, G, ST(s), ck_of(p, prec), p->blk_ofs);
+    return launch_leg_synthesis(p, prec, nmaps, alm, G, ST(s));
 }
 
 int hb_probe_fp32(int blocks, int threads, int iters, float *out, hb_stream_t s) {

@@ -139,7 +139,34 @@ struct hb_geom {
     void *alloc_base;
 };
 
-// A geometry plus (lmax, mmax) and the FP32 recursion checkpoints (see hb_plan.cu).
+namespace hb {
+// Scaled recursion tables of the FP64 scalar Legendre kernels (definitions in hb_legendre.cu, built by
+// hb_plan.cu): LT_N values per order m and step k (two l: l = m + 2k and l + 1), in 16-byte groups
+enum {
+    LT_A = 0,  // alpha_k
+    LT_G,      // gamma_k
+    LT_P,      // N_k eps_{l+1}
+    LT_Q,      // N_k eps_{l+2}, 0 if l + 2 > lmax
+    LT_B0,     // -2 M_{l-1}^2 (0 at k = 0)
+    LT_B1,     // 2 M_l^2
+    LT_M0,     // (-1)^k M_l
+    LT_M1,     // (-1)^k M_{l+1}
+    LT_NX,     // N_k, 0 if l + 1 > lmax
+    LT_N = 12
+};
+struct LegTab {
+    double *base;
+    int64_t *ofs;  // [mmax+2] first row of each m
+    __device__ __forceinline__ double *row(int m, int64_t k) const { return base + (ofs[m] + k) * LT_N; }
+};
+// per-unit checkpoint flags: one byte per 64 ring pairs, rows padded to 8 bytes with FL_DEAD
+enum { FL_CLEAN = 0, FL_MIXED = 1, FL_DEAD = 2 };
+__host__ __device__ __forceinline__ int64_t flag_stride(int64_t npairs) { return ((npairs + 63) / 64 + 7) / 8 * 8; }
+// ring pairs with x = cos theta >= LEG_X0 may run the two-l recursion in FP64 (hb_legendre.cu)
+constexpr double LEG_X0 = 0.5;
+}  // namespace hb
+
+// A geometry plus (lmax, mmax), the recursion tables and the FP32 recursion checkpoints (hb_plan.cu).
 struct hb_plan {
     const hb_geom *g;
     int lmax, mmax, flags;
@@ -147,7 +174,11 @@ struct hb_plan {
     size_t bytes;
     int64_t *blk_ofs;       // [mmax+2] first checkpoint block of each m (scalar)
     int64_t *blk_ofs_spin;  // [mmax+2] same for the spin-2 recursions (blocks from max(m,2))
+    hb::LegTab leg;
+    float2 *leg32;          // FP32 plans: (A_l, B_l) of the one-step recursion, [blk_ofs[m] * 256 + l - m]
     float4 *ck;             // scalar checkpoints, or null
+    uint8_t *ck_flags;      // [blocks][flag_stride] FL_CLEAN: the 64 pairs start the block with e = 0, FL_MIXED: some
+                            // e < 0, FL_DEAD: all end the block with e < 0 (evanescent throughout)
     float4 *ckP, *ckM;      // spin-2 checkpoints, or null
 };
 
@@ -172,15 +203,12 @@ int launch_ring_analysis(const GeomDev &g, int precision, int nmaps, const void 
 int launch_ring_synthesis(const GeomDev &g, int precision, int nmaps, const void *Gm, int mmax, void *maps,
                           int64_t map_stride, const double *w, bool apply_weights, bool mdouble, int flags,
                           cudaStream_t st);
-// ck / blk_ofs: FP32 recursion checkpoints of a plan (null: no re-anchoring; FP64 ignores them).
 // mlist (device, nm entries; null: all orders 0..mmax): the orders to transform, F / G holding
 // one row per listed order in list order; alm rows of the other orders are left untouched
-// (analysis over several pair chunks clears the whole alm first).
-int launch_leg_analysis(const GeomDev &g, int precision, int nmaps, int lmax, int mmax, const void *Fm,
-                        void *alm, cudaStream_t st, const float4 *ck, const int64_t *blk_ofs, int nm = 0,
+// (FP64 analysis over several pair chunks clears the whole alm first).
+int launch_leg_analysis(const hb_plan *p, int precision, int nmaps, const void *Fm, void *alm, cudaStream_t st, int nm = 0,
                         const int32_t *mlist = nullptr);
-int launch_leg_synthesis(const GeomDev &g, int precision, int nmaps, int lmax, int mmax, const void *alm,
-                         void *Gm, cudaStream_t st, const float4 *ck, const int64_t *blk_ofs, int nm = 0,
+int launch_leg_synthesis(const hb_plan *p, int precision, int nmaps, const void *alm, void *Gm, cudaStream_t st, int nm = 0,
                          const int32_t *mlist = nullptr);
 int launch_spin_analysis(const GeomDev &g, int precision, int nmaps, int lmax, int mmax, const void *QFm,
                          const void *UFm, void *E, void *B, cudaStream_t st, const float4 *ckP, const float4 *ckM,

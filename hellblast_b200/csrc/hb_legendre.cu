@@ -1,463 +1,503 @@
-// Fused Legendre kernels for the scalar transform (plain per-map form, FP32 and FP64).
+// Scalar Legendre kernels in FP64 (the FP32 ones are in hb_legendre32.cu).
 //
 // Replaces the reference's per-m pipeline (sht_raw.py:46-56: one plm_recurrence launch per m
 // writing the [Nr, lmax+1] Lambda block to HBM (legendre.cu:2-35), host-side factorial norms
 // (sht_raw.py:26-28, which overflow above lmax 85), a per-ring host gather of F_r[m] and a
 // per-l scatter) and the synthesis loops of isht.py:11-23.
 //
-// One CTA per (m, block of ring pairs, map).  Each thread owns K ring pairs (north ring at
-// x = cos theta, south ring at -x) and runs the normalised recursion
-//     lambda_l = A_l x lambda_{l-1} + B_l lambda_{l-2},
-//     A_l = sqrt((4l^2-1)/(l^2-m^2)),  B_l = -A_l sqrt(((l-1)^2-m^2)/(4(l-1)^2-1)),
-// in registers, with the coefficients computed in FP64 per CTA and staged in shared memory.
-// The sectoral start lambda_mm = (-1)^m sqrt((2m+1)!!/((2m)!! 4pi)) sin^m theta is formed in
-// FP64 from log2 tables and carried as mantissa * 2^(S*e): while e < 0 the pair contributes
-// nothing (|lambda| < 2^-S/2 relative), and the recursion rescales by 2^-S whenever the
-// mantissa passes 2^(S/2), so nothing overflows or underflows up to lmax = 16383.
-// Equatorial symmetry lambda_lm(-x) = (-1)^(l+m) lambda_lm(x) folds north and south rings
-// into E = F_N + F_S (even l-m) and O = F_N - F_S (odd l-m).
-// In FP32, x is carried as a float pair (hi + lo) so that the sample positions keep ~48 bits:
-// a rounded cos(theta) shifts a ring by ~1e-7/sin(theta) rad, an l*dtheta phase error that
-// reaches 1e-4 at l ~ 4000.
+// Lambda is generated in registers and never stored.  Equatorial symmetry folds the north and
+// south rings of a pair into E = F_N + F_S (even l-m) and O = F_N - F_S (odd l-m).  With
+// eps_l = sqrt((l^2-m^2)/(4l^2-1)), x lambda_l = eps_{l+1} lambda_{l+1} + eps_l lambda_{l-1}, so the
+// functions r_k = lambda_{m+2k+1} / x carry both parities (Ishioka 2018, J. Meteor. Soc. Japan 96):
+//     lambda_{l+1} = x r_k,   lambda_l = eps_{l+1} r_k + eps_l r_{k-1}      (l = m + 2k),
+// and one recursion over k serves two l.  Scaled to r_k = N_k rho_k with
+// N_k N_{k+1} eps_{l+2} eps_{l+3} = 1/4 its last coefficient is 1; with s = sin theta and
+// alpha_k = 4 N_k^2 it runs on the difference d_k = rho_k - rho_{k-1},
+//     rho_k = rho_{k-1} + d_k,   d_{k+1} = d_k + (gamma_k - alpha_k s^2) rho_k,
+//     gamma_k = alpha_k (1 - eps_{l+1}^2 - eps_{l+2}^2) - 2,
+// which keeps its accuracy towards the poles, where rho varies slowly (Reinsch's form): 3
+// operations for two l and 4 per map for the contraction, against 6 and 4 in the one-step form
+// lambda_l = A x lambda_{l-1} + B lambda_{l-2}.  r_k grows like 1/x, so rings near the equator
+// (|x| < LEG_X0) use the one-step recursion, scaled the same way, lambda_l = M_l y_l,
+// M_l M_{l+1} eps_{l+1} = 1/2: y_{l+1} = 2 M_l^2 x y_l - y_{l-1}, 4 operations for two l (signs of
+// period 4 absorbed in the tables turn the subtraction into an addition).
+// Error against an independent 64-bit reference (alm2map, map2alm at nside 1024, lmax 2047): 3.3e-14,
+// 4.8e-14 (one-step form: 3.3e-14, 5.1e-14; with LEG_X0 = 0.3 instead of 0.5 it is 3.6e-14, 5.4e-14, at
+// 1 % less time).
 //
-// Analysis: a_lm = sum_pairs lambda_lm(x_p) (E or O)_p.  Each thread accumulates its K pairs
-// per l; TL consecutive l are staged in shared memory and reduced across the CTA.
-// Synthesis: G_N/S(m) = sum_l a_lm lambda_lm (+-1)^(l-m): per-pair register accumulators, a_lm
-// broadcast from shared memory, no cross-thread reduction.
+// The coefficients are tables of the plan (LegTab).  Start values come from log2 tables, carried as
+// mantissa * 2^(512 e): while e < 0 a value is below 2^-256, and the state is rescaled whenever it
+// passes 2^256, so nothing overflows or underflows up to lmax = 16383.
+//
+// What bounds the kernels: the FP64 pipe (62 FMA per clock and SM measured); the analysis adds a
+// warp reduction per l.  One map at nside 1024, lmax 2047: synthesis 2063 -> 1160 us, analysis
+// 2826 -> 1820 us (one-step form with a shared-memory reduction per l before).
 #include <cmath>
 
 #include "hb_internal.cuh"
 
 namespace hb {
 
-template <typename T> struct LegCfg;
-template <> struct LegCfg<float> {
-    static constexpr int SE = 64;  // exponent step of the running scale
-    static constexpr int TL = 16;  // l values per reduction group
-};
-template <> struct LegCfg<double> {
-    static constexpr int SE = 512;
-    static constexpr int TL = 8;
-};
+constexpr int LKB = 128;  // two-l steps per staged block of 256 l
 
-template <typename T> struct XRep;
-template <> struct XRep<float> {
-    float hi, lo;
-    __device__ __forceinline__ void load(const GeomDev &g, int64_t p) {
-        hi = g.pair_xhi[p];
-        lo = g.pair_xlo[p];
-    }
-    __device__ __forceinline__ float mul(float v) const { return fmaf(hi, v, lo * v); }
-    __device__ __forceinline__ void zero() { hi = lo = 0.f; }
-};
-template <> struct XRep<double> {
-    double x;
-    __device__ __forceinline__ void load(const GeomDev &g, int64_t p) { x = g.pair_x[p]; }
-    __device__ __forceinline__ double mul(double v) const { return x * v; }
-    __device__ __forceinline__ void zero() { x = 0.0; }
-};
-
-// (A_l, B_l) of the scalar recursion, l relative to m; l = m gives (0, 1) so that the loop can
-// start from the state (lambda_{m-1}, lambda_{m-2}) = (0, lambda_mm); l > lmax gives (0, 0).
-__device__ __forceinline__ void scalar_coef(int l, int m, int lmax, double &A, double &B) {
-    if (l == m) {
-        A = 0.0;
-        B = 1.0;
-        return;
-    }
-    if (l > lmax) {
-        A = B = 0.0;
-        return;
-    }
-    double ll = l, mm = m;
-    A = sqrt((4.0 * ll * ll - 1.0) / ((ll - mm) * (ll + mm)));
-    B = (l - 1 > m) ? -A * sqrt(((ll - 1.0 - mm) * (ll - 1.0 + mm)) / (4.0 * (ll - 1.0) * (ll - 1.0) - 1.0)) : 0.0;
+// start value lambda_mm = mant * 2^(512 e)
+__device__ __forceinline__ void sectoral_start64(const GeomDev &g, int m, int64_t p, double &mant, int &e) {
+    const double L = g.log2cm[m] + (double)m * g.pair_log2sin[p];
+    e = (int)floor((L + 256.0) / 512.0);
+    const double v = exp2(L - 512.0 * e);
+    mant = (m & 1) ? -v : v;
 }
 
-// start value of the scaled recursion: lambda_mm = mant * 2^(SE*e)
-template <typename T>
-__device__ __forceinline__ void sectoral_start(const GeomDev &g, int m, int64_t p, T &mant, int &e) {
-    constexpr int SE = LegCfg<T>::SE;
-    double L = g.log2cm[m] + (double)m * g.pair_log2sin[p];
-    int ee = (int)floor((L + 0.5 * SE) / SE);
-    double v = exp2(L - (double)SE * ee);
-    mant = (T)((m & 1) ? -v : v);
-    e = ee;
+// Recursion zones (see the file comment)
+enum { ZPOLE = 0, ZEQ = 1 };
+
+// U ring pairs per lane of one warp: pair 32 (grp U + u) + lane
+// ZPOLE: r = rho_{k-1}, d = d_k, w = -s^2.  ZEQ: r = y_{l-1}, d = y_{l-2}, w = x.
+template <int U> struct State {
+    double r[U], d[U], w[U];
+    int e[U];
+};
+template <int U> __device__ __forceinline__ int64_t unit_pair(int grp, int u, int lane) {
+    return (int64_t)(grp * U + u) * 32 + lane;
 }
 
-template <typename T> __device__ __forceinline__ T huge_v();
-template <> __device__ __forceinline__ float huge_v<float>() { return 4294967296.0f; }        // 2^32
-template <> __device__ __forceinline__ double huge_v<double>() { return 0x1p256; }
-template <typename T> __device__ __forceinline__ T down_v();
-template <> __device__ __forceinline__ float down_v<float>() { return 5.42101086242752217e-20f; }  // 2^-64
-template <> __device__ __forceinline__ double down_v<double>() { return 0x1p-512; }
-
-constexpr int COEF_CH = 256;  // l values per shared-memory coefficient chunk
-
-// Evanescent skip of the FP32 synthesis: a thread's K ring pairs are consecutive, so a warp
-// covers 32 K consecutive pairs.  Below its turning point a pair's recursion state has a negative
-// exponent (its values kept in units 2^-64 lower) and the exponent never decreases with l; if
-// every pair of the warp still has e < 0 at the checkpoint that ends the current 256-l block, the
-// warp skips the block (the next block re-anchors on its checkpoint anyway), dropping
-// contributions below 2^-64 of the result.  (The analysis kernel keeps its strided pair
-// mapping: its per-l block reduction runs for every warp, so skipping saved nothing there.)
-template <int K>
-__device__ __forceinline__ bool warp_block_dead(const float4 *__restrict__ ck, const int64_t *__restrict__ blk_ofs,
-                                                int m, int jnext, int64_t np, int64_t p0) {
-    if (blk_ofs[m] + jnext >= blk_ofs[m + 1]) return false;  // the block reaches lmax: no end checkpoint
-    const float4 *cb = ck + (blk_ofs[m] + jnext) * np;
-    bool dead = true;
+// ring positions and start values of a group; returns its zone
+template <int U> __device__ __forceinline__ int start_group(const GeomDev &g, const double *tab, int m, int grp, int lane, State<U> &S) {
+    double x[U];
+    bool pole = true;
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-        if (p0 + k < np) dead &= __float_as_int(cb[p0 + k].z) < 0;
-    return __all_sync(0xffffffffu, dead);
+    for (int u = 0; u < U; ++u) {
+        const int64_t p = unit_pair<U>(grp, u, lane);
+        x[u] = p < g.npairs ? g.pair_x[p] : 0.0;
+        if (p < g.npairs) pole &= x[u] >= LEG_X0;
+    }
+    const int zone = __all_sync(0xffffffffu, pole) ? ZPOLE : ZEQ;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int64_t p = unit_pair<U>(grp, u, lane);
+        S.w[u] = zone == ZPOLE ? (x[u] - 1.0) * (x[u] + 1.0) : x[u];
+        S.r[u] = S.d[u] = 0.0;
+        S.e[u] = 0;
+        if (p < g.npairs) {  // rho_0 = lambda_mm / (N_0 eps_{m+1}), y_m = lambda_mm / M_m
+            double mant;
+            sectoral_start64(g, m, p, mant, S.e[u]);
+            S.d[u] = mant / (zone == ZPOLE ? tab[LT_P] : tab[LT_M0]);
+        }
+    }
+    return zone;
 }
 
-template <typename T, int K, int NT>
-__global__ void __launch_bounds__(NT, 2) leg_analysis_kernel(GeomDev g, int lmax, int mmax, const c2_t<T> *__restrict__ Fm,
-                                                             int64_t fm_stride, c2_t<T> *__restrict__ alm,
-                                                             int64_t alm_stride, int atomic,
-                                                             const float4 *__restrict__ ck,
-                                                             const int64_t *__restrict__ blk_ofs,
-                                                             const int32_t *__restrict__ mlist) {
-    using V = c2_t<T>;
-    constexpr int TL = LegCfg<T>::TL;
-    constexpr int TPS = NT / TL;  // threads reducing one l slot
-    static_assert(TPS >= 1 && TPS <= 32 && (32 % TPS) == 0, "bad reduction shape");
-    __shared__ V coef[COEF_CH];
-    extern __shared__ __align__(16) unsigned char leg_dyn_smem[];
-    V(*red)[TL][NT] = reinterpret_cast<V(*)[TL][NT]>(leg_dyn_smem);  // [2][TL][NT]
+// one two-l step; f(u, even value, odd value) sees (rho, rho) in ZPOLE
+template <int ZONE, int U, typename Fn> __device__ __forceinline__ void two_step(State<U> &S, double2 c, Fn f) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (ZONE == ZPOLE) {
+            S.r[u] += S.d[u];
+            f(u, S.r[u], S.r[u]);
+            S.d[u] = fma(fma(c.x, S.w[u], c.y), S.r[u], S.d[u]);
+        } else {
+            S.d[u] = fma(c.x * S.w[u], S.r[u], S.d[u]);
+            S.r[u] = fma(c.y * S.w[u], S.d[u], S.r[u]);
+            f(u, S.d[u], S.r[u]);
+        }
+    }
+}
+
+enum { CLEAN = 0, MIXED = 1, DEAD = 2 };  // no / some / every value of the warp's group has e < 0
+
+template <int U> __device__ __forceinline__ int mode_of(const State<U> &S) {
+    bool neg = false, live = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        neg |= S.e[u] < 0;
+        live |= S.e[u] >= 0;
+    }
+    if (!__any_sync(0xffffffffu, neg)) return CLEAN;
+    return __any_sync(0xffffffffu, live) ? MIXED : DEAD;
+}
+
+// Brings values that have grown past 2^256 to the next exponent; up(u) is told of each.  False when
+// the warp has none (one vote, the usual case).
+template <int U, typename Fn> __device__ __forceinline__ bool rescale(State<U> &S, Fn up) {
+    bool any = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) any |= S.e[u] < 0 && fabs(S.r[u]) > 0x1p256;
+    if (!__any_sync(0xffffffffu, any)) return false;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (S.e[u] < 0 && fabs(S.r[u]) > 0x1p256) {
+            S.r[u] *= 0x1p-512;
+            S.d[u] *= 0x1p-512;
+            ++S.e[u];
+            up(u);
+        }
+    return true;
+}
+
+// four consecutive table values (rows are 16-byte aligned)
+__device__ __forceinline__ double4 four(const double *t) {
+    const double2 a = *reinterpret_cast<const double2 *>(t), b = *reinterpret_cast<const double2 *>(t + 2);
+    return make_double4(a.x, a.y, b.x, b.y);
+}
+
+// sum over the warp of NV values per lane: lane 2 i (NV 16) or i (NV 32) ends with the sum of v[i]
+template <int NV> __device__ __forceinline__ double warp_sums(double (&v)[NV], int lane) {
+    static_assert(NV == 16 || NV == 32, "values per lane");
+#pragma unroll
+    for (int h = NV / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double keep = up ? v[i + h] : v[i], send = up ? v[i] : v[i + h];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    if (NV == 16) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    return v[0];
+}
+
+// ------------------------------------------------------------------ analysis
+template <int NB, int U> struct Weights {
+    double er[NB][U], ei[NB][U], qr[NB][U], qi[NB][U];
+};
+
+// TL two-l steps: values times weights summed over the group's pairs, added to the warp's row
+// red[(step * NB + map) * 4 + (E re, E im, O re, O im)]; values with e < 0 count as zero
+template <int ZONE, bool GATED, int U, int NB, int TL>
+__device__ __forceinline__ void anal_chunk(State<U> &S, const Weights<NB, U> &W, const double2 *cf, double *red, int lane) {
+    double v[TL * NB * 4];
+#pragma unroll
+    for (int s = 0; s < TL; ++s) {
+        two_step<ZONE>(S, cf[s], [&](int u, double ve, double vo) {
+            if (GATED) {
+                ve = S.e[u] < 0 ? 0.0 : ve;
+                vo = S.e[u] < 0 ? 0.0 : vo;
+            }
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                double *a = v + (s * NB + b) * 4;
+                a[0] = u ? fma(ve, W.er[b][u], a[0]) : ve * W.er[b][u];
+                a[1] = u ? fma(ve, W.ei[b][u], a[1]) : ve * W.ei[b][u];
+                a[2] = u ? fma(vo, W.qr[b][u], a[2]) : vo * W.qr[b][u];
+                a[3] = u ? fma(vo, W.qi[b][u], a[3]) : vo * W.qi[b][u];
+            }
+        });
+    }
+    const double s = warp_sums<TL * NB * 4>(v, lane);
+    if (TL * NB * 4 == 32)
+        red[lane] += s;
+    else if (!(lane & 1))
+        red[lane >> 1] += s;
+}
+
+// a block's steps [0, nk) (nk a multiple of TL; past lmax the coefficients are zero); groups that
+// are evanescent as a whole run the recursion alone
+template <int ZONE, int U, int NB, int TL>
+__device__ __forceinline__ void anal_block(State<U> &S, const Weights<NB, U> &W, int nk, int &mode, const double2 *cf, double *red,
+                                           int lane) {
+    int k = 0;
+    while (mode != CLEAN && k < nk) {
+        if (mode == DEAD) {
+#pragma unroll
+            for (int s = 0; s < TL; ++s) two_step<ZONE>(S, cf[k + s], [](int, double, double) {});
+        } else {
+            anal_chunk<ZONE, true, U, NB, TL>(S, W, cf + k, red + k * NB * 4, lane);
+        }
+        k += TL;
+        if (rescale(S, [](int) {})) mode = mode_of(S);
+    }
+#pragma unroll 1
+    for (; k < nk; k += TL) anal_chunk<ZONE, false, U, NB, TL>(S, W, cf + k, red + k * NB * 4, lane);
+}
+
+// One CTA per (order, chunk of ring pairs, NB maps), every warp keeping one group of 32 U pairs in
+// registers over all l.  Per block of 256 l the warps' rows are summed by zone and combined to
+//     a_l = N_k eps_{l+1} c_k + N_{k-1} eps_l c_{k-1} + M_l e_k,   a_{l+1} = N_k o_k + M_{l+1} o'_k.
+template <int U, int NB, int TL, int NT>
+__global__ void __launch_bounds__(NT) leg_analysis64_kernel(GeomDev g, LegTab tb, int lmax, int mmax,
+                                                            const double2 *__restrict__ Fm, int64_t fm_stride,
+                                                            double2 *__restrict__ alm, int64_t alm_stride, int atomic,
+                                                            const int32_t *__restrict__ mlist) {
+    constexpr int NW = NT / 32, ROW = LKB * NB * 4;
+    __shared__ double2 ca[LKB], cb[LKB];
+    __shared__ double cprev[2 * NB];
+    __shared__ int wzone[NW];
+    extern __shared__ double red[];  // [NW][LKB][NB][4], then the sums [zone][LKB][NB][4]
+    double *sum = red + NW * ROW;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = blockIdx.y * NW + warp;
     // F row blockIdx.x holds order m (all orders, or the orders of mlist in list order)
-    const int m = mlist ? mlist[blockIdx.x] : blockIdx.x, chunk = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
+    const int m = mlist ? mlist[blockIdx.x] : blockIdx.x;
     if (m < 0 || m > mmax) return;  // a listed order outside the plan: nothing read or written
     const int64_t np = g.npairs;
-    const V *F = Fm + b * fm_stride + (int64_t)blockIdx.x * np * 2;
-    V *out = alm + b * alm_stride;
-
-    T l1[K], l2[K];
-    XRep<T> x[K];
-    V ge[K], go[K];
-    int e[K];
-    bool anyneg = false;
+    const double2 *F = Fm + (int64_t)blockIdx.z * NB * fm_stride + (int64_t)blockIdx.x * np * 2;
+    const double *tab = tb.row(m, 0);
+    const bool any = (int64_t)grp * U * 32 < np;
+    State<U> S;
+    Weights<NB, U> W;
+    const int zone = start_group(g, tab, m, grp, lane, S);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const int64_t p = (int64_t)chunk * NT * K + (int64_t)k * NT + tid;
-        l1[k] = (T)0;
-        if (p < np) {
-            x[k].load(g, p);
-            T mant;
-            sectoral_start<T>(g, m, p, mant, e[k]);
-            l2[k] = mant;
-            V fn = F[2 * p], fs = F[2 * p + 1];
-            ge[k] = cadd(fn, fs);
-            go[k] = csub(fn, fs);
-            if (e[k] < 0) {
-                ge[k] = go[k] = mk2((T)0, (T)0);
-                anyneg = true;
+    for (int u = 0; u < U; ++u) {
+        const int64_t p = unit_pair<U>(grp, u, lane);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            W.er[b][u] = W.ei[b][u] = W.qr[b][u] = W.qi[b][u] = 0.0;
+            if (p < np) {
+                const double2 fn = F[b * fm_stride + 2 * p], fs = F[b * fm_stride + 2 * p + 1];
+                const double x = zone == ZPOLE ? g.pair_x[p] : 1.0;
+                W.er[b][u] = fn.x + fs.x;
+                W.ei[b][u] = fn.y + fs.y;
+                W.qr[b][u] = (fn.x - fs.x) * x;
+                W.qi[b][u] = (fn.y - fs.y) * x;
             }
-        } else {
-            x[k].zero();
-            l2[k] = (T)0;
-            e[k] = 0;
-            ge[k] = go[k] = mk2((T)0, (T)0);
         }
     }
-
-    int rb = 0;
-    for (int l0 = m; l0 <= lmax; l0 += TL) {
-        const int lrel = l0 - m;
-        if ((lrel % COEF_CH) == 0) {
-            __syncthreads();
-            for (int i = tid; i < COEF_CH; i += NT) {
-                double A, B;
-                scalar_coef(l0 + i, m, lmax, A, B);
-                coef[i] = mk2((T)A, (T)B);
-            }
-            __syncthreads();
-            if constexpr (sizeof(T) == 4) {
-                if (ck != nullptr && lrel > 0) {  // re-anchor on the FP64-computed state
-                    const float4 *cb = ck + (blk_ofs[m] + lrel / COEF_CH) * np;
-                    anyneg = false;
-#pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        const int64_t p = (int64_t)chunk * NT * K + (int64_t)k * NT + tid;
-                        if (p < np) {
-                            const float4 c = cb[p];
-                            l1[k] = c.x;
-                            l2[k] = c.y;
-                            const int en = __float_as_int(c.z);
-                            if (en != e[k]) {
-                                e[k] = en;
-                                if (en == 0) {
-                                    V fn = F[2 * p], fs = F[2 * p + 1];
-                                    ge[k] = cadd(fn, fs);
-                                    go[k] = csub(fn, fs);
-                                } else {
-                                    ge[k] = go[k] = mk2((T)0, (T)0);
-                                }
-                            }
-                            anyneg |= e[k] < 0;
-                        }
-                    }
-                }
-            }
+    int mode = mode_of(S);
+    double *mine = red + warp * ROW;
+    if (lane == 0) wzone[warp] = any ? zone : -1;
+    for (int l0 = m; l0 <= lmax; l0 += 2 * LKB, tab += LKB * LT_N) {
+        const int nk = min(LKB, (lmax - l0) / 2 + 1), nkp = (nk + TL - 1) / TL * TL;
+        for (int i = tid; i < LKB; i += NT) {
+            const double4 z = make_double4(0.0, 0.0, 0.0, 0.0);
+            const double4 a = i < nk ? four(tab + (int64_t)i * LT_N + LT_A) : z, b = i < nk ? four(tab + (int64_t)i * LT_N + LT_B0) : z;
+            ca[i] = make_double2(a.x, a.y);
+            cb[i] = make_double2(b.x, b.y);
         }
-        const V *cf = coef + (lrel % COEF_CH);
-#pragma unroll
-        for (int s = 0; s < TL; ++s) {
-            const V ab = cf[s];
-            T ar = (T)0, ai = (T)0;
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                T v = ab.x * x[k].mul(l1[k]) + ab.y * l2[k];
-                l2[k] = l1[k];
-                l1[k] = v;
-                const V gg = (s & 1) ? go[k] : ge[k];
-                ar = fma(v, gg.x, ar);
-                ai = fma(v, gg.y, ai);
+        for (int i = lane; i < ROW; i += 32) mine[i] = 0.0;
+        __syncthreads();
+        if (any) {
+            if (zone == ZPOLE)
+                anal_block<ZPOLE, U, NB, TL>(S, W, nkp, mode, ca, mine, lane);
+            else
+                anal_block<ZEQ, U, NB, TL>(S, W, nkp, mode, cb, mine, lane);
+        }
+        __syncthreads();
+        for (int i = tid; i < 2 * nk * NB * 4; i += NT) {
+            const int z = i >= nk * NB * 4, o = i - z * nk * NB * 4;
+            double s = 0.0;
+            for (int w = 0; w < NW; ++w)
+                if (wzone[w] == z) s += red[w * ROW + o];
+            sum[z * ROW + o] = s;
+        }
+        __syncthreads();
+        for (int i = tid; i < nk * NB; i += NT) {
+            const int k = i % nk, b = i / nk, l = l0 + 2 * k;
+            const double *A = sum + (k * NB + b) * 4, *B = A + ROW, *t = tab + (int64_t)k * LT_N;
+            double2 q = make_double2(0.0, 0.0);
+            if (l > m) {
+                const double *c = k > 0 ? A - NB * 4 : cprev + 2 * b;
+                q = make_double2(t[LT_Q - LT_N] * c[0], t[LT_Q - LT_N] * c[1]);
             }
-            red[rb][s][tid] = mk2(ar, ai);
-            if ((s & 3) == 3 && __any_sync(0xffffffffu, anyneg)) {
-                anyneg = false;
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    if (e[k] < 0) {
-                        if (fabs(l1[k]) > huge_v<T>()) {
-                            l1[k] *= down_v<T>();
-                            l2[k] *= down_v<T>();
-                            if (++e[k] == 0) {
-                                const int64_t p = (int64_t)chunk * NT * K + (int64_t)k * NT + tid;
-                                V fn = F[2 * p], fs = F[2 * p + 1];
-                                ge[k] = cadd(fn, fs);
-                                go[k] = csub(fn, fs);
-                            }
-                        }
-                        anyneg |= e[k] < 0;
-                    }
+            const double2 v0 = make_double2(t[LT_P] * A[0] + t[LT_M0] * B[0] + q.x, t[LT_P] * A[1] + t[LT_M0] * B[1] + q.y);
+            const double2 v1 = make_double2(t[LT_NX] * A[2] + t[LT_M1] * B[2], t[LT_NX] * A[3] + t[LT_M1] * B[3]);
+            double2 *dst = alm + ((int64_t)blockIdx.z * NB + b) * alm_stride + alm_idx(lmax, l, m);
+            if (atomic) {
+                atomicAdd(&dst[0].x, v0.x);
+                atomicAdd(&dst[0].y, v0.y);
+                if (l < lmax) {
+                    atomicAdd(&dst[1].x, v1.x);
+                    atomicAdd(&dst[1].y, v1.y);
                 }
+            } else {
+                dst[0] = v0;
+                if (l < lmax) dst[1] = v1;
             }
         }
         __syncthreads();
-        {
-            const int s = tid / TPS, sub = tid % TPS;
-            T rr = (T)0, ri = (T)0;
-#pragma unroll
-            for (int j = 0; j < TL; ++j) {
-                const V v = red[rb][s][sub + j * TPS];
-                rr += v.x;
-                ri += v.y;
-            }
-#pragma unroll
-            for (int off = TPS / 2; off >= 1; off >>= 1) {
-                rr += __shfl_xor_sync(0xffffffffu, rr, off);
-                ri += __shfl_xor_sync(0xffffffffu, ri, off);
-            }
-            const int l = l0 + s;
-            if (sub == 0 && l <= lmax) {
-                V *dst = out + alm_idx(lmax, l, m);
-                if (atomic) {
-                    atomicAdd(&dst->x, rr);
-                    atomicAdd(&dst->y, ri);
-                } else {
-                    *dst = mk2(rr, ri);
-                }
-            }
-        }
-        rb ^= 1;
+        if (tid < 2 * NB) cprev[tid] = sum[((LKB - 1) * NB + tid / 2) * 4 + tid % 2];
     }
 }
 
-template <typename T, int K, int NT>
-__global__ void __launch_bounds__(NT, 2) leg_synthesis_kernel(GeomDev g, int lmax, int mmax, const c2_t<T> *__restrict__ alm,
-                                                              int64_t alm_stride, c2_t<T> *__restrict__ Gm,
-                                                              int64_t gm_stride, const float4 *__restrict__ ck,
-                                                              const int64_t *__restrict__ blk_ofs,
-                                                              const int32_t *__restrict__ mlist) {
-    using V = c2_t<T>;
-    __shared__ V coef[COEF_CH];
-    __shared__ V acoef[COEF_CH];
-    // G row blockIdx.x holds order m (all orders, or the orders of mlist in list order)
-    const int m = mlist ? mlist[blockIdx.x] : blockIdx.x, chunk = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
+// ------------------------------------------------------------------ synthesis
+struct alignas(16) ACoef {  // factors of the even and the odd value
+    double cr, ci, dr, di;
+};
+template <int NB, int U> struct Sums {
+    double er[NB][U], ei[NB][U], qr[NB][U], qi[NB][U];
+};
+
+template <int ZONE, int U, int NB>
+__device__ __forceinline__ void synth_step(State<U> &S, Sums<NB, U> &A, double2 c, const ACoef *ac) {
+    ACoef a[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) a[b] = ac[b * LKB];
+    two_step<ZONE>(S, c, [&](int u, double ve, double vo) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            A.er[b][u] = fma(ve, a[b].cr, A.er[b][u]);
+            A.ei[b][u] = fma(ve, a[b].ci, A.ei[b][u]);
+            A.qr[b][u] = fma(vo, a[b].dr, A.qr[b][u]);
+            A.qi[b][u] = fma(vo, a[b].di, A.qi[b][u]);
+        }
+    });
+}
+
+// the sums are kept in units of 2^(512 e); groups that are evanescent as a whole (below 2^-256)
+// run the recursion alone
+template <int ZONE, int U, int NB>
+__device__ __forceinline__ void synth_block(State<U> &S, Sums<NB, U> &A, int nk, int &mode, const double2 *cf, const ACoef *ac) {
+    int k = 0;
+    while (mode != CLEAN && k < nk) {
+        if (mode == DEAD) {
+#pragma unroll
+            for (int s = 0; s < 4; ++s) two_step<ZONE>(S, cf[k + s], [](int, double, double) {});
+        } else {
+#pragma unroll
+            for (int s = 0; s < 4; ++s) synth_step<ZONE>(S, A, cf[k + s], ac + k + s);
+        }
+        k += 4;
+        const bool up = rescale(S, [&](int u) {
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                A.er[b][u] *= 0x1p-512;
+                A.ei[b][u] *= 0x1p-512;
+                A.qr[b][u] *= 0x1p-512;
+                A.qi[b][u] *= 0x1p-512;
+            }
+        });
+        if (up) mode = mode_of(S);
+    }
+#pragma unroll 4
+    for (; k < nk; ++k) synth_step<ZONE>(S, A, cf[k], ac + k);
+}
+
+// One warp per (group of 32 U ring pairs, order, NB maps): the warps of larger CTAs would wait for
+// each other at every block, since those near the pole spend less on it.
+template <int U, int NB, int MINB>
+__global__ void __launch_bounds__(32, MINB) leg_synthesis64_kernel(GeomDev g, LegTab tb, int lmax, int mmax,
+                                                                  const double2 *__restrict__ alm, int64_t alm_stride,
+                                                                  double2 *__restrict__ Gm, int64_t gm_stride,
+                                                                  const int32_t *__restrict__ mlist) {
+    __shared__ double2 cf[LKB];
+    __shared__ ACoef ac[NB * LKB];
+    const int lane = threadIdx.x, grp = blockIdx.x;
+    // G row blockIdx.y holds order m (all orders, or the orders of mlist in list order)
+    const int m = mlist ? mlist[blockIdx.y] : blockIdx.y;
     if (m < 0 || m > mmax) return;  // a listed order outside the plan: nothing read or written
     const int64_t np = g.npairs;
-    const V *a = alm + b * alm_stride;
-    V *G = Gm + b * gm_stride + (int64_t)blockIdx.x * np * 2;
-
-    T l1[K], l2[K];
-    XRep<T> x[K];
-    V ae[K], ao[K];
-    int e[K];
-    bool anyneg = false;
+    const double2 *a = alm + (int64_t)blockIdx.z * NB * alm_stride;
+    const double *tab = tb.row(m, 0);
+    State<U> S;
+    Sums<NB, U> A;
+    const int zone = start_group(g, tab, m, grp, lane, S);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const int64_t p = (int64_t)chunk * NT * K + (int64_t)tid * K + k;
-        l1[k] = (T)0;
-        ae[k] = ao[k] = mk2((T)0, (T)0);
-        if (p < np) {
-            x[k].load(g, p);
-            T mant;
-            sectoral_start<T>(g, m, p, mant, e[k]);
-            l2[k] = mant;
-            anyneg |= e[k] < 0;
-        } else {
-            x[k].zero();
-            l2[k] = (T)0;
-            e[k] = 0;
-        }
-    }
-    bool skip = false;  // this warp's rows are all evanescent through the current block
-    for (int l0 = m; l0 <= lmax; l0 += 4) {
-        const int lrel = l0 - m;
-        if ((lrel % COEF_CH) == 0) {
-            __syncthreads();
-            for (int i = tid; i < COEF_CH; i += NT) {
-                double A, B;
-                scalar_coef(l0 + i, m, lmax, A, B);
-                coef[i] = mk2((T)A, (T)B);
-                acoef[i] = (l0 + i <= lmax) ? a[alm_idx(lmax, l0 + i, m)] : mk2((T)0, (T)0);
-            }
-            __syncthreads();
-            if constexpr (sizeof(T) == 4) {
-                if (ck != nullptr && lrel > 0) {  // re-anchor on the FP64-computed state
-                    const float4 *cb = ck + (blk_ofs[m] + lrel / COEF_CH) * np;
-                    anyneg = false;
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        const int64_t p = (int64_t)chunk * NT * K + (int64_t)tid * K + k;
-                        if (p < np) {
-                            const float4 c = cb[p];
-                            l1[k] = c.x;
-                            l2[k] = c.y;
-                            const int en = __float_as_int(c.z);
-                            if (en != e[k]) {  // accumulators are kept in units of 2^(64 e)
-                                const float f = ldexpf(1.0f, 64 * max(-3, e[k] - en));
-                                ae[k] = cscale(ae[k], f);
-                                ao[k] = cscale(ao[k], f);
-                                e[k] = en;
-                            }
-                            anyneg |= e[k] < 0;
-                        }
+        for (int b = 0; b < NB; ++b) A.er[b][u] = A.ei[b][u] = A.qr[b][u] = A.qi[b][u] = 0.0;
+    int mode = mode_of(S);
+    for (int l0 = m; l0 <= lmax; l0 += 2 * LKB, tab += LKB * LT_N) {
+        const int nk = min(LKB, (lmax - l0) / 2 + 1), nkp = (nk + 3) / 4 * 4;
+        __syncwarp();
+#pragma unroll
+        for (int k = lane; k < LKB; k += 32) {
+            const int l = l0 + 2 * k;
+            double2 c = make_double2(0.0, 0.0);
+            ACoef v[NB] = {};
+            if (k < nk) {
+                const double *t = tab + (int64_t)k * LT_N;
+                const double4 f = four(t + (zone == ZPOLE ? LT_A : LT_B0));
+                const double n = t[LT_NX];
+                c = make_double2(f.x, f.y);
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    const double2 *al = a + b * alm_stride + alm_idx(lmax, l, m);
+                    const double2 z = make_double2(0.0, 0.0), a0 = al[0], a1 = l + 1 <= lmax ? al[1] : z;
+                    if (zone == ZPOLE) {
+                        const double2 a2 = l + 2 <= lmax ? al[2] : z;
+                        v[b] = {f.z * a0.x + f.w * a2.x, f.z * a0.y + f.w * a2.y, n * a1.x, n * a1.y};
+                    } else {
+                        v[b] = {f.z * a0.x, f.z * a0.y, f.w * a1.x, f.w * a1.y};
                     }
                 }
-                if (ck != nullptr)
-                    skip = warp_block_dead<K>(ck, blk_ofs, m, lrel / COEF_CH + 1, np,
-                                              (int64_t)chunk * NT * K + (int64_t)tid * K);
             }
-        }
-        if (skip) continue;
-        const int i0 = lrel % COEF_CH;
+            cf[k] = c;
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const V ab = coef[i0 + s], av = acoef[i0 + s];
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                T v = ab.x * x[k].mul(l1[k]) + ab.y * l2[k];
-                l2[k] = l1[k];
-                l1[k] = v;
-                if (s & 1) {
-                    ao[k].x = fma(v, av.x, ao[k].x);
-                    ao[k].y = fma(v, av.y, ao[k].y);
-                } else {
-                    ae[k].x = fma(v, av.x, ae[k].x);
-                    ae[k].y = fma(v, av.y, ae[k].y);
-                }
-            }
+            for (int b = 0; b < NB; ++b) ac[b * LKB + k] = v[b];
         }
-        if (__any_sync(0xffffffffu, anyneg)) {
-            anyneg = false;
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                if (e[k] < 0) {
-                    if (fabs(l1[k]) > huge_v<T>()) {
-                        l1[k] *= down_v<T>();
-                        l2[k] *= down_v<T>();
-                        ae[k] = cscale(ae[k], down_v<T>());
-                        ao[k] = cscale(ao[k], down_v<T>());
-                        ++e[k];
-                    }
-                    anyneg |= e[k] < 0;
-                }
-            }
-        }
+        __syncwarp();
+        if (zone == ZPOLE)
+            synth_block<ZPOLE, U, NB>(S, A, nkp, mode, cf, ac);
+        else
+            synth_block<ZEQ, U, NB>(S, A, nkp, mode, cf, ac);
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const int64_t p = (int64_t)chunk * NT * K + (int64_t)tid * K + k;
-        if (p < np) {
-            T f = (e[k] == 0) ? (T)1 : (T)ldexp(1.0, LegCfg<T>::SE * e[k]);
-            V gn = cscale(cadd(ae[k], ao[k]), f), gs = cscale(csub(ae[k], ao[k]), f);
-            G[2 * p] = gn;
-            G[2 * p + 1] = gs;
+    for (int u = 0; u < U; ++u) {
+        const int64_t p = unit_pair<U>(grp, u, lane);
+        if (p >= np) continue;
+        const double f = S.e[u] == 0 ? 1.0 : ldexp(1.0, 512 * S.e[u]), fq = zone == ZPOLE ? f * g.pair_x[p] : f;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            double2 *G = Gm + ((int64_t)blockIdx.z * NB + b) * gm_stride + ((int64_t)blockIdx.y * np + p) * 2;
+            G[0] = make_double2(f * A.er[b][u] + fq * A.qr[b][u], f * A.ei[b][u] + fq * A.qi[b][u]);
+            G[1] = make_double2(f * A.er[b][u] - fq * A.qr[b][u], f * A.ei[b][u] - fq * A.qi[b][u]);
         }
     }
 }
 
-template <typename T, int K, int NT>
-static int run_analysis(const GeomDev &g, int nmaps, int lmax, int mmax, const c2_t<T> *Fm, c2_t<T> *alm,
-                        cudaStream_t st, const float4 *ck, const int64_t *bo, int nm, const int32_t *mlist) {
-    const int64_t per = (int64_t)K * NT;
-    const int nchunks = (int)((g.npairs + per - 1) / per);
-    const int rows = mlist ? nm : mmax + 1;
-    const int64_t fm_stride = (int64_t)rows * g.npairs * 2;
-    const int64_t alm_stride = alm_size(lmax, mmax);
-    if (nchunks > 1) HB_CUDA_TRY(cudaMemsetAsync(alm, 0, sizeof(c2_t<T>) * alm_stride * nmaps, st));
-    const int smem = 2 * LegCfg<T>::TL * NT * (int)sizeof(c2_t<T>);
-    HB_CUDA_TRY(cudaFuncSetAttribute(leg_analysis_kernel<T, K, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    dim3 grid((unsigned)rows, (unsigned)nchunks, (unsigned)nmaps);
-    leg_analysis_kernel<T, K, NT><<<grid, NT, smem, st>>>(g, lmax, mmax, Fm, fm_stride, alm, alm_stride, nchunks > 1,
-                                                           ck, bo, mlist);
+// ------------------------------------------------------------------ launches
+struct LegArgs {
+    const hb_plan *p;
+    int rows;
+    const int32_t *mlist;
+    cudaStream_t st;
+    int64_t np() const { return p->g->d.npairs; }
+    int64_t f_stride() const { return (int64_t)rows * np() * 2; }
+    int64_t a_stride() const { return alm_size(p->lmax, p->mmax); }
+};
+
+template <int U, int NB, int TL, int NT> static int run_analysis(const LegArgs &L, int nz, const double2 *F, double2 *alm) {
+    const int64_t per = (int64_t)U * NT;
+    const int nchunks = (int)((L.np() + per - 1) / per);
+    if (nchunks > 1) HB_CUDA_TRY(cudaMemsetAsync(alm, 0, sizeof(double2) * L.a_stride() * NB * nz, L.st));
+    const int smem = (NT / 32 + 2) * LKB * NB * 4 * (int)sizeof(double);
+    HB_CUDA_TRY(cudaFuncSetAttribute(leg_analysis64_kernel<U, NB, TL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    dim3 grid((unsigned)L.rows, (unsigned)nchunks, (unsigned)nz);
+    leg_analysis64_kernel<U, NB, TL, NT><<<grid, NT, smem, L.st>>>(L.p->g->d, L.p->leg, L.p->lmax, L.p->mmax, F, L.f_stride(),
+                                                                   alm, L.a_stride(), nchunks > 1, L.mlist);
+    HB_CHECK_LAUNCH();
+    return HB_OK;
+}
+template <int U, int NB, int MINB> static int run_synthesis(const LegArgs &L, int nz, const double2 *alm, double2 *G) {
+    dim3 grid((unsigned)((L.np() + 32 * U - 1) / (32 * U)), (unsigned)L.rows, (unsigned)nz);
+    leg_synthesis64_kernel<U, NB, MINB><<<grid, 32, 0, L.st>>>(L.p->g->d, L.p->leg, L.p->lmax, L.p->mmax, alm, L.a_stride(), G,
+                                                               L.f_stride(), L.mlist);
     HB_CHECK_LAUNCH();
     return HB_OK;
 }
 
-template <typename T, int K, int NT>
-static int run_synthesis(const GeomDev &g, int nmaps, int lmax, int mmax, const c2_t<T> *alm, c2_t<T> *Gm,
-                         cudaStream_t st, const float4 *ck, const int64_t *bo, int nm, const int32_t *mlist) {
-    const int64_t per = (int64_t)K * NT;
-    const int nchunks = (int)((g.npairs + per - 1) / per);
-    const int rows = mlist ? nm : mmax + 1;
-    const int64_t gm_stride = (int64_t)rows * g.npairs * 2;
-    const int64_t alm_stride = alm_size(lmax, mmax);
-    dim3 grid((unsigned)rows, (unsigned)nchunks, (unsigned)nmaps);
-    leg_synthesis_kernel<T, K, NT><<<grid, NT, 0, st>>>(g, lmax, mmax, alm, alm_stride, Gm, gm_stride, ck, bo, mlist);
-    HB_CHECK_LAUNCH();
-    return HB_OK;
+// Pairs per lane and warps per CTA: large grids amortise the warp reduction (analysis) and the
+// coefficient loads (synthesis) over U = 4 pairs per lane; grids below 1024 pairs spread their few
+// pairs over more warps, since they do not fill the GPU.
+template <int NB> static int analysis_nb(const LegArgs &L, int nz, const double2 *F, double2 *alm) {
+    if (L.np() >= 1024) return run_analysis<4, NB, NB == 1 ? 4 : 2, NB == 1 ? 512 : 256>(L, nz, F, alm);
+    if (L.np() >= 256) return run_analysis<2, NB, NB == 1 ? 4 : 2, 256>(L, nz, F, alm);
+    return run_analysis<1, NB, NB == 1 ? 4 : 2, 128>(L, nz, F, alm);
+}
+template <int NB> static int synthesis_nb(const LegArgs &L, int nz, const double2 *alm, double2 *G) {
+    if (L.np() >= 1024) return run_synthesis<NB == 1 ? 4 : 2, NB, NB == 1 ? 16 : 14>(L, nz, alm, G);
+    return run_synthesis<1, NB, 16>(L, nz, alm, G);
 }
 
-template <typename T>
-static int analysis_t(const GeomDev &g, int nmaps, int lmax, int mmax, int nm, const int32_t *mlist, const c2_t<T> *Fm, c2_t<T> *alm,
-                      cudaStream_t st, const float4 *ck, const int64_t *bo) {
-    if (g.npairs >= 1024) return run_analysis<T, 8, 256>(g, nmaps, lmax, mmax, Fm, alm, st, ck, bo, nm, mlist);
-    if (g.npairs >= 256) return run_analysis<T, 4, 128>(g, nmaps, lmax, mmax, Fm, alm, st, ck, bo, nm, mlist);
-    if (g.npairs >= 64) return run_analysis<T, 2, 64>(g, nmaps, lmax, mmax, Fm, alm, st, ck, bo, nm, mlist);
-    return run_analysis<T, 1, 64>(g, nmaps, lmax, mmax, Fm, alm, st, ck, bo, nm, mlist);
+// maps in pairs that share one recursion: 11 operations per (two l, ring pair) for two maps, 7 for one
+template <typename Fn2, typename Fn1> static int by_two(int nmaps, Fn2 f2, Fn1 f1) {
+    if (nmaps >= 2)
+        if (int rc = f2(nmaps / 2, 0)) return rc;
+    return nmaps % 2 ? f1(1, nmaps - 1) : HB_OK;
 }
 
-template <typename T>
-static int synthesis_t(const GeomDev &g, int nmaps, int lmax, int mmax, int nm, const int32_t *mlist, const c2_t<T> *alm, c2_t<T> *Gm,
-                       cudaStream_t st, const float4 *ck, const int64_t *bo) {
-    if (g.npairs >= 1024) return run_synthesis<T, 8, 256>(g, nmaps, lmax, mmax, alm, Gm, st, ck, bo, nm, mlist);
-    if (g.npairs >= 256) return run_synthesis<T, 4, 128>(g, nmaps, lmax, mmax, alm, Gm, st, ck, bo, nm, mlist);
-    if (g.npairs >= 64) return run_synthesis<T, 2, 64>(g, nmaps, lmax, mmax, alm, Gm, st, ck, bo, nm, mlist);
-    return run_synthesis<T, 1, 64>(g, nmaps, lmax, mmax, alm, Gm, st, ck, bo, nm, mlist);
+int launch_leg_analysis64(const hb_plan *p, int nmaps, const double2 *F, double2 *alm, cudaStream_t st, int nm,
+                          const int32_t *mlist) {
+    const LegArgs L{p, mlist ? nm : p->mmax + 1, mlist, st};
+    const int64_t fs = L.f_stride(), as = L.a_stride();
+    return by_two(nmaps, [&](int nz, int b) { return analysis_nb<2>(L, nz, F + b * fs, alm + b * as); },
+                  [&](int nz, int b) { return analysis_nb<1>(L, nz, F + b * fs, alm + b * as); });
 }
 
-int launch_leg_analysis(const GeomDev &g, int precision, int nmaps, int lmax, int mmax, const void *Fm, void *alm,
-                        cudaStream_t st, const float4 *ck, const int64_t *bo, int nm, const int32_t *mlist) {
-    HB_NVTX("legendre_analysis");
-    if (precision == 32)
-        return analysis_t<float>(g, nmaps, lmax, mmax, nm, mlist, (const float2 *)Fm, (float2 *)alm, st, ck, bo);
-    return analysis_t<double>(g, nmaps, lmax, mmax, nm, mlist, (const double2 *)Fm, (double2 *)alm, st, nullptr,
-                              nullptr);
-}
-
-int launch_leg_synthesis(const GeomDev &g, int precision, int nmaps, int lmax, int mmax, const void *alm, void *Gm,
-                         cudaStream_t st, const float4 *ck, const int64_t *bo, int nm, const int32_t *mlist) {
-    HB_NVTX("legendre_synthesis");
-    if (precision == 32)
-        return synthesis_t<float>(g, nmaps, lmax, mmax, nm, mlist, (const float2 *)alm, (float2 *)Gm, st, ck, bo);
-    return synthesis_t<double>(g, nmaps, lmax, mmax, nm, mlist, (const double2 *)alm, (double2 *)Gm, st, nullptr,
-                               nullptr);
+int launch_leg_synthesis64(const hb_plan *p, int nmaps, const double2 *alm, double2 *G, cudaStream_t st, int nm,
+                           const int32_t *mlist) {
+    const LegArgs L{p, mlist ? nm : p->mmax + 1, mlist, st};
+    const int64_t fs = L.f_stride(), as = L.a_stride();
+    return by_two(nmaps, [&](int nz, int b) { return synthesis_nb<2>(L, nz, alm + b * as, G + b * fs); },
+                  [&](int nz, int b) { return synthesis_nb<1>(L, nz, alm + b * as, G + b * fs); });
 }
 
 }  // namespace hb

@@ -12,6 +12,12 @@
 //
 // Layout: ck[(blk_ofs[m] + j) * npairs + p] = float4(mu1, mu2, bits(e), 0) for block j of m
 // (block j starts at l = m + j*R for the scalar recursion, at l = max(m,2) + j*R for spin-2).
+// Each row of the scalar table has a flag byte per 64 pairs (hb_internal.cuh) by which the FP32
+// kernels skip blocks that stay evanescent.
+//
+// Every plan also holds the FP64 coefficient tables of the scalar recursions (LegTab): their scale
+// factors are products over l, which a kernel would have to rebuild per CTA (48 bytes per (l, m),
+// 0.4 GB at lmax 4095).  FP32 plans hold the one-step coefficients (8 bytes per (l, m)).
 #include <cmath>
 #include <vector>
 
@@ -40,16 +46,64 @@ __device__ __forceinline__ float4 to_f32_state(double v1, double v2, int e) {
     return make_float4((float)ldexp(v1, shi), (float)ldexp(v2, shi), __int_as_float(ef), 0.f);
 }
 
+// eps_l = sqrt((l^2 - m^2) / (4 l^2 - 1))
+__device__ __forceinline__ double leg_eps(int l, int m) {
+    const double ll = l, mm = m;
+    return sqrt((ll - mm) * (ll + mm) / ((2.0 * ll - 1.0) * (2.0 * ll + 1.0)));
+}
+
+// LegTab rows of one order per thread.  N_k and M_l follow from their neighbours' products
+// N_k N_{k+1} eps_{l+2} eps_{l+3} = 1/4 and M_l M_{l+1} eps_{l+1} = 1/2; the free first values are
+// the smooth ones, so that both stay of order one.
+__global__ void leg_table_kernel(int lmax, int mmax, LegTab tb) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m > mmax) return;
+    double e1 = leg_eps(m + 1, m), e2 = leg_eps(m + 2, m);
+    double N = sqrt(0.25 / (e1 * e2)), M = sqrt(0.5 / e1), Mprev = 0.0;
+    double *t = tb.row(m, 0);
+    for (int k = 0, l = m; l <= lmax; ++k, l += 2, t += LT_N) {
+        const double e3 = leg_eps(l + 3, m), a = 4.0 * N * N, M1 = 0.5 / (e1 * M), sg = (k & 1) ? -1.0 : 1.0;
+        t[LT_A] = a;
+        t[LT_G] = a * (1.0 - e1 * e1 - e2 * e2) - 2.0;
+        t[LT_P] = N * e1;
+        t[LT_Q] = l + 2 <= lmax ? N * e2 : 0.0;
+        t[LT_NX] = l + 1 <= lmax ? N : 0.0;
+        t[LT_B0] = -2.0 * Mprev * Mprev;
+        t[LT_B1] = 2.0 * M * M;
+        t[LT_M0] = sg * M;
+        t[LT_M1] = sg * M1;
+        for (int i = LT_NX + 1; i < LT_N; ++i) t[i] = 0.0;
+        N = 0.25 / (e2 * e3 * N);
+        Mprev = M1;
+        M = 0.5 / (e2 * M1);
+        e1 = e3;
+        e2 = leg_eps(l + 4, m);
+    }
+}
+
 constexpr int CKR = 256;   // checkpoint block length (== COEF_CH of the Legendre kernels)
 constexpr int CK_NT = 128;
 
-// ck (may be null): states at the block starts; ck_mid (may be null): states at l0 + R/2 of every
-// block that reaches that far, same indexing.
-// states at the start of every CKR-l block (ck), and optionally at its quarter points
-// l0 + CKR/4 (ck_q1), l0 + CKR/2 (ck_mid) and l0 + 3 CKR/4 (ck_q3), same indexing; a state past
-// lmax is not written
+// (A_l, B_l) of the FP32 kernels, zero past lmax; l = m gives (0, 1): the first block's state is
+// (0, lambda_mm)
+__global__ void leg32_coef_kernel(int lmax, const int64_t *__restrict__ blk_ofs, float2 *__restrict__ tab) {
+    const int m = blockIdx.x;
+    float2 *t = tab + blk_ofs[m] * CKR;
+    const int64_t n = (blk_ofs[m + 1] - blk_ofs[m]) * CKR;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+        double A = 0.0, B = i == 0 ? 1.0 : 0.0;
+        if (i > 0 && m + i <= lmax) ck_scalar_coef(m + (int)i, m, A, B);
+        t[i] = make_float2((float)A, (float)B);
+    }
+}
+
+
+// states at the start of every CKR-l block (ck, with its flags per 64 pairs), and optionally at its
+// quarter points l0 + CKR/4 (ck_q1), l0 + CKR/2 (ck_mid) and l0 + 3 CKR/4 (ck_q3), same indexing; a
+// state past lmax is not written
 __global__ void __launch_bounds__(CK_NT) ck_scalar_kernel(GeomDev g, int lmax, const int64_t *__restrict__ blk_ofs,
-                                                          float4 *__restrict__ ck, float4 *__restrict__ ck_mid,
+                                                          float4 *__restrict__ ck,
+                                                          uint8_t *__restrict__ flags, float4 *__restrict__ ck_mid,
                                                           float4 *__restrict__ ck_q1 = nullptr,
                                                           float4 *__restrict__ ck_q3 = nullptr) {
     const int m = blockIdx.x;
@@ -63,22 +117,25 @@ __global__ void __launch_bounds__(CK_NT) ck_scalar_kernel(GeomDev g, int lmax, c
     double l1 = 0.0, l2 = exp2(L - 512.0 * e);
     if (m & 1) l2 = -l2;
     const int64_t o = blk_ofs[m] * np;
+    __shared__ int any_neg[CK_NT / 64], any_live[CK_NT / 64];
+    const int64_t fstride = flag_stride(np);
     for (int l0 = m; l0 <= lmax; l0 += CKR) {
         const int64_t oj = o + (int64_t)((l0 - m) / CKR) * np + p;
-        // state at the start of this block: (lambda_{l0-1}, lambda_{l0-2}); block 0 holds (0, lambda_mm)
-        if (live && ck) ck[oj] = to_f32_state(l1, l2, e);
         __syncthreads();
         for (int i = threadIdx.x; i < CKR; i += CK_NT) {
             int l = l0 + i;
-            double A = 0.0, B = 0.0;
-            if (l == m) {
-                B = 1.0;
-            } else if (l <= lmax) {
-                ck_scalar_coef(l, m, A, B);
-            }
+            double A = 0.0, B = 1.0;
+            if (l > m && l <= lmax) ck_scalar_coef(l, m, A, B);
             cf[i] = make_double2(A, B);
         }
+        if (threadIdx.x < CK_NT / 64) any_neg[threadIdx.x] = any_live[threadIdx.x] = 0;
         __syncthreads();
+        // state at the start of this block: (lambda_{l0-1}, lambda_{l0-2}); block 0 holds (0, lambda_mm)
+        if (live && ck) {
+            const float4 st = to_f32_state(l1, l2, e);
+            ck[oj] = st;
+            if (__float_as_int(st.z) < 0) any_neg[threadIdx.x / 64] = 1;
+        }
         const int n = min(CKR, lmax - l0 + 1);
         for (int i = 0; i < n; ++i) {
             if (i == CKR / 2 && live && ck_mid) ck_mid[oj] = to_f32_state(l1, l2, e);
@@ -92,6 +149,16 @@ __global__ void __launch_bounds__(CK_NT) ck_scalar_kernel(GeomDev g, int lmax, c
                 l2 *= 0x1p-512;
                 ++e;
             }
+        }
+        if (flags) {
+            // by the larger of the last two values: one alone can be near zero on an oscillating pair
+            if (live && __float_as_int(to_f32_state(fmax(fabs(l1), fabs(l2)), 0.0, e).z) >= 0) any_live[threadIdx.x / 64] = 1;
+            __syncthreads();
+            // the last CTA of a row also fills its padding
+            const int64_t unit = blockIdx.y * (CK_NT / 64) + threadIdx.x;
+            if (unit < fstride && (threadIdx.x < CK_NT / 64 || blockIdx.y == gridDim.y - 1))
+                flags[(blk_ofs[m] + (l0 - m) / CKR) * fstride + unit] =
+                    threadIdx.x >= CK_NT / 64 || !any_live[threadIdx.x] ? FL_DEAD : (any_neg[threadIdx.x] ? FL_MIXED : FL_CLEAN);
         }
     }
 }
@@ -155,7 +222,7 @@ __global__ void __launch_bounds__(CK_NT) ck_spin_kernel(GeomDev g, int lmax, con
 int launch_ck_mid(const hb_plan *p, float4 *ck_mid, float4 *ck_q1, float4 *ck_q3) {
     const int64_t np = p->g->d.npairs;
     dim3 grid((unsigned)(p->mmax + 1), (unsigned)((np + CK_NT - 1) / CK_NT));
-    ck_scalar_kernel<<<grid, CK_NT>>>(p->g->d, p->lmax, p->blk_ofs, nullptr, ck_mid, ck_q1, ck_q3);
+    ck_scalar_kernel<<<grid, CK_NT>>>(p->g->d, p->lmax, p->blk_ofs, nullptr, nullptr, ck_mid, ck_q1, ck_q3);
     HB_CUDA_TRY(cudaGetLastError());
     return HB_OK;
 }
@@ -178,16 +245,20 @@ int hb_plan_create(const hb_geom *g, int lmax, int mmax, int flags, hb_plan **ou
     p->mmax = mmax;
     p->flags = flags;
     const int64_t np = g->d.npairs;
-    std::vector<int64_t> ofs(mmax + 2), ofs_s(mmax + 2);
-    ofs[0] = ofs_s[0] = 0;
+    std::vector<int64_t> ofs(mmax + 2), ofs_s(mmax + 2), ofs_t(mmax + 2);
+    ofs[0] = ofs_s[0] = ofs_t[0] = 0;
     for (int m = 0; m <= mmax; ++m) {
         ofs[m + 1] = ofs[m] + nblk(lmax, m);
         ofs_s[m + 1] = ofs_s[m] + nblk(lmax, m > 2 ? m : 2);
+        ofs_t[m + 1] = ofs_t[m] + (lmax - m) / 2 + 1;
     }
     const bool scalar = (flags & HB_PLAN_FP32) != 0, spin = (flags & HB_PLAN_SPIN2_FP32) != 0;
     size_t bytes = 0;
     auto carve = [&](size_t b) { size_t o = bytes; bytes += (b + 255) & ~(size_t)255; return o; };
-    size_t o_ofs = carve(8 * (mmax + 2)), o_ofss = carve(8 * (mmax + 2));
+    size_t o_ofs = carve(8 * (mmax + 2)), o_ofss = carve(8 * (mmax + 2)), o_ofst = carve(8 * (mmax + 2));
+    const size_t o_leg = carve(8 * LT_N * (size_t)ofs_t[mmax + 1]);
+    const size_t o_flags = scalar ? carve((size_t)ofs[mmax + 1] * flag_stride(np)) : 0;
+    const size_t o_leg32 = scalar ? carve(8 * (size_t)ofs[mmax + 1] * CKR) : 0;
     size_t o_ck = scalar ? carve(16 * (size_t)ofs[mmax + 1] * np) : 0;
     size_t o_ckp = spin ? carve(16 * (size_t)ofs_s[mmax + 1] * np) : 0;
     size_t o_ckm = spin ? carve(16 * (size_t)ofs_s[mmax + 1] * np) : 0;
@@ -201,16 +272,25 @@ int hb_plan_create(const hb_geom *g, int lmax, int mmax, int flags, hb_plan **ou
     p->bytes = bytes;
     p->blk_ofs = (int64_t *)(base + o_ofs);
     p->blk_ofs_spin = (int64_t *)(base + o_ofss);
+    p->leg = {(double *)(base + o_leg), (int64_t *)(base + o_ofst)};
+    p->leg32 = scalar ? (float2 *)(base + o_leg32) : nullptr;
+    p->ck_flags = scalar ? (uint8_t *)(base + o_flags) : nullptr;
     p->ck = scalar ? (float4 *)(base + o_ck) : nullptr;
     p->ckP = spin ? (float4 *)(base + o_ckp) : nullptr;
     p->ckM = spin ? (float4 *)(base + o_ckm) : nullptr;
     int rc = HB_OK;
     if (cudaMemcpy(p->blk_ofs, ofs.data(), 8 * (mmax + 2), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(p->blk_ofs_spin, ofs_s.data(), 8 * (mmax + 2), cudaMemcpyHostToDevice) != cudaSuccess)
+        cudaMemcpy(p->blk_ofs_spin, ofs_s.data(), 8 * (mmax + 2), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(p->leg.ofs, ofs_t.data(), 8 * (mmax + 2), cudaMemcpyHostToDevice) != cudaSuccess)
         rc = fail(HB_ERR_CUDA, "hb_plan_create: upload failed");
     dim3 grid((unsigned)(mmax + 1), (unsigned)((np + CK_NT - 1) / CK_NT));
+    if (rc == HB_OK) {
+        leg_table_kernel<<<(unsigned)(mmax / 32 + 1), 32>>>(lmax, mmax, p->leg);
+        if (scalar) leg32_coef_kernel<<<(unsigned)(mmax + 1), 256>>>(lmax, p->blk_ofs, p->leg32);
+        if (cudaGetLastError() != cudaSuccess) rc = fail(HB_ERR_CUDA, "hb_plan_create: table kernel launch");
+    }
     if (rc == HB_OK && scalar) {
-        ck_scalar_kernel<<<grid, CK_NT>>>(g->d, lmax, p->blk_ofs, p->ck, nullptr);
+        ck_scalar_kernel<<<grid, CK_NT>>>(g->d, lmax, p->blk_ofs, p->ck, p->ck_flags, nullptr);
         if (cudaGetLastError() != cudaSuccess) rc = fail(HB_ERR_CUDA, "hb_plan_create: checkpoint kernel launch");
     }
     if (rc == HB_OK && spin) {

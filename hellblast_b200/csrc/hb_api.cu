@@ -30,7 +30,6 @@ static int check_ws(void *ws, size_t have, size_t need, const char *who) {
     return HB_OK;
 }
 
-#define HB_PLAN_ARGS(p) (p)->g->d, prec, nmaps, (p)->lmax, (p)->mmax
 
 static int map2alm_impl(const hb_plan *p, int nmaps, const void *maps, const double *w, void *alm, void *ws,
                         size_t wsb, int flags, cudaStream_t st, int prec, const char *who) {
@@ -101,8 +100,7 @@ static int map2alm_spin_impl(const hb_plan *p, int nmaps, const void *Q, const v
     if ((rc = launch_ring_analysis(d, prec, nmaps, U, d.npix, wr, UF, p->mmax, f, adjoint_of_synth, adjoint_of_synth,
                                    st)))
         return rc;
-    return launch_spin_analysis(HB_PLAN_ARGS(p), QF, UF, E, B, st, prec == 32 ? p->ckP : nullptr,
-                                prec == 32 ? p->ckM : nullptr, p->blk_ofs_spin);
+    return launch_spin_analysis(p, prec, nmaps, QF, UF, E, B, st);
 }
 
 // spin-2 synthesis; with adjoint_of_anal the ring synthesis applies the pixel weights and c_m = 1
@@ -119,8 +117,7 @@ static int alm2map_spin_impl(const hb_plan *p, int nmaps, const void *E, const v
     if ((rc = check_ws(ws, wsb, 2 * half, who))) return rc;
     const GeomDev &d = p->g->d;
     char *QG = (char *)ws, *UG = (char *)ws + half;
-    if ((rc = launch_spin_synthesis(HB_PLAN_ARGS(p), E, B, QG, UG, st, prec == 32 ? p->ckP : nullptr,
-                                    prec == 32 ? p->ckM : nullptr, p->blk_ofs_spin)))
+    if ((rc = launch_spin_synthesis(p, prec, nmaps, E, B, QG, UG, st)))
         return rc;
     if ((rc = launch_ring_synthesis(d, prec, nmaps, QG, p->mmax, Q, d.npix, w, adjoint_of_anal, !adjoint_of_anal, flags,
                                     st)))

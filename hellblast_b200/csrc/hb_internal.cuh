@@ -180,6 +180,8 @@ struct hb_plan {
     uint8_t *ck_flags;      // [blocks][flag_stride] FL_CLEAN: the 64 pairs start the block with e = 0, FL_MIXED: some
                             // e < 0, FL_DEAD: all end the block with e < 0 (evanescent throughout)
     float4 *ckP, *ckM;      // spin-2 checkpoints, or null
+    uint8_t *ck_flags_spin;  // as ck_flags (a pair is live when P or M is)
+    float4 *spin32;         // (a, b, c, 0) of the spin-2 recursions, [blk_ofs_spin[m] * 256 + l - max(m, 2)]
 };
 
 namespace hb {
@@ -210,12 +212,10 @@ int launch_leg_analysis(const hb_plan *p, int precision, int nmaps, const void *
                         const int32_t *mlist = nullptr);
 int launch_leg_synthesis(const hb_plan *p, int precision, int nmaps, const void *alm, void *Gm, cudaStream_t st, int nm = 0,
                          const int32_t *mlist = nullptr);
-int launch_spin_analysis(const GeomDev &g, int precision, int nmaps, int lmax, int mmax, const void *QFm,
-                         const void *UFm, void *E, void *B, cudaStream_t st, const float4 *ckP, const float4 *ckM,
-                         const int64_t *blk_ofs);
-int launch_spin_synthesis(const GeomDev &g, int precision, int nmaps, int lmax, int mmax, const void *E,
-                          const void *B, void *QGm, void *UGm, cudaStream_t st, const float4 *ckP,
-                          const float4 *ckM, const int64_t *blk_ofs);
+int launch_spin_analysis(const hb_plan *p, int precision, int nmaps, const void *QFm, const void *UFm, void *E, void *B,
+                         cudaStream_t st);
+int launch_spin_synthesis(const hb_plan *p, int precision, int nmaps, const void *E, const void *B, void *QGm, void *UGm,
+                          cudaStream_t st);
 // FFT twiddle table and Bluestein chirp spectra of a geometry
 int build_fft_tables(GeomDev &g, cudaStream_t st);
 // pair-packed FP32 ring FFTs (hb_ringpack.cu) over the geometry's pk_* pairs

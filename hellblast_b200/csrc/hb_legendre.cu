@@ -477,18 +477,21 @@ template <int NB> static int synthesis_nb(const LegArgs &L, int nz, const double
     return run_synthesis<1, NB, 16>(L, nz, alm, G);
 }
 
-// maps in pairs that share one recursion: 11 operations per (two l, ring pair) for two maps, 7 for one
-template <typename Fn2, typename Fn1> static int by_two(int nmaps, Fn2 f2, Fn1 f1) {
-    if (nmaps >= 2)
-        if (int rc = f2(nmaps / 2, 0)) return rc;
-    return nmaps % 2 ? f1(1, nmaps - 1) : HB_OK;
+// Maps in pairs that share one recursion: 11 operations per (two l, ring pair) for two maps, 7 for one.
+// Below 256 pairs one launch of single maps: these are bound by latency (3 maps at nside 64, lmax 100:
+// 6 us, 9 us as a pair and a single).
+template <typename Fn2, typename Fn1> static int by_two(int nmaps, int64_t np, Fn2 f2, Fn1 f1) {
+    const int n2 = np >= 256 ? nmaps / 2 : 0;
+    if (n2)
+        if (int rc = f2(n2, 0)) return rc;
+    return nmaps > 2 * n2 ? f1(nmaps - 2 * n2, 2 * n2) : HB_OK;
 }
 
 int launch_leg_analysis64(const hb_plan *p, int nmaps, const double2 *F, double2 *alm, cudaStream_t st, int nm,
                           const int32_t *mlist) {
     const LegArgs L{p, mlist ? nm : p->mmax + 1, mlist, st};
     const int64_t fs = L.f_stride(), as = L.a_stride();
-    return by_two(nmaps, [&](int nz, int b) { return analysis_nb<2>(L, nz, F + b * fs, alm + b * as); },
+    return by_two(nmaps, L.np(), [&](int nz, int b) { return analysis_nb<2>(L, nz, F + b * fs, alm + b * as); },
                   [&](int nz, int b) { return analysis_nb<1>(L, nz, F + b * fs, alm + b * as); });
 }
 
@@ -496,7 +499,7 @@ int launch_leg_synthesis64(const hb_plan *p, int nmaps, const double2 *alm, doub
                            const int32_t *mlist) {
     const LegArgs L{p, mlist ? nm : p->mmax + 1, mlist, st};
     const int64_t fs = L.f_stride(), as = L.a_stride();
-    return by_two(nmaps, [&](int nz, int b) { return synthesis_nb<2>(L, nz, alm + b * as, G + b * fs); },
+    return by_two(nmaps, L.np(), [&](int nz, int b) { return synthesis_nb<2>(L, nz, alm + b * as, G + b * fs); },
                   [&](int nz, int b) { return synthesis_nb<1>(L, nz, alm + b * as, G + b * fs); });
 }
 

@@ -471,19 +471,25 @@ template <int NB> static int synthesis_nb(const Leg32 &L, int nz, const float2 *
     return run_synthesis<1, NB, 20>(L, nz, alm, G);
 }
 
+// Maps in pairs that share one recursion; below 256 ring pairs one launch of single maps, which are
+// bound by latency there.
+template <typename Fn2, typename Fn1> static int by_two(int nmaps, int64_t np, Fn2 f2, Fn1 f1) {
+    const int n2 = np >= 256 ? nmaps / 2 : 0;
+    if (n2)
+        if (int rc = f2(n2, 0)) return rc;
+    return nmaps > 2 * n2 ? f1(nmaps - 2 * n2, 2 * n2) : HB_OK;
+}
 static int analysis32(const hb_plan *p, int nmaps, const float2 *F, float2 *alm, cudaStream_t st, int nm, const int32_t *mlist) {
     const Leg32 L{p, mlist ? nm : p->mmax + 1, mlist, st};
-    const int n2 = nmaps / 2;
-    if (n2)
-        if (int rc = analysis_nb<2>(L, n2, F, alm)) return rc;
-    return nmaps % 2 ? analysis_nb<1>(L, 1, F + 2 * n2 * L.f_stride(), alm + 2 * n2 * L.a_stride()) : HB_OK;
+    const int64_t fs = L.f_stride(), as = L.a_stride();
+    return by_two(nmaps, L.np(), [&](int nz, int b) { return analysis_nb<2>(L, nz, F + b * fs, alm + b * as); },
+                  [&](int nz, int b) { return analysis_nb<1>(L, nz, F + b * fs, alm + b * as); });
 }
 static int synthesis32(const hb_plan *p, int nmaps, const float2 *alm, float2 *G, cudaStream_t st, int nm, const int32_t *mlist) {
     const Leg32 L{p, mlist ? nm : p->mmax + 1, mlist, st};
-    const int n2 = nmaps / 2;
-    if (n2)
-        if (int rc = synthesis_nb<2>(L, n2, alm, G)) return rc;
-    return nmaps % 2 ? synthesis_nb<1>(L, 1, alm + 2 * n2 * L.a_stride(), G + 2 * n2 * L.f_stride()) : HB_OK;
+    const int64_t fs = L.f_stride(), as = L.a_stride();
+    return by_two(nmaps, L.np(), [&](int nz, int b) { return synthesis_nb<2>(L, nz, alm + b * as, G + b * fs); },
+                  [&](int nz, int b) { return synthesis_nb<1>(L, nz, alm + b * as, G + b * fs); });
 }
 
 int launch_leg_analysis64(const hb_plan *p, int nmaps, const double2 *F, double2 *alm, cudaStream_t st, int nm,

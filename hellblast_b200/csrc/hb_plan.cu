@@ -98,6 +98,15 @@ __global__ void leg32_coef_kernel(int lmax, const int64_t *__restrict__ blk_ofs,
 }
 
 
+// one row of the flag table: the CTA's CK_NT / 64 units, the last CTA of a row also its padding
+__device__ __forceinline__ void write_flags(uint8_t *flags, int64_t row, int64_t np, const int *any_neg, const int *any_live) {
+    const int64_t stride = flag_stride(np), unit = (int64_t)blockIdx.y * (CK_NT / 64) + threadIdx.x;
+    if (unit < stride && (threadIdx.x < CK_NT / 64 || blockIdx.y == gridDim.y - 1))
+        flags[row * stride + unit] = threadIdx.x >= CK_NT / 64 || !any_live[threadIdx.x] ? FL_DEAD
+                                     : any_neg[threadIdx.x]                              ? FL_MIXED
+                                                                                         : FL_CLEAN;
+}
+
 // states at the start of every CKR-l block (ck, with its flags per 64 pairs), and optionally at its
 // quarter points l0 + CKR/4 (ck_q1), l0 + CKR/2 (ck_mid) and l0 + 3 CKR/4 (ck_q3), same indexing; a
 // state past lmax is not written
@@ -118,7 +127,6 @@ __global__ void __launch_bounds__(CK_NT) ck_scalar_kernel(GeomDev g, int lmax, c
     if (m & 1) l2 = -l2;
     const int64_t o = blk_ofs[m] * np;
     __shared__ int any_neg[CK_NT / 64], any_live[CK_NT / 64];
-    const int64_t fstride = flag_stride(np);
     for (int l0 = m; l0 <= lmax; l0 += CKR) {
         const int64_t oj = o + (int64_t)((l0 - m) / CKR) * np + p;
         __syncthreads();
@@ -154,11 +162,7 @@ __global__ void __launch_bounds__(CK_NT) ck_scalar_kernel(GeomDev g, int lmax, c
             // by the larger of the last two values: one alone can be near zero on an oscillating pair
             if (live && __float_as_int(to_f32_state(fmax(fabs(l1), fabs(l2)), 0.0, e).z) >= 0) any_live[threadIdx.x / 64] = 1;
             __syncthreads();
-            // the last CTA of a row also fills its padding
-            const int64_t unit = blockIdx.y * (CK_NT / 64) + threadIdx.x;
-            if (unit < fstride && (threadIdx.x < CK_NT / 64 || blockIdx.y == gridDim.y - 1))
-                flags[(blk_ofs[m] + (l0 - m) / CKR) * fstride + unit] =
-                    threadIdx.x >= CK_NT / 64 || !any_live[threadIdx.x] ? FL_DEAD : (any_neg[threadIdx.x] ? FL_MIXED : FL_CLEAN);
+            write_flags(flags, blk_ofs[m] + (l0 - m) / CKR, np, any_neg, any_live);
         }
     }
 }
@@ -174,8 +178,22 @@ __device__ __forceinline__ void ck_spin_coef(int lp, int m, double &a, double &b
     c = n1m * (l + 1) * R0 / (l * R1);
 }
 
+// (a, b, c) of the FP32 kernels, zero past lmax; l = max(m, 2) gives (0, 0, -1): the first block's
+// state is (0, start value)
+__global__ void spin32_coef_kernel(int lmax, const int64_t *__restrict__ blk_ofs, float4 *__restrict__ tab) {
+    const int m = blockIdx.x, l0 = m > 2 ? m : 2;
+    float4 *t = tab + blk_ofs[m] * CKR;
+    const int64_t n = (blk_ofs[m + 1] - blk_ofs[m]) * CKR;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+        double a = 0.0, b = 0.0, c = i == 0 ? -1.0 : 0.0;
+        if (i > 0 && l0 + i <= lmax) ck_spin_coef(l0 + (int)i, m, a, b, c);
+        t[i] = make_float4((float)a, (float)b, (float)c, 0.f);
+    }
+}
+
 __global__ void __launch_bounds__(CK_NT) ck_spin_kernel(GeomDev g, int lmax, const int64_t *__restrict__ blk_ofs,
-                                                        float4 *__restrict__ ckP, float4 *__restrict__ ckM) {
+                                                        float4 *__restrict__ ckP, float4 *__restrict__ ckM,
+                                                        uint8_t *__restrict__ flags) {
     const int m = blockIdx.x;
     const int64_t p = (int64_t)blockIdx.y * CK_NT + threadIdx.x;
     __shared__ double4 cf[CKR];
@@ -190,12 +208,17 @@ __global__ void __launch_bounds__(CK_NT) ck_spin_kernel(GeomDev g, int lmax, con
     double sp = (m & 1) ? -1.0 : 1.0, sm = (m >= 2) ? sp : 1.0;
     double P1 = 0.0, P2 = sp * exp2(LP - 512.0 * ep), M1 = 0.0, M2 = sm * exp2(LM - 512.0 * em);
     float4 *oP = ckP + blk_ofs[m] * np, *oM = ckM + blk_ofs[m] * np;
+    __shared__ int any_neg[CK_NT / 64], any_live[CK_NT / 64];
     for (int lb = l0s; lb <= lmax; lb += CKR) {
-        if (live) {
-            oP[(int64_t)((lb - l0s) / CKR) * np + p] = to_f32_state(P1, P2, ep);
-            oM[(int64_t)((lb - l0s) / CKR) * np + p] = to_f32_state(M1, M2, em);
-        }
         __syncthreads();
+        if (threadIdx.x < CK_NT / 64) any_neg[threadIdx.x] = any_live[threadIdx.x] = 0;
+        __syncthreads();
+        if (live) {
+            const float4 sP = to_f32_state(P1, P2, ep), sM = to_f32_state(M1, M2, em);
+            oP[(int64_t)((lb - l0s) / CKR) * np + p] = sP;
+            oM[(int64_t)((lb - l0s) / CKR) * np + p] = sM;
+            if (__float_as_int(sP.z) < 0 || __float_as_int(sM.z) < 0) any_neg[threadIdx.x / 64] = 1;
+        }
         for (int i = threadIdx.x; i < CKR; i += CK_NT) {
             int lp = lb + i;
             double a = 0.0, b = 0.0, c = 0.0;
@@ -216,6 +239,11 @@ __global__ void __launch_bounds__(CK_NT) ck_spin_kernel(GeomDev g, int lmax, con
             if (ep < 0 && fabs(P1) > 0x1p256) { P1 *= 0x1p-512; P2 *= 0x1p-512; ++ep; }
             if (em < 0 && fabs(M1) > 0x1p256) { M1 *= 0x1p-512; M2 *= 0x1p-512; ++em; }
         }
+        if (live && (__float_as_int(to_f32_state(fmax(fabs(P1), fabs(P2)), 0.0, ep).z) >= 0 ||
+                     __float_as_int(to_f32_state(fmax(fabs(M1), fabs(M2)), 0.0, em).z) >= 0))
+            any_live[threadIdx.x / 64] = 1;
+        __syncthreads();
+        write_flags(flags, blk_ofs[m] + (lb - l0s) / CKR, np, any_neg, any_live);
     }
 }
 
@@ -260,6 +288,8 @@ int hb_plan_create(const hb_geom *g, int lmax, int mmax, int flags, hb_plan **ou
     const size_t o_flags = scalar ? carve((size_t)ofs[mmax + 1] * flag_stride(np)) : 0;
     const size_t o_leg32 = scalar ? carve(8 * (size_t)ofs[mmax + 1] * CKR) : 0;
     size_t o_ck = scalar ? carve(16 * (size_t)ofs[mmax + 1] * np) : 0;
+    const size_t o_spin32 = spin ? carve(16 * (size_t)ofs_s[mmax + 1] * CKR) : 0;
+    const size_t o_flags_s = spin ? carve((size_t)ofs_s[mmax + 1] * flag_stride(np)) : 0;
     size_t o_ckp = spin ? carve(16 * (size_t)ofs_s[mmax + 1] * np) : 0;
     size_t o_ckm = spin ? carve(16 * (size_t)ofs_s[mmax + 1] * np) : 0;
     char *base = nullptr;
@@ -276,6 +306,8 @@ int hb_plan_create(const hb_geom *g, int lmax, int mmax, int flags, hb_plan **ou
     p->leg32 = scalar ? (float2 *)(base + o_leg32) : nullptr;
     p->ck_flags = scalar ? (uint8_t *)(base + o_flags) : nullptr;
     p->ck = scalar ? (float4 *)(base + o_ck) : nullptr;
+    p->spin32 = spin ? (float4 *)(base + o_spin32) : nullptr;
+    p->ck_flags_spin = spin ? (uint8_t *)(base + o_flags_s) : nullptr;
     p->ckP = spin ? (float4 *)(base + o_ckp) : nullptr;
     p->ckM = spin ? (float4 *)(base + o_ckm) : nullptr;
     int rc = HB_OK;
@@ -294,7 +326,8 @@ int hb_plan_create(const hb_geom *g, int lmax, int mmax, int flags, hb_plan **ou
         if (cudaGetLastError() != cudaSuccess) rc = fail(HB_ERR_CUDA, "hb_plan_create: checkpoint kernel launch");
     }
     if (rc == HB_OK && spin) {
-        ck_spin_kernel<<<grid, CK_NT>>>(g->d, lmax, p->blk_ofs_spin, p->ckP, p->ckM);
+        spin32_coef_kernel<<<(unsigned)(mmax + 1), 256>>>(lmax, p->blk_ofs_spin, p->spin32);
+        ck_spin_kernel<<<grid, CK_NT>>>(g->d, lmax, p->blk_ofs_spin, p->ckP, p->ckM, p->ck_flags_spin);
         if (cudaGetLastError() != cudaSuccess) rc = fail(HB_ERR_CUDA, "hb_plan_create: spin checkpoint kernel launch");
     }
     if (rc == HB_OK && cudaDeviceSynchronize() != cudaSuccess) rc = fail(HB_ERR_CUDA, "hb_plan_create: table build failed");

@@ -489,23 +489,22 @@ static int spin_synthesis_t(const GeomDev &g, int nmaps, int lmax, int mmax, con
     return run_spin_synthesis<T, 1, 64>(g, nmaps, lmax, mmax, E, B, QG, UG, st, ckP, ckM, bo);
 }
 
-int launch_spin_analysis(const GeomDev &g, int precision, int nmaps, int lmax, int mmax, const void *QFm,
-                         const void *UFm, void *E, void *B, cudaStream_t st, const float4 *ckP, const float4 *ckM,
-                         const int64_t *bo) {
+int launch_spin_analysis32(const hb_plan *p, int nmaps, const float2 *QF, const float2 *UF, float2 *E, float2 *B, cudaStream_t st);
+int launch_spin_synthesis32(const hb_plan *p, int nmaps, const float2 *E, const float2 *B, float2 *QG, float2 *UG, cudaStream_t st);
+
+int launch_spin_analysis(const hb_plan *p, int precision, int nmaps, const void *QFm, const void *UFm, void *E, void *B,
+                         cudaStream_t st) {
     if (precision == 32)
-        return spin_analysis_t<float>(g, nmaps, lmax, mmax, (const float2 *)QFm, (const float2 *)UFm, (float2 *)E,
-                                      (float2 *)B, st, ckP, ckM, bo);
-    return spin_analysis_t<double>(g, nmaps, lmax, mmax, (const double2 *)QFm, (const double2 *)UFm, (double2 *)E,
+        return launch_spin_analysis32(p, nmaps, (const float2 *)QFm, (const float2 *)UFm, (float2 *)E, (float2 *)B, st);
+    return spin_analysis_t<double>(p->g->d, nmaps, p->lmax, p->mmax, (const double2 *)QFm, (const double2 *)UFm, (double2 *)E,
                                    (double2 *)B, st, nullptr, nullptr, nullptr);
 }
 
-int launch_spin_synthesis(const GeomDev &g, int precision, int nmaps, int lmax, int mmax, const void *E,
-                          const void *B, void *QGm, void *UGm, cudaStream_t st, const float4 *ckP,
-                          const float4 *ckM, const int64_t *bo) {
+int launch_spin_synthesis(const hb_plan *p, int precision, int nmaps, const void *E, const void *B, void *QGm, void *UGm,
+                          cudaStream_t st) {
     if (precision == 32)
-        return spin_synthesis_t<float>(g, nmaps, lmax, mmax, (const float2 *)E, (const float2 *)B, (float2 *)QGm,
-                                       (float2 *)UGm, st, ckP, ckM, bo);
-    return spin_synthesis_t<double>(g, nmaps, lmax, mmax, (const double2 *)E, (const double2 *)B, (double2 *)QGm,
+        return launch_spin_synthesis32(p, nmaps, (const float2 *)E, (const float2 *)B, (float2 *)QGm, (float2 *)UGm, st);
+    return spin_synthesis_t<double>(p->g->d, nmaps, p->lmax, p->mmax, (const double2 *)E, (const double2 *)B, (double2 *)QGm,
                                     (double2 *)UGm, st, nullptr, nullptr, nullptr);
 }
 

@@ -1,4 +1,4 @@
-"""GPU tests of the scalar Legendre kernels where their tiling can go wrong: block remainders in l,
+"""GPU tests of the Legendre kernels (scalar and spin-2) where their tiling can go wrong: block remainders in l,
 order cut-offs, odd numbers of maps, ring-pair counts around the sets a warp holds, rings in no
 particular order, pairs that are evanescent at every l; against the FP64 oracle.
 
@@ -60,3 +60,20 @@ def test_unsorted_rings(hb, oracle, nrings, lmax):
     _pair(hb, oracle, g, lmax, lmax, 1,
           lambda a, p: hb.alm2map_gpu(a[0], th, nphi, lmax, phi0=phi0, flat=True, precision=p)[None],
           lambda m, p: hb.map2alm_gpu(m[0], th, nphi, w, lmax, phi0=phi0, precision=p)[None], nrings)
+
+
+@pytest.mark.parametrize("nside,lmax,mmax,nmaps", [
+    (2, 1, 1, 1), (2, 2, 0, 2), (8, 257, 4, 1), (16, 258, 258, 2), (64, 130, 127, 3), (128, 300, 3, 1), (512, 40, 40, 2)])
+def test_spin_sizes(hb, oracle, nside, lmax, mmax, nmaps):
+    g = oracle.ring_tables(nside)
+    rng = np.random.default_rng(nside + lmax)
+    a = [_alm(oracle, rng, nmaps, lmax, mmax) for _ in range(2)]
+    q = [rng.standard_normal((nmaps, g["npix"])) for _ in range(2)]
+    ref_map = [oracle.alm2map_spin2(e, b, g, lmax, mmax) for e, b in zip(*a)]
+    ref_alm = [oracle.map2alm_spin2(x, y, g, lmax, mmax) for x, y in zip(*q)]
+    for prec, tol in (("fp64", 1e-10), ("fp32", 1e-5)):
+        got = hb.hp_compat.alm2map_spin(*(torch.from_numpy(x).cuda() for x in a), 2, nside=nside, lmax=lmax, mmax=mmax, precision=prec)
+        back = hb.hp_compat.map2alm_spin(*(torch.from_numpy(x).cuda() for x in q), 2, lmax=lmax, mmax=mmax, precision=prec)
+        for i in range(2):
+            assert rel2(got[i].double().cpu().numpy(), np.stack([r[i] for r in ref_map])) < tol, (prec, "map")
+            assert rel2(back[i].to(torch.complex128).cpu().numpy(), np.stack([r[i] for r in ref_alm])) < tol, (prec, "alm")

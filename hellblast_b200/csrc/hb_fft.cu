@@ -12,8 +12,12 @@
 // Work decomposition: one CTA per (ring pair, map), pairs fastest in the grid; it transforms
 // the pair's north ring, then its south ring, in one shared-memory buffer.  The analysis keeps
 // the north ring's F(m) in shared memory and writes each m's (north, south) entry as one vector
-// store, so two neighbouring CTAs fill each 32-byte sector of F.  Pairs are launched in classes
-// of equal convolution length, each class with its own shared-memory size.
+// store, so two neighbouring CTAs fill each 32-byte sector of F.  Pairs are grouped in classes of
+// equal convolution length.  The classes up to L = 1024 share one launch (longest rings first), the
+// longer ones, whose CTAs fill the GPU and want their own shared-memory size, have one each: a
+// small class's launch is bound by the latency of one CTA (12 us of table building and barriers),
+// so its time adds up over the classes.  One map, 7 and 8 launches merged into one: FP32 at nside
+// 1024 163 -> 35 us, FP64 at nside 64 100 -> 17 us (synthesis).
 //
 // FFT engine: a length L = 2^logL transform runs logL / 4 radix-16 stages and, when logL % 4 = r
 // is not zero, one radix-2^r stage.  Every stage is a pass in registers: each thread loads the
@@ -239,9 +243,16 @@ __device__ __forceinline__ int alias_sign(double phi0_pi, int n) {
 // small against the block, S = 2^j <= 32 neighbouring lanes share one k and each takes every
 // S-th alias m0 + q n of its residue classes, so the alias loops of the small polar rings
 // (up to mmax / n aliases per class) do not run on one thread each.
-__device__ __forceinline__ int lanes_per_bin(int K) {
+// The block counts as class_threads of the pair's class, whatever the launch has: the order of the
+// fold's sum depends on S.
+__host__ __device__ __forceinline__ int class_threads(int L) {  // one radix-16 butterfly per thread where the class allows
+    return L / 16 < 64 ? 64 : (L / 16 > 256 ? 256 : L / 16);
+}
+__device__ __forceinline__ int lanes_per_bin(const GeomDev &g, int pair, int K) {
+    const int rn = g.pair_ring[2 * pair], rs = g.pair_ring[2 * pair + 1];
+    const int nt = class_threads(max(rn >= 0 ? g.fft_len[rn] : 1, rs >= 0 ? g.fft_len[rs] : 1));
     int S = 1;
-    while (S < 32 && 2 * S * K <= (int)blockDim.x) S *= 2;
+    while (S < 32 && 2 * S * K <= nt) S *= 2;
     return S;
 }
 
@@ -367,7 +378,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
     V *buf = reinterpret_cast<V *>(smem_raw);
     V *tab = buf + padded_len(Lcls);
     V *stn = tab + trig_entries<T>(Lcls, mmax);  // north ring's F(m), m <= mmax (stage_n)
-    const int pair = pairs[blockIdx.x], b = blockIdx.y;  // pairs fastest: neighbours complete F's sectors
+    const int pair = pairs[gridDim.x - 1 - blockIdx.x], b = blockIdx.y;  // pairs fastest: neighbours complete F's sectors
     const int64_t np = g.npairs;
     V *out = Fm + b * fm_stride;
     auto slot = [&](int m) -> int64_t { return fg_off(m, pair, np, mblk != 0) * 2; };  // (north, south) of m
@@ -414,7 +425,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
         // exp(-i m0 phi0) s^j: one phase product per residue class m0 instead of one per alias.
         const bool nophase = flags & HB_F_NOPHASE;
         const int s = nophase ? 1 : alias_sign(g.phi0_pi[r], n);
-        const int K = N / 2 + 1, SL = lanes_per_bin(K), q0 = threadIdx.x & (SL - 1), kstep = blockDim.x / SL;
+        const int K = N / 2 + 1, SL = lanes_per_bin(g, pair, K), q0 = threadIdx.x & (SL - 1), kstep = blockDim.x / SL;
         auto emit_class = [&](int m0, V X) {  // aliases q = q0, q0 + S, ... of class m0
             const V Y = cscale(nophase ? X : cmul(X, R.P(m0)), scale);
             const V Yn = s > 0 ? Y : mk2(-Y.x, -Y.y);
@@ -463,7 +474,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
     V *buf = reinterpret_cast<V *>(smem_raw);
     V *tab = buf + padded_len(Lcls);
     V *ts = tab + trig_entries<T>(Lcls, mmax);  // staged G(m) of the current ring, m <= mmax (when stage_t)
-    const int pair = pairs[blockIdx.x], b = blockIdx.y;  // pairs fastest: neighbours share G's sectors
+    const int pair = pairs[gridDim.x - 1 - blockIdx.x], b = blockIdx.y;  // pairs fastest: neighbours share G's sectors
     const int64_t np = g.npairs;
     const V *gin = Gm + b * gm_stride;
     const Tw<T> tw = twiddles<T>(g);
@@ -505,7 +516,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
         // (HEALPix rings) that is exp(i m0 phi0) sum_j s^j G(m0 + j n): one add per alias.
         const bool nophase = flags & HB_F_NOPHASE;
         const int s = nophase ? 1 : alias_sign(g.phi0_pi[r], n);
-        const int K = N / 2 + 1, SL = lanes_per_bin(K), q0 = threadIdx.x & (SL - 1), kstep = blockDim.x / SL;
+        const int K = N / 2 + 1, SL = lanes_per_bin(g, pair, K), q0 = threadIdx.x & (SL - 1), kstep = blockDim.x / SL;
         // this lane's part of S(m0): aliases q = q0, q0 + SL, ..., before the factor exp(i m0 phi0)
         // when s != 0
         auto Ssum = [&](int m0) -> V {
@@ -753,8 +764,14 @@ static int sm_count() {
 // CTAs of `bytes` dynamic shared memory that fit on one SM (1 KB reserved per CTA)
 static int ctas_by_smem(size_t bytes) { return (int)((size_t)smem_per_sm() / (bytes + 1024)); }
 
-// one radix-16 butterfly per thread where the class allows, 64 to 256 threads
-static int class_threads(int L) { return std::max(64, std::min(256, L / 16)); }
+// Number of leading classes (ascending L) that share one launch (see the file comment); all of them
+// when their pairs are under two per SM
+int merged_classes(int ncls, const int *L, const int64_t *first) {
+    if (ncls > 0 && first[ncls] <= 2 * 148) return ncls;
+    int n = 0;
+    while (n < ncls && L[n] <= 1024) ++n;
+    return n;
+}
 
 template <typename T>
 static int check_smem(const GeomDev &g, int mmax) {
@@ -786,9 +803,10 @@ static int launch_analysis_t(const GeomDev &g, int nmaps, const T *maps, int64_t
     const int *clsL = f32 ? g.rest_L : g.cls_L;
     const int64_t *clsF = f32 ? g.rest_first : g.cls_first;
     const int32_t *clsP = f32 ? g.rest_pairs : g.cls_pairs;
-    for (int c = 0; c < ncls; ++c) {
+    const int nmerge = merged_classes(ncls, clsL, clsF);
+    for (int c = nmerge ? nmerge - 1 : 0; c < ncls; ++c) {
         const int L = clsL[c];
-        const int64_t first = clsF[c], cnt = clsF[c + 1] - first;
+        const int64_t first = c < nmerge ? 0 : clsF[c], cnt = clsF[c + 1] - first;
         // stage the north ring's F(m) for joint (north, south) stores unless that costs CTAs per SM
         const size_t base_smem = class_smem<T>(L, mmax), stage_bytes = sizeof(c2_t<T>) * (size_t)(mmax + 1);
         const int ctas0 = ctas_by_smem(base_smem), ctas1 = ctas_by_smem(base_smem + stage_bytes);
@@ -825,9 +843,10 @@ static int launch_synthesis_t(const GeomDev &g, int nmaps, const c2_t<T> *Gm, in
     const int *clsL = f32 ? g.rest_L : g.cls_L;
     const int64_t *clsF = f32 ? g.rest_first : g.cls_first;
     const int32_t *clsP = f32 ? g.rest_pairs : g.cls_pairs;
-    for (int c = 0; c < ncls; ++c) {
+    const int nmerge = merged_classes(ncls, clsL, clsF);
+    for (int c = nmerge ? nmerge - 1 : 0; c < ncls; ++c) {
         const int L = clsL[c];
-        const int64_t first = clsF[c], cnt = clsF[c + 1] - first;
+        const int64_t first = c < nmerge ? 0 : clsF[c], cnt = clsF[c + 1] - first;
         const bool stage_t = class_smem_syn<T>(L, mmax, true) <= (size_t)max_smem_optin();
         const int smem = (int)class_smem_syn<T>(L, mmax, stage_t), nt = class_threads(L);
         HB_CUDA_TRY(cudaFuncSetAttribute(ring_synthesis_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

@@ -216,6 +216,8 @@ int launch_spin_analysis(const hb_plan *p, int precision, int nmaps, const void 
                          cudaStream_t st);
 int launch_spin_synthesis(const hb_plan *p, int precision, int nmaps, const void *E, const void *B, void *QGm, void *UGm,
                           cudaStream_t st);
+// leading ring-FFT classes (ascending L) that share one launch
+int merged_classes(int ncls, const int *L, const int64_t *first);
 // FFT twiddle table and Bluestein chirp spectra of a geometry
 int build_fft_tables(GeomDev &g, cudaStream_t st);
 // pair-packed FP32 ring FFTs (hb_ringpack.cu) over the geometry's pk_* pairs

@@ -15,11 +15,19 @@
 // Rotation (the reference's convention, rotate_alm_euler.py / wigner_full.py:79-96):
 //   a'_{lm} = sum_{m'=-l..l} exp(-i m alpha) d^l_{mm'}(beta) exp(-i m' gamma) a_{lm'},
 // a_{l,-m'} = (-1)^{m'} conj(a_{lm'}) for the real field; healpy m-major layout, m >= 0 stored.
-// One CTA per output order m; its threads take input orders m', each running the recursion over
-// l and adding its term to the CTA's shared accumulator row a'_{l m} (warp reduction, then one
-// shared-memory atomic per warp and l).
+//
+// Rotation kernel: R_l = s_l(m) s_l(m') with s_l(k) = sqrt(l^2 - k^2), so a step needs no root or
+// division per (l, m, m').  A thread takes one m' >= 0 with both signs and MM output orders m, which
+// share 1/s_l(m') and the phase-rotated input z = exp(-i m' gamma) a_{lm'}: with p = d_{m,m'}, q = (-1)^m'
+// d_{m,-m'} the two signs add (p + q) Re z + i (p - q) Im z.  The factors of m are a table in shared
+// memory.  Bound by issue: per l about 32 operations shared by the MM orders and 14 per order
+// (a step with two roots and a division took over 100 per (l, m, m')), then the sum
+// over m': TL l at a time by a transposing warp reduction (16 values per lane), one shared atomic each.
+// CTAs hold chunks of 256 orders m' and add to the output with global atomics when there are
+// several.  One set of alm at lmax 767: 2880 -> 635 us.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "hb_internal.cuh"
 
@@ -114,61 +122,207 @@ __global__ void __launch_bounds__(ROT_NT) wigner_d_kernel(int l, int nbeta, cons
     }
 }
 
-// a'_{lm} for one output order m per CTA (see the file comment)
-__global__ void __launch_bounds__(ROT_NT) rotate_alm_kernel(int lmax, const double2 *__restrict__ ain,
-                                                           double2 *__restrict__ aout, double alpha, double x,
-                                                           double lc, double ls, int flip, double gamma) {
-    extern __shared__ double2 acc[];  // [lmax + 1]
-    const int m = blockIdx.x, b = blockIdx.y;
-    const int64_t nalm = alm_idx(lmax, lmax, lmax) + 1;
-    const double2 *a = ain + b * nalm;
-    for (int l = threadIdx.x; l <= lmax; l += blockDim.x) acc[l] = make_double2(0.0, 0.0);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    // input orders m' in [-lmax, lmax], one per thread per pass (every warp makes the same passes)
-    for (int base = -lmax; base <= lmax; base += ROT_NT) {
-        const int mp = base + (int)threadIdx.x;
-        const bool act = mp <= lmax;
-        const int amp = abs(mp);
-        const int l0 = act ? max(m, amp) : lmax + 1;
-        // exp(-i m' gamma); a_{l,-m'} = (-1)^{m'} conj a_{l m'}; the (-1)^{m-m'} of a reduced beta
-        double gs, gc;
-        sincos(-(double)mp * gamma, &gs, &gc);
-        double sg = (mp < 0 && (amp & 1)) ? -1.0 : 1.0;
-        if (flip && ((m - mp) & 1)) sg = -sg;
-        int lw = l0;  // the warp walks l from its smallest l0; lanes before their own l0 add zero
-        for (int o = 16; o > 0; o >>= 1) lw = min(lw, __shfl_xor_sync(0xffffffffu, lw, o));
-        if (lw > lmax) continue;
-        double d0 = 0.0, d1 = 0.0;
-        int e = -1;
-        if (act && l0 <= lmax) d_edge(m, mp, lc, ls, d1, e);
-        for (int l = lw; l <= lmax; ++l) {
-            if (act && l > l0) d_step(l - 1, m, mp, x, d0, d1, e);
-            double tr = 0.0, ti = 0.0;
-            if (act && l >= l0 && e == 0) {
-                const double2 v = a[alm_idx(lmax, l, amp)];
-                const double vi = mp < 0 ? -v.y : v.y;
-                const double dv = sg * d1;
-                tr = dv * (v.x * gc - vi * gs);
-                ti = dv * (v.x * gs + vi * gc);
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                tr += __shfl_xor_sync(0xffffffffu, tr, o);
-                ti += __shfl_xor_sync(0xffffffffu, ti, o);
-            }
-            if (lane == 0 && (tr != 0.0 || ti != 0.0)) {
-                atomicAdd(&acc[l].x, tr);
-                atomicAdd(&acc[l].y, ti);
-            }
+constexpr int ROT_V = 16;  // values per lane of the warp reduction: TL * MM * 2
+
+// sum over the warp of 16 values per lane: lane 2 i ends with the sum of v[i]
+__device__ __forceinline__ double warp_sums16(double (&v)[ROT_V], int lane) {
+#pragma unroll
+    for (int h = ROT_V / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double keep = up ? v[i + h] : v[i], send = up ? v[i] : v[i + h];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
     }
-    __syncthreads();
-    double as, ac;
-    sincos(-(double)m * alpha, &as, &ac);
-    for (int l = m + (int)threadIdx.x; l <= lmax; l += blockDim.x) {
-        const double2 v = acc[l];
-        aout[b * nalm + alm_idx(lmax, l, m)] = make_double2(v.x * ac - v.y * as, v.x * as + v.y * ac);
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// d^{l0}_{m,m'} as in d_edge, log factorials from a table
+__device__ __forceinline__ void d_edge_tab(const double *lf, int m, int mp, double lc, double ls, double &mant, int &e) {
+    if (!lf) return d_edge(m, mp, lc, ls, mant, e);
+    int j, k, sh;
+    if (m >= abs(mp)) {  // m >= 0 here
+        j = m; k = mp; sh = 0;
+    } else if (mp > 0) {
+        j = mp; k = m; sh = (m - j) & 1;
+    } else {
+        j = -mp; k = -m; sh = 0;
     }
+    const double l2e = 1.4426950408889634073599246810018921;  // log2 e
+    double L2 = 0.5 * (lf[2 * j] - lf[j + k] - lf[j - k]) * l2e;
+    if (j + k > 0) L2 += (double)(j + k) * lc;
+    if (j - k > 0) L2 += (double)(j - k) * ls;
+    if (!(L2 > -1.0e300)) {  // -inf: an exact zero that the recursion keeps
+        mant = 0.0;
+        e = 0;
+        return;
+    }
+    e = (int)floor((L2 + 128.0) / 256.0);
+    mant = exp2(L2 - 256.0 * (double)e) * ((((j - k) & 1) ^ sh) ? -1.0 : 1.0);
+}
+
+struct RotElem {  // d_{l-1}, d_l of one (m, m') and their scale exponent
+    double d0, d1;
+    int e;
+    template <bool CLEAN> __device__ __forceinline__ void step(double t, double c) {
+        const double v = fma(t, d1, -(c * d0));
+        d0 = d1;
+        d1 = v;
+        if (CLEAN) return;
+        // past 2^128 (by the high word, off the FP64 pipe): bring the scale up by 2^256
+        if (e < 0 && (__double2hiint(v) & 0x7fffffff) > 0x47f00000) {
+            d0 *= 0x1p-256;
+            d1 *= 0x1p-256;
+            ++e;
+        }
+    }
+    __device__ __forceinline__ double value() const { return e == 0 ? d1 : 0.0; }
+};
+
+// factors of d_l = ((L(L+1) x - m m') F / s_l(m')) d_{l-1} - (C s_L(m') / s_l(m')) d_{l-2}, L = l - 1:
+// F = (2L+1) / (L s_l(m)), C = (l/L) s_L(m) / s_l(m); zero for l <= m and l = 1
+__device__ __forceinline__ double2 rot_factors(int l, int m) {
+    const int L = l - 1;
+    if (l <= m || L <= 0) return make_double2(0.0, 0.0);
+    const double s2 = (double)(l - m) * (double)(l + m);
+    return make_double2((2.0 * L + 1.0) / (L * sqrt(s2)), (double)l / L * sqrt((double)max(L - m, 0) * (double)(L + m) / s2));
+}
+
+// acc [lmax + 1 - mb][MM] and, with TAB, the factors of (l, m) alike and the log factorials
+template <int MM, bool TAB> size_t rot_smem(int lmax) {
+    return (TAB ? 32 : 16) * (size_t)MM * (size_t)(lmax + 1) + (TAB ? 8 * (size_t)(2 * lmax + 1) : 0);
+}
+
+template <int MM, bool TAB>
+__global__ void __launch_bounds__(ROT_NT, 2) rotate_alm_kernel(int lmax, const double2 *__restrict__ ain,
+                                                           double2 *__restrict__ aout, double alpha, double x, double lc,
+                                                           double ls, int flip, double gamma, int atomic) {
+    constexpr int TL = ROT_V / (2 * MM);
+    extern __shared__ double2 rot_smem_buf[];
+    const int mb = blockIdx.x * MM, tid = threadIdx.x, lane = tid & 31;
+    const int64_t nalm = alm_idx(lmax, lmax, lmax) + 1;
+    const double2 *a = ain + blockIdx.z * nalm;
+    const int rows = lmax + 1 - mb;
+    double2 *acc = rot_smem_buf, *fc = acc + rows * MM;
+    double *lf = TAB ? reinterpret_cast<double *>(fc + rows * MM) : nullptr;
+    const int mp0 = blockIdx.y * ROT_NT, lmin = max(mb, mp0);  // nothing happens below
+    for (int i = tid; i < rows * MM; i += ROT_NT) {
+        if (TAB) fc[i] = rot_factors(mb + i / MM, mb + i % MM);
+        acc[i] = make_double2(0.0, 0.0);
+    }
+    if (TAB)
+        for (int i = tid; i <= 2 * lmax; i += ROT_NT) lf[i] = lgamma((double)i + 1.0);
+    __syncthreads();
+    const int mp = mp0 + tid;
+    const bool act = mp <= lmax;
+    double gs, gc;
+    sincos((double)mp * gamma, &gs, &gc);
+    if (flip && (mp & 1)) {  // (-1)^{m-m'} of a reduced beta: the m' half of it here
+        gs = -gs;
+        gc = -gc;
+    }
+    const double qs = mp == 0 ? 0.0 : (mp & 1) ? -1.0 : 1.0;  // m' = 0 has one sign only
+    RotElem P[MM], Q[MM];
+#pragma unroll
+    for (int i = 0; i < MM; ++i) {  // edge values, held until l passes l0 = max(m, m')
+        P[i] = {0.0, 0.0, 0};
+        Q[i] = {0.0, 0.0, 0};
+        if (act && mb + i <= lmax) {
+            d_edge_tab(lf, mb + i, mp, lc, ls, P[i].d1, P[i].e);
+            d_edge_tab(lf, mb + i, -mp, lc, ls, Q[i].d1, Q[i].e);
+        }
+    }
+    const double mp2 = (double)mp * (double)mp;
+    double inv = 0.0;  // 1 / s_{l-1}(m')
+    const int lw = max(lmin, __shfl_sync(0xffffffffu, mp, 0));
+    const double2 *col = a + alm_idx(lmax, 0, act ? mp : 0);
+    if (lw > mp) inv = rsqrt((double)(lw - 1) * (double)(lw - 1) - mp2);
+    if (lw - 1 <= mp) inv = 0.0;
+    // TL values of l.  CLEAN: every element of the warp is past its edge and at e = 0 (most of the range),
+    // so nothing is held back, rescaled or masked.
+    const auto rows_at = [&](int l0, auto clean) {
+        constexpr bool CLEAN = decltype(clean)::value;
+        double v[ROT_V];
+#pragma unroll
+        for (int s = 0; s < TL; ++s) {
+            const int l = l0 + s;
+            const bool on = act && (CLEAN || (l >= mp && l <= lmax));
+            const double2 z0 = on ? col[l] : make_double2(0.0, 0.0);
+            const double dl = (double)l, dL = dl - 1.0;
+            const double i1 = CLEAN || l > mp ? rsqrt(fma(dl, dl, -mp2)) : 0.0;
+            const double r = fma(dL, dL, -mp2) * inv * i1, X = dL * dl * x;  // r = s_{l-1}(m') / s_l(m')
+            inv = i1;
+            const double zr = fma(z0.x, gc, z0.y * gs), zi = fma(z0.y, gc, -(z0.x * gs));
+#pragma unroll
+            for (int i = 0; i < MM; ++i) {
+                const int m = mb + i, k = (CLEAN ? l : min(l, lmax)) - mb;
+                double p, q;
+                if (CLEAN || (on && l > max(m, mp))) {
+                    const double2 f = TAB ? fc[k * MM + i] : rot_factors(l, m);
+                    const double g = f.x * i1, c = f.y * r, mm = (double)m * (double)mp;
+                    // l = 1 from l0 = 0 (m = m' = 0): P_1 = x P_0
+                    P[i].template step<CLEAN>(!CLEAN && l == 1 && m == 0 && mp == 0 ? x : (X - mm) * g, c);
+                    Q[i].template step<CLEAN>((X + mm) * g, c);
+                }
+                if (CLEAN) {
+                    p = P[i].d1;
+                    q = qs * Q[i].d1;
+                } else {
+                    const bool in = on && l >= m;
+                    p = in ? P[i].value() : 0.0;
+                    q = in ? qs * Q[i].value() : 0.0;
+                }
+                v[(s * MM + i) * 2] = (p + q) * zr;
+                v[(s * MM + i) * 2 + 1] = (p - q) * zi;
+            }
+        }
+        const double t = warp_sums16(v, lane);
+        const int i = lane >> 1, l = l0 + i / (2 * MM), k = (l - mb) * MM + (i / 2) % MM;
+        if (!(lane & 1) && l <= lmax) atomicAdd((i & 1) ? &acc[k].y : &acc[k].x, t);
+    };
+    int l0 = lw;
+    for (; l0 <= lmax; l0 += TL) {
+        bool neg = l0 <= max(mb + MM - 1, act ? mp : 0) || l0 + TL - 1 > lmax || l0 < 2;
+#pragma unroll
+        for (int i = 0; i < MM; ++i) neg |= (P[i].e | Q[i].e) < 0;
+        if (!__any_sync(0xffffffffu, neg)) break;
+        rows_at(l0, std::false_type());
+    }
+    for (; l0 + TL - 1 <= lmax; l0 += TL) rows_at(l0, std::true_type());
+    if (l0 <= lmax) rows_at(l0, std::false_type());
+    __syncthreads();
+    for (int i = tid; i < rows * MM; i += ROT_NT) {
+        const int l = mb + i / MM, m = mb + i % MM;
+        if (m > l || l < lmin) continue;
+        double as, ac;
+        sincos((double)m * alpha, &as, &ac);
+        if (flip && (m & 1)) {
+            as = -as;
+            ac = -ac;
+        }
+        const double2 t = acc[i];
+        double2 *o = aout + blockIdx.z * nalm + alm_idx(lmax, l, m);
+        const double2 w = make_double2(t.x * ac + t.y * as, t.y * ac - t.x * as);  // times exp(-i m alpha)
+        if (atomic) {
+            atomicAdd(&o->x, w.x);
+            atomicAdd(&o->y, w.y);
+        } else {
+            *o = w;
+        }
+    }
+}
+
+template <int MM, bool TAB>
+int run_rotate(int lmax, int nmaps, const double2 *in, double2 *out, double alpha, const BetaRed &br, double gamma, cudaStream_t st) {
+    const size_t smem = rot_smem<MM, TAB>(lmax);
+    const int chunks = lmax / ROT_NT + 1;
+    HB_CUDA_TRY(cudaFuncSetAttribute(rotate_alm_kernel<MM, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (chunks > 1) HB_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double2) * (size_t)alm_size(lmax, lmax) * nmaps, st));
+    rotate_alm_kernel<MM, TAB><<<dim3((unsigned)(lmax / MM + 1), (unsigned)chunks, (unsigned)nmaps), ROT_NT, smem, st>>>(
+        lmax, in, out, alpha, br.x, br.lc, br.ls, br.flip ? 1 : 0, gamma, chunks > 1 ? 1 : 0);
+    HB_CHECK_LAUNCH();
+    return HB_OK;
 }
 
 }  // namespace
@@ -193,13 +347,15 @@ int hb_rotate_alm(int lmax, int nmaps, const void *alm_in, void *alm_out, double
                   hb_stream_t s) {
     if (lmax < 0 || lmax > HB_MAX_L || nmaps < 1 || nmaps > 65535 || !alm_in || !alm_out || alm_in == alm_out)
         return fail(HB_ERR_INVALID, "hb_rotate_alm: bad arguments (lmax <= 16383, out of place)");
-    const size_t smem = sizeof(double2) * (size_t)(lmax + 1);
-    HB_CUDA_TRY(cudaFuncSetAttribute(rotate_alm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const BetaRed br = beta_reduce(beta);
-    rotate_alm_kernel<<<dim3((unsigned)(lmax + 1), (unsigned)nmaps), ROT_NT, smem, (cudaStream_t)s>>>(
-        lmax, (const double2 *)alm_in, (double2 *)alm_out, alpha, br.x, br.lc, br.ls, br.flip ? 1 : 0, gamma);
-    HB_CHECK_LAUNCH();
-    return HB_OK;
+    const auto *in = (const double2 *)alm_in;
+    auto *out = (double2 *)alm_out;
+    // Two orders per CTA while the tables fit (lmax <= 2800), else one, without tables where they do not
+    // fit either.  At lmax 767 two orders take 635 us, four 676 us (both at two CTAs per SM).
+    const auto st = (cudaStream_t)s;
+    if (rot_smem<2, true>(lmax) <= 220 * 1024) return run_rotate<2, true>(lmax, nmaps, in, out, alpha, br, gamma, st);
+    if (rot_smem<1, true>(lmax) <= 220 * 1024) return run_rotate<1, true>(lmax, nmaps, in, out, alpha, br, gamma, st);
+    return run_rotate<1, false>(lmax, nmaps, in, out, alpha, br, gamma, st);
 }
 
 }  // extern "C"

@@ -113,3 +113,32 @@ def test_gpu_rotation_large_lmax_invariants():
     assert float(torch.linalg.norm(back - a) / torch.linalg.norm(a)) < 1e-10
     c0, c1 = hb.alm2cl(a), hb.alm2cl(r)
     assert float(torch.max(torch.abs(c1 - c0) / c0[2:].min())) < 1e-9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lmax,beta", [(0, 0.4), (1, 2.5), (2, 0.0), (31, 4.0), (32, math.pi), (65, -0.7)])
+def test_gpu_rotation_sizes_vs_oracle(oracle, lmax, beta):
+    """Edges of the kernel's tiling: warps of 32 input orders, odd numbers of output orders."""
+    import torch
+    from hellblast_b200 import rotate
+    alm = oracle.synalm(1.0 / (np.arange(lmax + 1) + 2.0) ** 2, seed=lmax + 1)
+    got = rotate.rotate_alm_euler(torch.from_numpy(alm).cuda(), 0.3, beta, -0.7).cpu().numpy()
+    want = oracle.rotate_alm_euler(alm, lmax, 0.3, beta, -0.7)
+    assert np.max(np.abs(got - want)) < 1e-11 * np.max(np.abs(want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lmax", [255, 256, 301, 2810, 4700])
+def test_gpu_rotation_inverse(lmax):
+    """Chunks of 256 input orders, and the variants for large lmax: a rotation and its inverse give the input back
+    (1e-10 L2: two rotations, each of some 1e-12 from the edge values' logarithms)."""
+    import torch
+    from hellblast_b200 import alm_ops, rotate
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(lmax)
+    n = alm_ops.alm_size(lmax)
+    a = torch.complex(torch.randn(n, generator=gen, device="cuda", dtype=torch.float64),
+                      torch.randn(n, generator=gen, device="cuda", dtype=torch.float64))
+    a[: lmax + 1] = a[: lmax + 1].real.to(a.dtype)
+    b = rotate.rotate_alm_euler(rotate.rotate_alm_euler(a, 0.3, 1.1, -0.7), 0.7, -1.1, -0.3)
+    assert float(torch.linalg.norm(a - b) / torch.linalg.norm(a)) < 1e-10

@@ -105,7 +105,7 @@ def alm2cl(alms, alms2=None, lmax: int | None = None, mmax: int | None = None):
     squeeze = t.dim() == 1
     t2 = t.reshape(-1, t.shape[-1])
     b = None if alms2 is None else as_tensor(alms2).reshape(-1, t.shape[-1])
-    cl = ops.alm2cl(t2, b, lmax_in, mm)
+    cl = ops.call(ops.alm2cl, t2, b, lmax_in, mm)
     cl = cl[:, :lmax + 1]
     return like_input(cl[0] if squeeze else cl, alms)
 

@@ -19,23 +19,23 @@ class Map2Alm(torch.autograd.Function):
     def forward(ctx, maps, pid, weights):
         ctx.save_for_backward(weights)
         ctx.pid = pid
-        return ops.map2alm(maps, pid, weights, 0)
+        return ops.call(ops.map2alm, maps, pid, weights, 0)
 
     @staticmethod
     def backward(ctx, galm):
         (weights,) = ctx.saved_tensors
-        return ops.map2alm_adjoint(galm.contiguous(), ctx.pid, weights, 0), None, None
+        return ops.call(ops.map2alm_adjoint, galm.contiguous(), ctx.pid, weights, 0), None, None
 
 
 class Alm2Map(torch.autograd.Function):
     @staticmethod
     def forward(ctx, alm, pid):
         ctx.pid = pid
-        return ops.alm2map(alm, pid, 0)
+        return ops.call(ops.alm2map, alm, pid, 0)
 
     @staticmethod
     def backward(ctx, gmap):
-        return ops.alm2map_adjoint(gmap.contiguous(), ctx.pid, 0), None
+        return ops.call(ops.alm2map_adjoint, gmap.contiguous(), ctx.pid, 0), None
 
 
 class Map2AlmSpin2(torch.autograd.Function):
@@ -43,14 +43,14 @@ class Map2AlmSpin2(torch.autograd.Function):
     def forward(ctx, Q, U, pid, weights):
         ctx.save_for_backward(weights)
         ctx.pid = pid
-        return ops.map2alm_spin2(Q, U, pid, weights, 0)
+        return ops.call(ops.map2alm_spin2, Q, U, pid, weights, 0)
 
     @staticmethod
     def backward(ctx, gE, gB):
         (weights,) = ctx.saved_tensors
         gE = gE.contiguous()
         gB = gB.contiguous()
-        gQ, gU = ops.map2alm_spin2_adjoint(gE, gB, ctx.pid, weights, 0)
+        gQ, gU = ops.call(ops.map2alm_spin2_adjoint, gE, gB, ctx.pid, weights, 0)
         return gQ, gU, None, None
 
 
@@ -58,11 +58,11 @@ class Alm2MapSpin2(torch.autograd.Function):
     @staticmethod
     def forward(ctx, E, B, pid):
         ctx.pid = pid
-        return ops.alm2map_spin2(E, B, pid, 0)
+        return ops.call(ops.alm2map_spin2, E, B, pid, 0)
 
     @staticmethod
     def backward(ctx, gQ, gU):
-        gE, gB = ops.alm2map_spin2_adjoint(gQ.contiguous(), gU.contiguous(), ctx.pid, 0)
+        gE, gB = ops.call(ops.alm2map_spin2_adjoint, gQ.contiguous(), gU.contiguous(), ctx.pid, 0)
         return gE, gB, None
 
 
@@ -73,7 +73,7 @@ class Alm2Cl(torch.autograd.Function):
     def forward(ctx, alm, lmax, mmax):
         ctx.save_for_backward(alm)
         ctx.cfg = (lmax, mmax)
-        return ops.alm2cl(alm, None, lmax, mmax)
+        return ops.call(ops.alm2cl, alm, None, lmax, mmax)
 
     @staticmethod
     def backward(ctx, gcl):

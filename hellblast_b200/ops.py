@@ -24,7 +24,7 @@ def _prec(dtype: torch.dtype) -> int:
 
 
 def _stream(dev: torch.device) -> int:
-    return torch.cuda.current_stream(dev).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if dev.index is None else dev.index)
 
 
 def _check_cuda(*ts):
@@ -54,8 +54,34 @@ def _rtype(prec):
     return torch.float32 if prec == 32 else torch.float64
 
 
-@torch.library.custom_op("hb::map2alm", mutates_args=())
-def map2alm(maps: torch.Tensor, pid: int, weights: Optional[torch.Tensor], flags: int) -> torch.Tensor:
+_direct: dict = {}
+
+
+def _op(name: str, fn):
+    op = torch.library.custom_op(name, fn, mutates_args=())
+    _direct[op] = fn
+    return op
+
+
+def _plain(args) -> bool:
+    """Whether nothing but the computation can happen in a call: ordinary tensors outside autograd,
+    and no tracer, mode, transform (vmap, forward AD) or profiler that has to see the operator."""
+    for a in args:
+        if isinstance(a, torch.Tensor) and (type(a) is not torch.Tensor or (a.requires_grad and torch.is_grad_enabled())):
+            return False
+    return not (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
+                or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None
+                or torch.autograd.forward_ad._current_level >= 0 or torch.autograd._profiler_enabled())
+
+
+def call(op, *args):
+    """``op(*args)`` for one of the operators below.  Plain calls run its implementation directly:
+    the custom-operator machinery takes about 11 us of host time per call, as long as the kernels of a
+    whole transform at nside 16."""
+    return _direct[op](*args) if _plain(args) else op(*args)
+
+
+def _map2alm(maps: torch.Tensor, pid: int, weights: Optional[torch.Tensor], flags: int) -> torch.Tensor:
     _check_cuda(maps, weights)
     p = G.get_plan(pid)
     maps = maps.contiguous()
@@ -67,14 +93,16 @@ def map2alm(maps: torch.Tensor, pid: int, weights: Optional[torch.Tensor], flags
     return out
 
 
+map2alm = _op("hb::map2alm", _map2alm)
+
+
 @map2alm.register_fake
 def _(maps, pid, weights, flags):
     p = G.get_plan(pid)
     return maps.new_empty((maps.shape[0], alm_size(p.lmax, p.mmax)), dtype=_ctype(_prec(maps.dtype)))
 
 
-@torch.library.custom_op("hb::alm2map", mutates_args=())
-def alm2map(alm: torch.Tensor, pid: int, flags: int) -> torch.Tensor:
+def _alm2map(alm: torch.Tensor, pid: int, flags: int) -> torch.Tensor:
     _check_cuda(alm)
     p = G.get_plan(pid)
     alm = alm.contiguous()
@@ -86,13 +114,15 @@ def alm2map(alm: torch.Tensor, pid: int, flags: int) -> torch.Tensor:
     return out
 
 
+alm2map = _op("hb::alm2map", _alm2map)
+
+
 @alm2map.register_fake
 def _(alm, pid, flags):
     return alm.new_empty((alm.shape[0], G.get_plan(pid).npix), dtype=_rtype(_prec(alm.dtype)))
 
 
-@torch.library.custom_op("hb::alm2map_adjoint", mutates_args=())
-def alm2map_adjoint(maps: torch.Tensor, pid: int, flags: int) -> torch.Tensor:
+def _alm2map_adjoint(maps: torch.Tensor, pid: int, flags: int) -> torch.Tensor:
     _check_cuda(maps)
     p = G.get_plan(pid)
     maps = maps.contiguous()
@@ -104,14 +134,16 @@ def alm2map_adjoint(maps: torch.Tensor, pid: int, flags: int) -> torch.Tensor:
     return out
 
 
+alm2map_adjoint = _op("hb::alm2map_adjoint", _alm2map_adjoint)
+
+
 @alm2map_adjoint.register_fake
 def _(maps, pid, flags):
     p = G.get_plan(pid)
     return maps.new_empty((maps.shape[0], alm_size(p.lmax, p.mmax)), dtype=_ctype(_prec(maps.dtype)))
 
 
-@torch.library.custom_op("hb::map2alm_adjoint", mutates_args=())
-def map2alm_adjoint(alm: torch.Tensor, pid: int, weights: Optional[torch.Tensor], flags: int) -> torch.Tensor:
+def _map2alm_adjoint(alm: torch.Tensor, pid: int, weights: Optional[torch.Tensor], flags: int) -> torch.Tensor:
     _check_cuda(alm, weights)
     p = G.get_plan(pid)
     alm = alm.contiguous()
@@ -123,13 +155,15 @@ def map2alm_adjoint(alm: torch.Tensor, pid: int, weights: Optional[torch.Tensor]
     return out
 
 
+map2alm_adjoint = _op("hb::map2alm_adjoint", _map2alm_adjoint)
+
+
 @map2alm_adjoint.register_fake
 def _(alm, pid, weights, flags):
     return alm.new_empty((alm.shape[0], G.get_plan(pid).npix), dtype=_rtype(_prec(alm.dtype)))
 
 
-@torch.library.custom_op("hb::map2alm_spin2", mutates_args=())
-def map2alm_spin2(Q: torch.Tensor, U: torch.Tensor, pid: int, weights: Optional[torch.Tensor],
+def _map2alm_spin2(Q: torch.Tensor, U: torch.Tensor, pid: int, weights: Optional[torch.Tensor],
                   flags: int) -> tuple[torch.Tensor, torch.Tensor]:
     _check_cuda(Q, U, weights)
     p = G.get_plan(pid)
@@ -143,6 +177,9 @@ def map2alm_spin2(Q: torch.Tensor, U: torch.Tensor, pid: int, weights: Optional[
     return E, B
 
 
+map2alm_spin2 = _op("hb::map2alm_spin2", _map2alm_spin2)
+
+
 @map2alm_spin2.register_fake
 def _(Q, U, pid, weights, flags):
     p = G.get_plan(pid)
@@ -150,8 +187,7 @@ def _(Q, U, pid, weights, flags):
     return e, torch.empty_like(e)
 
 
-@torch.library.custom_op("hb::alm2map_spin2", mutates_args=())
-def alm2map_spin2(E: torch.Tensor, B: torch.Tensor, pid: int, flags: int) -> tuple[torch.Tensor, torch.Tensor]:
+def _alm2map_spin2(E: torch.Tensor, B: torch.Tensor, pid: int, flags: int) -> tuple[torch.Tensor, torch.Tensor]:
     _check_cuda(E, B)
     p = G.get_plan(pid)
     E, B = E.contiguous(), B.contiguous()
@@ -164,14 +200,16 @@ def alm2map_spin2(E: torch.Tensor, B: torch.Tensor, pid: int, flags: int) -> tup
     return Q, U
 
 
+alm2map_spin2 = _op("hb::alm2map_spin2", _alm2map_spin2)
+
+
 @alm2map_spin2.register_fake
 def _(E, B, pid, flags):
     q = E.new_empty((E.shape[0], G.get_plan(pid).npix), dtype=_rtype(_prec(E.dtype)))
     return q, torch.empty_like(q)
 
 
-@torch.library.custom_op("hb::alm2map_spin2_adjoint", mutates_args=())
-def alm2map_spin2_adjoint(gQ: torch.Tensor, gU: torch.Tensor, pid: int,
+def _alm2map_spin2_adjoint(gQ: torch.Tensor, gU: torch.Tensor, pid: int,
                           flags: int) -> tuple[torch.Tensor, torch.Tensor]:
     _check_cuda(gQ, gU)
     p = G.get_plan(pid)
@@ -185,6 +223,9 @@ def alm2map_spin2_adjoint(gQ: torch.Tensor, gU: torch.Tensor, pid: int,
     return gE, gB
 
 
+alm2map_spin2_adjoint = _op("hb::alm2map_spin2_adjoint", _alm2map_spin2_adjoint)
+
+
 @alm2map_spin2_adjoint.register_fake
 def _(gQ, gU, pid, flags):
     p = G.get_plan(pid)
@@ -192,8 +233,7 @@ def _(gQ, gU, pid, flags):
     return e, torch.empty_like(e)
 
 
-@torch.library.custom_op("hb::map2alm_spin2_adjoint", mutates_args=())
-def map2alm_spin2_adjoint(gE: torch.Tensor, gB: torch.Tensor, pid: int, weights: Optional[torch.Tensor],
+def _map2alm_spin2_adjoint(gE: torch.Tensor, gB: torch.Tensor, pid: int, weights: Optional[torch.Tensor],
                           flags: int) -> tuple[torch.Tensor, torch.Tensor]:
     _check_cuda(gE, gB, weights)
     p = G.get_plan(pid)
@@ -207,14 +247,16 @@ def map2alm_spin2_adjoint(gE: torch.Tensor, gB: torch.Tensor, pid: int, weights:
     return gQ, gU
 
 
+map2alm_spin2_adjoint = _op("hb::map2alm_spin2_adjoint", _map2alm_spin2_adjoint)
+
+
 @map2alm_spin2_adjoint.register_fake
 def _(gE, gB, pid, weights, flags):
     q = gE.new_empty((gE.shape[0], G.get_plan(pid).npix), dtype=_rtype(_prec(gE.dtype)))
     return q, torch.empty_like(q)
 
 
-@torch.library.custom_op("hb::alm2cl", mutates_args=())
-def alm2cl(alm1: torch.Tensor, alm2: Optional[torch.Tensor], lmax: int, mmax: int) -> torch.Tensor:
+def _alm2cl(alm1: torch.Tensor, alm2: Optional[torch.Tensor], lmax: int, mmax: int) -> torch.Tensor:
     _check_cuda(alm1, alm2)
     alm1 = alm1.contiguous()
     if alm2 is not None:
@@ -224,6 +266,9 @@ def alm2cl(alm1: torch.Tensor, alm2: Optional[torch.Tensor], lmax: int, mmax: in
     L.call(f"hb_alm2cl_f{prec}", lmax, mmax, nmaps, alm1.data_ptr(), None if alm2 is None else alm2.data_ptr(),
            cl.data_ptr(), _stream(alm1.device))
     return cl
+
+
+alm2cl = _op("hb::alm2cl", _alm2cl)
 
 
 @alm2cl.register_fake

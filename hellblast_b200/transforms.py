@@ -53,6 +53,15 @@ def device_weights(weights, g: G.Geometry, device) -> torch.Tensor | None:
     return as_tensor(weights, torch.float64).reshape(-1).contiguous().to(device)
 
 
+def _rows(t: torch.Tensor, n: int, dtype: torch.dtype) -> torch.Tensor:
+    """[..., n] -> contiguous [rows, n] of ``dtype`` (the tensor itself when it is that already)."""
+    if t.dim() != 2 or t.shape[1] != n:
+        t = t.reshape(-1, n)
+    if t.dtype != dtype:
+        t = t.to(dtype)
+    return t.contiguous()
+
+
 def map2alm(maps, g: G.Geometry, lmax: int, mmax: int | None = None, weights=None, precision=None,
             ref_compat=None) -> torch.Tensor:
     """maps: flat [npix] or [nmaps, npix] -> alm [nalm] / [nmaps, nalm] (healpy layout)."""
@@ -60,11 +69,11 @@ def map2alm(maps, g: G.Geometry, lmax: int, mmax: int | None = None, weights=Non
     t = flatten_rings(maps) if isinstance(maps, (list, tuple)) else as_tensor(maps)
     rt = resolve_precision(precision, t.dtype)
     squeeze = t.dim() == 1
-    t = t.reshape(-1, g.npix).to(rt).contiguous()
+    t = _rows(t, g.npix, rt)
     if ref_compat not in REF_COMPAT:
         raise ValueError("ref_compat must be None, 'fallback' or 'raw'")
     p = G.plan(g, lmax, mmax, precision=32 if rt == torch.float32 else 64)
-    alm = ops.map2alm(t, p.pid, device_weights(weights, g, t.device), REF_COMPAT[ref_compat])
+    alm = ops.call(ops.map2alm, t, p.pid, device_weights(weights, g, t.device), REF_COMPAT[ref_compat])
     if ref_compat == "raw":
         mcut = min(mmax, int(np.max(g.nphi)) // 2)  # sht_raw.py:43 mmax_eff
         if mcut < mmax:
@@ -78,13 +87,13 @@ def alm2map(alm, g: G.Geometry, lmax: int, mmax: int | None = None, precision=No
     rt = resolve_precision(precision, t.dtype)
     ct = torch.complex64 if rt == torch.float32 else torch.complex128
     squeeze = t.dim() == 1
-    t = t.reshape(-1, t.shape[-1]).to(ct).contiguous()
+    t = _rows(t, t.shape[-1], ct)
     if t.shape[-1] != ops.alm_size(lmax, mmax):
         raise ValueError(f"alm has {t.shape[-1]} entries, expected {ops.alm_size(lmax, mmax)} for "
                          f"lmax={lmax}, mmax={mmax}")
     flags = L.HB_F_NOPHASE if ref_compat else 0
     p = G.plan(g, lmax, mmax, precision=32 if rt == torch.float32 else 64)
-    out = ops.alm2map(t, p.pid, flags)
+    out = ops.call(ops.alm2map, t, p.pid, flags)
     return out[0] if squeeze else out
 
 
@@ -102,11 +111,11 @@ def map2alm_spin2(Q, U, g: G.Geometry, lmax: int, mmax: int | None = None, weigh
     u = flatten_rings(U) if isinstance(U, (list, tuple)) else as_tensor(U)
     rt = resolve_precision(precision, q.dtype)
     squeeze = q.dim() == 1
-    q = q.reshape(-1, g.npix).to(rt).contiguous()
-    u = u.reshape(-1, g.npix).to(rt).contiguous()
+    q = _rows(q, g.npix, rt)
+    u = _rows(u, g.npix, rt)
     p = G.plan(g, lmax, mmax, precision=32 if rt == torch.float32 else 64, spin=True)
     flags = (L.HB_F_NOPHASE | L.HB_F_NOFOLD) if ref_compat else 0
-    E, B = ops.map2alm_spin2(q, -u if ref_compat else u, p.pid, device_weights(weights, g, q.device), flags)
+    E, B = ops.call(ops.map2alm_spin2, q, -u if ref_compat else u, p.pid, device_weights(weights, g, q.device), flags)
     if ref_compat:
         B = -B
         mcut = min(mmax, int(np.max(g.nphi)) // 2)  # spin.py:53 mmax_eff
@@ -128,10 +137,10 @@ def alm2map_spin2(E, B, g: G.Geometry, lmax: int, mmax: int | None = None, preci
     rt = resolve_precision(precision, e.dtype)
     ct = torch.complex64 if rt == torch.float32 else torch.complex128
     squeeze = e.dim() == 1
-    e = e.reshape(-1, e.shape[-1]).to(ct).contiguous()
-    b = b.reshape(-1, b.shape[-1]).to(ct).contiguous()
+    e = _rows(e, e.shape[-1], ct)
+    b = _rows(b, b.shape[-1], ct)
     p = G.plan(g, lmax, mmax, precision=32 if rt == torch.float32 else 64, spin=True)
-    Q, U = ops.alm2map_spin2(e, b, p.pid, L.HB_F_NOPHASE if ref_compat else 0)
+    Q, U = ops.call(ops.alm2map_spin2, e, b, p.pid, L.HB_F_NOPHASE if ref_compat else 0)
     if ref_compat:
         U = -U
     return (Q[0], U[0]) if squeeze else (Q, U)

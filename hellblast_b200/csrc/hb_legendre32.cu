@@ -15,9 +15,9 @@
 // recursion, shared by the NB maps of a CTA).  Two ring pairs share each packed instruction, which
 // leaves half the issue slots to loads and reductions; blocks of 256 l in which a set of pairs stays
 // evanescent are skipped by the plan's flags (a quarter of the work at lmax = 2 nside).
-// One map at nside 1024, lmax 2047: synthesis 1636 -> 890 us (66 % FMA pipe), analysis 2000 -> 1510 us
-// (46 %; blocks in which pairs still cross from e < 0 take a fifth of it); the arithmetic and the order of every sum
-// are unchanged (same bits).
+// One map at nside 1024, lmax 2047: synthesis 1636 -> 890 us (66 % FMA pipe), analysis 2000 -> 1320 us
+// (51 %; following the pairs that leave e < 0 within a block takes 160 us of it).  The arithmetic and the
+// order of every sum of the analysis are unchanged (same bits).
 #include <cmath>
 
 #include "hb_f32x2.cuh"
@@ -54,6 +54,13 @@ __device__ __forceinline__ void block_state(const GeomDev &g, int m, int j, int6
         l2 = c.y;
         e = __float_as_int(c.z);
     }
+}
+
+// whether a pair that starts a block with e < 0 keeps e < 0 through it, by the next block's checkpoint row:
+// both of its values below 2^-32 (one alone can be near zero on an oscillating pair)
+__device__ __forceinline__ bool stays_dead(const float4 *next, int64_t p) {
+    const float4 c = next[p];
+    return __float_as_int(c.z) < 0 && fabsf(c.y) < F32_UP;
 }
 
 struct alignas(16) Coef2 {  // (A_l, B_l), each in both halves
@@ -112,18 +119,17 @@ __device__ __forceinline__ void anal_step4(AState<K, NB> &S, const Coef2 *cf, fl
     }
 }
 
-// Moves to the next exponent after every fourth row; true if the warp had any.  A pair that reaches
-// e = 0 gets its weights from the thread's column fw of the staged (north, south) coefficients.
-template <int U0, int K, int NB, int NT> __device__ __forceinline__ bool anal_rescale(AState<K, NB> &S, const float4 *fw) {
-    unsigned bits = 0;  // live values stay far below 2^32, so a larger one has e < 0
-#pragma unroll
-    for (int u = U0; u < K; u += 2) bits = bits_or(bits, S.l1[u / 2]);
-    if (!__any_sync(0xffffffffu, maybe_big(bits))) return false;
+// Moves to the next exponent after every fourth row, in the pair sets up to um (the last one with e < 0
+// in the warp).  A pair that reaches e = 0 gets its weights from the thread's column fw of the staged
+// (north, south) coefficients.
+template <int U0, int K, int NB, int NT> __device__ __forceinline__ void anal_rescale(AState<K, NB> &S, int um, const float4 *fw) {
 #pragma unroll
     for (int u = U0; u < K; u += 2) {
+        if (u > um) break;
+        // live values stay far below 2^32, so a larger one has e < 0
+        if (!__any_sync(0xffffffffu, maybe_big(bits_or(0, S.l1[u / 2])))) continue;
         float v[2], f[2] = {1.f, 1.f};
         unpk(S.l1[u / 2], v[0], v[1]);
-        if (!__any_sync(0xffffffffu, maybe_big(bits_or(0, S.l1[u / 2])))) continue;
 #pragma unroll
         for (int h = 0; h < 2; ++h)
             if (S.e[u + h] < 0 && fabsf(v[h]) > F32_UP) {
@@ -136,14 +142,15 @@ template <int U0, int K, int NB, int NT> __device__ __forceinline__ bool anal_re
         S.l1[u / 2] = mul2(S.l1[u / 2], pk(f[0], f[1]));
         S.l2[u / 2] = mul2(S.l2[u / 2], pk(f[0], f[1]));
     }
-    return true;
 }
 
-template <int U0, int K, int NB> __device__ __forceinline__ bool any_negative(const AState<K, NB> &S) {
-    int neg = 0;
+// last even u whose pair sets u, u + 1 hold an e < 0 in the warp (-1: none)
+template <int U0, int K, int NB> __device__ __forceinline__ int last_negative(const AState<K, NB> &S) {
+    int um = -1;
 #pragma unroll
-    for (int u = U0; u < K; ++u) neg |= S.e[u];
-    return __any_sync(0xffffffffu, neg < 0);
+    for (int u = U0; u < K; u += 2)
+        if (__any_sync(0xffffffffu, (S.e[u] | S.e[u + 1]) < 0)) um = u;
+    return um;
 }
 
 // Rows 0 .. n-1 of the block for the pair sets U0 .. K-1 (the sets before them are evanescent).  Item
@@ -152,14 +159,15 @@ template <int U0, int K, int NB, int NT>
 __device__ __forceinline__ void anal_rows(AState<K, NB> &S, const Coef2 *cf, float2 *red, const float4 *fw, float2 *out, int n) {
     constexpr int SUBS = NT / 16, RB = 16 / NB;
     const int tid = threadIdx.x, item = tid / SUBS, sub = tid % SUBS;
-    bool mixed = any_negative<U0>(S);
+    int um = last_negative<U0>(S);
     for (int r0 = 0; r0 < n; r0 += RB, cf += RB) {
         float2 *buf = red + ((r0 / RB) & 1) * RB * NB * NT;
 #pragma unroll
         for (int s = 0; s < RB; s += 4) {
             anal_step4<U0, K, NB, NT>(S, cf + s, buf + s * NB * NT + tid);
-            if (mixed && anal_rescale<U0, K, NB, NT>(S, fw)) mixed = any_negative<U0>(S);
+            if (um >= 0) anal_rescale<U0, K, NB, NT>(S, um, fw);
         }
+        if (um >= 0) um = last_negative<U0>(S);
         __syncthreads();
         float rr = 0.f, ri = 0.f;
 #pragma unroll
@@ -206,7 +214,7 @@ __global__ void __launch_bounds__(NT, MINB) leg_analysis32_kernel(GeomDev g, int
     if (m < 0 || m > mmax || l0 > lmax) return;  // a listed order outside the plan: nothing read or written
     const int64_t np = g.npairs, blk = blk_ofs[m] + j;
     const int n = min(LB, lmax - l0 + 1);
-    const float4 *ckrow = ck + blk * np;
+    const float4 *ckrow = ck + blk * np, *cknext = blk + 1 < blk_ofs[m + 1] ? ckrow + np : nullptr;
     const uint8_t *fl = flags + blk * flag_stride(np);
     const float2 *F = Fm + (int64_t)blockIdx.z * NB * fm_stride + (int64_t)blockIdx.y * np * 2;
 #pragma unroll
@@ -248,6 +256,12 @@ __global__ void __launch_bounds__(NT, MINB) leg_analysis32_kernel(GeomDev g, int
                     set_weights(S, u + i, b, S.e[u + i] < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : f);
                 }
             }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)  // evanescent over the whole block: no values, and no exponent to follow
+                if (S.e[u + i] < 0 && cknext && stays_dead(cknext, p0 + (u + i) * NT + tid)) {
+                    a1[i] = a2[i] = 0.f;
+                    S.e[u + i] = 0;
+                }
             S.l1[u / 2] = pk(a1[0], a1[1]);
             S.l2[u / 2] = pk(a2[0], a2[1]);
             S.xh[u / 2] = pk(xh[0], xh[1]);

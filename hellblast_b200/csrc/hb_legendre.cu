@@ -35,6 +35,7 @@
 #include <cmath>
 
 #include "hb_internal.cuh"
+#include "hb_warp.cuh"
 
 namespace hb {
 
@@ -138,22 +139,6 @@ template <int U, typename Fn> __device__ __forceinline__ bool rescale(State<U> &
 __device__ __forceinline__ double4 four(const double *t) {
     const double2 a = *reinterpret_cast<const double2 *>(t), b = *reinterpret_cast<const double2 *>(t + 2);
     return make_double4(a.x, a.y, b.x, b.y);
-}
-
-// sum over the warp of NV values per lane: lane 2 i (NV 16) or i (NV 32) ends with the sum of v[i]
-template <int NV> __device__ __forceinline__ double warp_sums(double (&v)[NV], int lane) {
-    static_assert(NV == 16 || NV == 32, "values per lane");
-#pragma unroll
-    for (int h = NV / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
-        const bool up = lane & o;
-#pragma unroll
-        for (int i = 0; i < h; ++i) {
-            const double keep = up ? v[i + h] : v[i], send = up ? v[i] : v[i + h];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-    if (NV == 16) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-    return v[0];
 }
 
 // ------------------------------------------------------------------ analysis

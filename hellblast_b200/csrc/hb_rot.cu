@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "hb_internal.cuh"
+#include "hb_warp.cuh"
 
 namespace hb {
 namespace {
@@ -123,20 +124,6 @@ __global__ void __launch_bounds__(ROT_NT) wigner_d_kernel(int l, int nbeta, cons
 }
 
 constexpr int ROT_V = 16;  // values per lane of the warp reduction: TL * MM * 2
-
-// sum over the warp of 16 values per lane: lane 2 i ends with the sum of v[i]
-__device__ __forceinline__ double warp_sums16(double (&v)[ROT_V], int lane) {
-#pragma unroll
-    for (int h = ROT_V / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
-        const bool up = lane & o;
-#pragma unroll
-        for (int i = 0; i < h; ++i) {
-            const double keep = up ? v[i + h] : v[i], send = up ? v[i] : v[i + h];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
 
 // d^{l0}_{m,m'} as in d_edge, log factorials from a table
 __device__ __forceinline__ void d_edge_tab(const double *lf, int m, int mp, double lc, double ls, double &mant, int &e) {
@@ -277,7 +264,7 @@ __global__ void __launch_bounds__(ROT_NT, 2) rotate_alm_kernel(int lmax, const d
                 v[(s * MM + i) * 2 + 1] = (p - q) * zi;
             }
         }
-        const double t = warp_sums16(v, lane);
+        const double t = warp_sums<ROT_V>(v, lane);
         const int i = lane >> 1, l = l0 + i / (2 * MM), k = (l - mb) * MM + (i / 2) % MM;
         if (!(lane & 1) && l <= lmax) atomicAdd((i & 1) ? &acc[k].y : &acc[k].x, t);
     };

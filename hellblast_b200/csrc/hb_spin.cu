@@ -1,4 +1,5 @@
-// Spin-2 (Q/U <-> E/B) Legendre kernels, FP32 and FP64.
+// Spin-2 (Q/U <-> E/B) Legendre kernels in FP64 (the FP32 ones are in hb_spin32.cu), and the launchers
+// of both.
 //
 // Replaces map2alm_spin_gpu / eb_from_qu_gpu / qu_from_eb_gpu (spin.py:32-115) and the
 // closed-form Wigner sum wigner_d_ms_sum (wigner_d_ms.cu:20-50, one launch per (m, s), O(lmax^2)
@@ -15,478 +16,429 @@
 // started at l0 = max(m,2) from the closed-form d^{l0}_{m,+-2} (log-scaled; P and M carry
 // separate running exponents: their ratio near the poles is cot^4(theta/2)).
 // Mirror symmetry: _s lambda(pi - theta) = (-1)^(l+m) _{-s}lambda(theta).
+//
+// The recursions run scaled, P_l = N_l rho_l with N_l N_{l+1} eps_{l+1} = 1/2, eps_l = 1 / a_{l-1}:
+//     rho_{l+1} = (A_l x +- A_l beta_l) rho_l - rho_{l-1},   A_l = 2 N_l^2,  beta_l = 2m / (l (l+1)),
+// 2 operations per function and l instead of 5.  N_l follows from its products over l, scanned by a
+// warp when a block's coefficients are staged.  Values are mantissa * 2^(512 e) and count as zero while
+// e < 0 (below 2^-256).
+//
+// What bounds the kernels: the FP64 pipe, 4 operations per (l, ring pair) for the recursions and 8 per map
+// for the contraction, and in the analysis the warp reductions.  Three Q/U maps at nside 256, lmax 700:
+// synthesis 523 -> 440 us, analysis 1261 -> 636 us.
 #include <cmath>
 
 #include "hb_internal.cuh"
+#include "hb_warp.cuh"
 
 namespace hb {
 
-template <typename T> struct SpinCfg;
-template <> struct SpinCfg<float> {
-    static constexpr int SE = 64;
-    static constexpr int TL = 16;
-};
-template <> struct SpinCfg<double> {
-    static constexpr int SE = 512;
-    static constexpr int TL = 8;
-};
+constexpr int SPB = 128;  // l per staged block
 
-template <typename T> struct V4;
-template <> struct V4<float> { using type = float4; };
-template <> struct V4<double> { using type = double4; };
-template <typename T> using v4_t = typename V4<T>::type;
-__device__ __forceinline__ float4 mk4(float a, float b, float c, float d) { return make_float4(a, b, c, d); }
-__device__ __forceinline__ double4 mk4(double a, double b, double c, double d) { return make_double4(a, b, c, d); }
-
-template <typename T> struct SXRep;
-template <> struct SXRep<float> {
-    float hi, lo;
-    __device__ __forceinline__ void load(const GeomDev &g, int64_t p) { hi = g.pair_xhi[p]; lo = g.pair_xlo[p]; }
-    __device__ __forceinline__ float mul(float v) const { return fmaf(hi, v, lo * v); }
-    __device__ __forceinline__ void zero() { hi = lo = 0.f; }
-};
-template <> struct SXRep<double> {
-    double x;
-    __device__ __forceinline__ void load(const GeomDev &g, int64_t p) { x = g.pair_x[p]; }
-    __device__ __forceinline__ double mul(double v) const { return x * v; }
-    __device__ __forceinline__ void zero() { x = 0.0; }
-};
-
-template <typename T> __device__ __forceinline__ T s_huge();
-template <> __device__ __forceinline__ float s_huge<float>() { return 4294967296.0f; }
-template <> __device__ __forceinline__ double s_huge<double>() { return 0x1p256; }
-template <typename T> __device__ __forceinline__ T s_down();
-template <> __device__ __forceinline__ float s_down<float>() { return 5.42101086242752217e-20f; }
-template <> __device__ __forceinline__ double s_down<double>() { return 0x1p-512; }
-
-// coefficients that produce lambda_{lp} from lambda_{lp-1}, lambda_{lp-2}:
-// (a, b, c) of l = lp-1; lp == l0 injects the start value held in lambda_{l0-2}; lp > lmax -> 0
-__device__ __forceinline__ void spin_coef(int lp, int m, int l0, int lmax, double &a, double &b, double &c) {
-    if (lp == l0) {
-        a = 0.0; b = 0.0; c = -1.0;
-        return;
-    }
-    if (lp > lmax || lp < l0) {
-        a = b = c = 0.0;
-        return;
-    }
-    const double l = lp - 1, mm = m;
-    const double R1 = sqrt(((l + 1) * (l + 1) - mm * mm) * ((l + 1) * (l + 1) - 4.0));
-    const double R0 = sqrt(fmax(0.0, (l * l - mm * mm) * (l * l - 4.0)));
-    const double n10 = sqrt((2 * l + 3) / (2 * l + 1)), n1m = sqrt((2 * l + 3) / (2 * l - 1));
-    a = n10 * (2 * l + 1) * (l + 1) / R1;
-    b = n10 * (2 * l + 1) * 2.0 * mm / (l * R1);
-    c = n1m * (l + 1) * R0 / (l * R1);
-}
-
-// log-scaled start values of P (s=+2 function, d_{m,-2}) and M (d_{m,+2}) at l0 = max(m,2)
-template <typename T>
-__device__ __forceinline__ void spin_start(const GeomDev &g, int m, int64_t p, T &mp, int &ep, T &mm, int &em) {
-    constexpr int SE = SpinCfg<T>::SE;
+// log-scaled start values of P (d_{m,-2}) and M (d_{m,+2}) at l0 = max(m, 2)
+__device__ __forceinline__ void spin_start64(const GeomDev &g, int m, int64_t p, double &mp, int &ep, double &mm, int &em) {
     const double lc = g.pair_log2ch[p], ls = g.pair_log2sh[p], k = g.log2spin[m];
     const int u = m + 2, v = m >= 2 ? m - 2 : 2 - m;
     const double LP = k + v * lc + u * ls, LM = k + u * lc + v * ls;
     const double sp = (m & 1) ? -1.0 : 1.0, sm = (m >= 2) ? sp : 1.0;
-    ep = (int)floor((LP + 0.5 * SE) / SE);
-    em = (int)floor((LM + 0.5 * SE) / SE);
-    mp = (T)(sp * exp2(LP - (double)SE * ep));
-    mm = (T)(sm * exp2(LM - (double)SE * em));
+    ep = (int)floor((LP + 256.0) / 512.0);
+    em = (int)floor((LM + 256.0) / 512.0);
+    mp = sp * exp2(LP - 512.0 * ep);
+    mm = sm * exp2(LM - 512.0 * em);
 }
 
-constexpr int SCOEF_CH = 256;  // == the plan's checkpoint block length
-
-// Per pair and parity class (even / odd l-m, slots s&1 after the l0 parity swap), the weights
-//   E += P WPE + M WME,   B += P WPB + M WMB
-// with, for parity eps = (-1)^(l-m):
-//   Qe = QN + eps QS, Qo = QN - eps QS, Ue = UN + eps US, Uo = UN - eps US,
-//   WPE = -(Qe + i Uo)/2, WME = -(Qe - i Uo)/2, WPB = -(Ue - i Qo)/2, WMB = -(Ue + i Qo)/2.
-template <typename V, typename T>
-__device__ __forceinline__ void spin_weights(V qn, V qs, V un, V us, T eps, V &wpe, V &wme, V &wpb, V &wmb) {
-    V Qe = mk2(qn.x + eps * qs.x, qn.y + eps * qs.y), Qo = mk2(qn.x - eps * qs.x, qn.y - eps * qs.y);
-    V Ue = mk2(un.x + eps * us.x, un.y + eps * us.y), Uo = mk2(un.x - eps * us.x, un.y - eps * us.y);
-    const T h = (T)-0.5;
-    // i*z = (-z.y, z.x)
-    wpe = mk2(h * (Qe.x - Uo.y), h * (Qe.y + Uo.x));
-    wme = mk2(h * (Qe.x + Uo.y), h * (Qe.y - Uo.x));
-    wpb = mk2(h * (Ue.x + Qo.y), h * (Ue.y - Qo.x));
-    wmb = mk2(h * (Ue.x - Qo.y), h * (Ue.y + Qo.x));
+// eps_l^2 = (l^2 - m^2)(l^2 - 4) / (l^2 (4 l^2 - 1))
+__device__ __forceinline__ double spin_eps2(int l, int m) {
+    const double ll = l, mm = m, l2 = ll * ll;
+    return ((ll - mm) * (ll + mm) * (l2 - 4.0)) / (l2 * (4.0 * l2 - 1.0));
 }
+// A of the first l: the smooth choice (N = (2 eps)^-1/2), so that N stays of order one
+__device__ __forceinline__ double spin_a0(int l0, int m) { return rsqrt(spin_eps2(l0 + 1, m)); }
 
-template <typename T, int K, int NT>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 1) spin_analysis_kernel(GeomDev g, int lmax, int mmax, const c2_t<T> *__restrict__ QF,
-                                                           const c2_t<T> *__restrict__ UF, int64_t fm_stride,
-                                                           c2_t<T> *__restrict__ Eo, c2_t<T> *__restrict__ Bo,
-                                                           int64_t alm_stride, int atomic,
-                                                           const float4 *__restrict__ ckP,
-                                                           const float4 *__restrict__ ckM,
-                                                           const int64_t *__restrict__ blk_ofs) {
-    using V = c2_t<T>;
-    using W = v4_t<T>;
-    constexpr int TL = SpinCfg<T>::TL;
-    constexpr int TPS = NT / TL;
-    static_assert(TPS >= 1 && TPS <= 32 && (32 % TPS) == 0, "bad reduction shape");
-    __shared__ W coef[SCOEF_CH];
-    extern __shared__ __align__(16) unsigned char spin_dyn_smem[];
-    W(*red)[TL][NT] = reinterpret_cast<W(*)[TL][NT]>(spin_dyn_smem);
-    const int m = blockIdx.x, chunk = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
-    const int l0 = m > 2 ? m : 2;
-    const int par0 = (l0 - m) & 1;
-    const int64_t np = g.npairs;
-    const V *Qf = QF + b * fm_stride + (int64_t)m * np * 2;
-    const V *Uf = UF + b * fm_stride + (int64_t)m * np * 2;
-    V *Eout = Eo + b * alm_stride, *Bout = Bo + b * alm_stride;
-
-    T P1[K], P2[K], M1[K], M2[K];
-    SXRep<T> x[K];
-    int ep[K], em[K];
-    V wpe[2][K], wme[2][K], wpb[2][K], wmb[2][K];  // [slot parity][k]
-    bool anyneg = false;
-    auto load_w = [&](int k, int64_t p, bool gp, bool gm) {
-        V qn = Qf[2 * p], qs = Qf[2 * p + 1], un = Uf[2 * p], us = Uf[2 * p + 1];
-        for (int q = 0; q < 2; ++q) {
-            // slot parity q corresponds to l-m parity q ^ par0
-            T eps = ((q ^ par0) & 1) ? (T)-1 : (T)1;
-            V a1, a2, a3, a4;
-            spin_weights<V, T>(qn, qs, un, us, eps, a1, a2, a3, a4);
-            const V z = mk2((T)0, (T)0);
-            wpe[q][k] = gp ? a1 : z;
-            wpb[q][k] = gp ? a3 : z;
-            wme[q][k] = gm ? a2 : z;
-            wmb[q][k] = gm ? a4 : z;
-        }
-    };
+// Step coefficients of rows l0 .. l0 + SPB - 1 by one warp: cf = (A, A beta) taking rho_l to rho_{l+1}, nl =
+// N_l.  carry: A_{l0}, updated for the next block.  Even rows: A_{l+2} = A_l eps_{l+1}^2 / eps_{l+2}^2, each
+// lane multiplying its two ratios, a scan over the lanes joining them.  Odd rows follow from the row
+// before, A_l A_{l+1} eps_{l+1}^2 = 1, so that rounding cannot drift in that product (it acts like a change
+// of x: two independent chains gave 20 to 100 times the error).
+__device__ __forceinline__ void spin_rows(int l0, int m, int lane, double2 *cf, double *nl, double &carry) {
+    const int l = l0 + 4 * lane;
+    double e[4];
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const int64_t p = (int64_t)chunk * NT * K + (int64_t)k * NT + tid;
-        P1[k] = M1[k] = (T)0;
-        if (p < np) {
-            x[k].load(g, p);
-            spin_start<T>(g, m, p, P2[k], ep[k], M2[k], em[k]);
-            load_w(k, p, ep[k] >= 0, em[k] >= 0);
-            anyneg |= (ep[k] < 0) || (em[k] < 0);
-        } else {
-            x[k].zero();
-            P2[k] = M2[k] = (T)0;
-            ep[k] = em[k] = 0;
-            for (int q = 0; q < 2; ++q) wpe[q][k] = wme[q][k] = wpb[q][k] = wmb[q][k] = mk2((T)0, (T)0);
+    for (int i = 0; i < 4; ++i) e[i] = spin_eps2(l + 1 + i, m);
+    const double q = e[0] / e[1];
+    double pe = q * (e[2] / e[3]);  // A_{l+4} / A_l
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double a = __shfl_up_sync(0xffffffffu, pe, o);
+        if (lane >= o) pe *= a;
+    }
+    double xe = __shfl_up_sync(0xffffffffu, pe, 1);
+    if (lane == 0) xe = 1.0;
+    double A[4];
+    A[0] = carry * xe;
+    A[1] = 1.0 / (e[0] * A[0]);
+    A[2] = A[0] * q;
+    A[3] = 1.0 / (e[2] * A[2]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double dl = (double)(l + i);
+        cf[4 * lane + i] = make_double2(A[i], A[i] * (2.0 * m) / (dl * (dl + 1.0)));
+        nl[4 * lane + i] = sqrt(0.5 * A[i]);
+    }
+    carry *= __shfl_sync(0xffffffffu, pe, 31);
+}
+
+enum { CLEAN = 0, MIXED = 1, DEAD = 2 };  // no / some / every value of the warp's group has e < 0
+
+// U ring pairs per lane of one warp: pair 32 (grp U + u) + lane.  (p1, m1) at l, (p0, m0) at l - 1
+template <int U> struct State {
+    double p1[U], p0[U], m1[U], m0[U], x[U];
+    int ep[U], em[U];
+};
+
+template <int U> __device__ __forceinline__ void start_group(const GeomDev &g, int m, int l0, int grp, int lane, State<U> &S) {
+    const double inv = 1.0 / sqrt(0.5 * spin_a0(l0, m));  // 1 / N_{l0}
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int64_t p = (int64_t)(grp * U + u) * 32 + lane;
+        S.p1[u] = S.p0[u] = S.m1[u] = S.m0[u] = S.x[u] = 0.0;
+        S.ep[u] = S.em[u] = 0;
+        if (p < g.npairs) {
+            S.x[u] = g.pair_x[p];
+            spin_start64(g, m, p, S.p1[u], S.ep[u], S.m1[u], S.em[u]);
+            S.p1[u] *= inv;
+            S.m1[u] *= inv;
         }
     }
-    int rb = 0;
-    for (int lb = l0; lb <= lmax; lb += TL) {
-        const int lrel = lb - l0;
-        if ((lrel % SCOEF_CH) == 0) {
-            __syncthreads();
-            for (int i = tid; i < SCOEF_CH; i += NT) {
-                double a, bb, c;
-                spin_coef(lb + i, m, l0, lmax, a, bb, c);
-                coef[i] = mk4((T)a, (T)bb, (T)c, (T)0);
-            }
-            __syncthreads();
-            if constexpr (sizeof(T) == 4) {
-                if (ckP != nullptr && lrel > 0) {  // re-anchor both recursions on the FP64 states
-                    const int64_t row = (blk_ofs[m] + lrel / SCOEF_CH) * np;
-                    anyneg = false;
+}
+
+// hands (P_l, M_l) to f(u, P, M), then takes the step to l + 1
+template <int U, typename Fn> __device__ __forceinline__ void spin_step(State<U> &S, double2 c, Fn f) {
 #pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        const int64_t p = (int64_t)chunk * NT * K + (int64_t)k * NT + tid;
-                        if (p < np) {
-                            const float4 cp = ckP[row + p], cm = ckM[row + p];
-                            P1[k] = cp.x; P2[k] = cp.y; M1[k] = cm.x; M2[k] = cm.y;
-                            const int np_ = __float_as_int(cp.z), nm_ = __float_as_int(cm.z);
-                            if (np_ != ep[k] || nm_ != em[k]) {
-                                ep[k] = np_;
-                                em[k] = nm_;
-                                load_w(k, p, ep[k] >= 0, em[k] >= 0);
-                            }
-                            anyneg |= (ep[k] < 0) || (em[k] < 0);
-                        }
-                    }
-                }
-            }
+    for (int u = 0; u < U; ++u) {
+        const double p = S.p1[u], q = S.m1[u];
+        f(u, p, q);
+        S.p1[u] = fma(fma(c.x, S.x[u], c.y), p, -S.p0[u]);
+        S.m1[u] = fma(fma(c.x, S.x[u], -c.y), q, -S.m0[u]);
+        S.p0[u] = p;
+        S.m0[u] = q;
+    }
+}
+
+template <int U> __device__ __forceinline__ int mode_of(const State<U> &S) {
+    bool neg = false, live = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        neg |= (S.ep[u] < 0) | (S.em[u] < 0);
+        live |= (S.ep[u] >= 0) | (S.em[u] >= 0);
+    }
+    if (!__any_sync(0xffffffffu, neg)) return CLEAN;
+    return __any_sync(0xffffffffu, live) ? MIXED : DEAD;
+}
+
+__device__ __forceinline__ bool past(double v) { return (__double2hiint(v) & 0x7fffffff) >= 0x4ff00000; }  // |v| >= 2^256
+
+// values that have grown past 2^256 move to the next exponent; upP(u), upM(u) are told.  False when the
+// warp has none.
+template <int U, typename FP, typename FM> __device__ __forceinline__ bool rescale(State<U> &S, FP upP, FM upM) {
+    bool any = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) any |= (S.ep[u] < 0 && past(S.p1[u])) || (S.em[u] < 0 && past(S.m1[u]));
+    if (!__any_sync(0xffffffffu, any)) return false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (S.ep[u] < 0 && past(S.p1[u])) {
+            S.p1[u] *= 0x1p-512;
+            S.p0[u] *= 0x1p-512;
+            ++S.ep[u];
+            upP(u);
         }
-        const W *cf = coef + (lrel % SCOEF_CH);
+        if (S.em[u] < 0 && past(S.m1[u])) {
+            S.m1[u] *= 0x1p-512;
+            S.m0[u] *= 0x1p-512;
+            ++S.em[u];
+            upM(u);
+        }
+    }
+    return true;
+}
+
+// ------------------------------------------------------------------ analysis
+// With eps = (-1)^(l-m), Qe = QN + eps QS, Qo = QN - eps QS (U alike): E += P w + M v, B += -i P w' + i M v',
+// w = -(Qe + i Uo)/2, v = -(Qe - i Uo)/2 and w', v' the same of the other parity.
+template <int U> struct Weights {
+    double2 w[2][U], v[2][U];  // [l - m even, odd]
+};
+
+// TL rows: sums over the group's pairs, added to the warp's row red[row * 4 + (E re, E im, B re, B im)]
+template <bool GATED, int U, int PAR>
+__device__ __forceinline__ void anal_chunk(State<U> &S, const Weights<U> &W, const double2 *cf, double *red, int lane) {
+    double a[16];
 #pragma unroll
-        for (int s = 0; s < TL; ++s) {
-            const W cc = cf[s];
-            T er = 0, ei = 0, br = 0, bi = 0;
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                T tp = cc.z * P2[k], tm = cc.z * M2[k];
-                T vp = fma(cc.x, x[k].mul(P1[k]), fma(cc.y, P1[k], -tp));
-                T vm = fma(cc.x, x[k].mul(M1[k]), fma(-cc.y, M1[k], -tm));
-                P2[k] = P1[k]; P1[k] = vp;
-                M2[k] = M1[k]; M1[k] = vm;
-                const int q = s & 1;
-                er = fma(vp, wpe[q][k].x, fma(vm, wme[q][k].x, er));
-                ei = fma(vp, wpe[q][k].y, fma(vm, wme[q][k].y, ei));
-                br = fma(vp, wpb[q][k].x, fma(vm, wmb[q][k].x, br));
-                bi = fma(vp, wpb[q][k].y, fma(vm, wmb[q][k].y, bi));
+    for (int s = 0; s < 4; ++s) {
+        const int k = (s + PAR) & 1;
+        spin_step(S, cf[s], [&](int u, double p, double q) {
+            if (GATED) {
+                p = S.ep[u] < 0 ? 0.0 : p;
+                q = S.em[u] < 0 ? 0.0 : q;
             }
-            red[rb][s][tid] = mk4(er, ei, br, bi);
-            if ((s & 3) == 3 && __any_sync(0xffffffffu, anyneg)) {
-                anyneg = false;
+            const double2 w = W.w[k][u], v = W.v[k][u], wo = W.w[k ^ 1][u], vo = W.v[k ^ 1][u];
+            double *o = a + 4 * s;
+            o[0] = fma(p, w.x, u ? fma(q, v.x, o[0]) : q * v.x);
+            o[1] = fma(p, w.y, u ? fma(q, v.y, o[1]) : q * v.y);
+            o[2] = fma(p, wo.y, u ? fma(-q, vo.y, o[2]) : -q * vo.y);
+            o[3] = fma(-p, wo.x, u ? fma(q, vo.x, o[3]) : q * vo.x);
+        });
+    }
+    const double t = warp_sums<16>(a, lane);
+    if (!(lane & 1)) red[lane >> 1] += t;
+}
+
+template <int U, int PAR>
+__device__ __forceinline__ void anal_block(State<U> &S, const Weights<U> &W, int n, int &mode, const double2 *cf, double *red, int lane) {
+    int k = 0;
+    while (mode != CLEAN && k < n) {
+        if (mode == DEAD) {
 #pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    bool ch = false;
-                    if (ep[k] < 0 && fabs(P1[k]) > s_huge<T>()) {
-                        P1[k] *= s_down<T>(); P2[k] *= s_down<T>();
-                        ch = (++ep[k] == 0);
-                    }
-                    if (em[k] < 0 && fabs(M1[k]) > s_huge<T>()) {
-                        M1[k] *= s_down<T>(); M2[k] *= s_down<T>();
-                        ++em[k];
-                        if (em[k] == 0) ch = true;
-                    }
-                    if (ch) load_w(k, (int64_t)chunk * NT * K + (int64_t)k * NT + tid, ep[k] >= 0, em[k] >= 0);
-                    anyneg |= (ep[k] < 0) || (em[k] < 0);
-                }
+            for (int s = 0; s < 4; ++s) spin_step(S, cf[k + s], [](int, double, double) {});
+        } else {
+            anal_chunk<true, U, PAR>(S, W, cf + k, red + 4 * k, lane);
+        }
+        k += 4;
+        if (rescale(S, [](int) {}, [](int) {})) mode = mode_of(S);
+    }
+#pragma unroll 1
+    for (; k < n; k += 4) anal_chunk<false, U, PAR>(S, W, cf + k, red + 4 * k, lane);
+}
+
+// One CTA per (order, chunk of ring pairs, map), every warp keeping one group of 32 U pairs in registers
+// over all l
+template <int U, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) spin_analysis64_kernel(GeomDev g, int lmax, const double2 *__restrict__ QF,
+                                                                   const double2 *__restrict__ UF, int64_t fm_stride,
+                                                                   double2 *__restrict__ Eo, double2 *__restrict__ Bo,
+                                                                   int64_t alm_stride, int atomic) {
+    constexpr int NW = NT / 32, ROW = SPB * 4;
+    __shared__ double2 cf[SPB];
+    __shared__ double nl[SPB];
+    extern __shared__ double red[];  // [NW][SPB][4]
+    const int m = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = blockIdx.y * NW + warp;
+    const int ls = m > 2 ? m : 2, par0 = (ls - m) & 1;
+    const int64_t np = g.npairs;
+    const double2 *Qf = QF + b * fm_stride + (int64_t)m * np * 2, *Uf = UF + b * fm_stride + (int64_t)m * np * 2;
+    double2 *E = Eo + b * alm_stride, *B = Bo + b * alm_stride;
+    if (!atomic && tid < 2 && m + tid < ls && m + tid <= lmax)  // E, B are zero for l < 2
+        E[alm_idx(lmax, m + tid, m)] = B[alm_idx(lmax, m + tid, m)] = make_double2(0.0, 0.0);
+    if (ls > lmax) return;
+    State<U> S;
+    Weights<U> W;
+    start_group(g, m, ls, grp, lane, S);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int64_t p = (int64_t)(grp * U + u) * 32 + lane;
+        double2 qn = make_double2(0.0, 0.0), qs = qn, un = qn, us = qn;
+        if (p < np) {
+            qn = Qf[2 * p];
+            qs = Qf[2 * p + 1];
+            un = Uf[2 * p];
+            us = Uf[2 * p + 1];
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const double2 Qe = k ? csub(qn, qs) : cadd(qn, qs), Uo = k ? cadd(un, us) : csub(un, us);
+            W.w[k][u] = make_double2(-0.5 * (Qe.x - Uo.y), -0.5 * (Qe.y + Uo.x));
+            W.v[k][u] = make_double2(-0.5 * (Qe.x + Uo.y), -0.5 * (Qe.y - Uo.x));
+        }
+    }
+    const bool any = (int64_t)grp * U * 32 < np;
+    int mode = mode_of(S);
+    double *mine = red + warp * ROW;
+    double carry = spin_a0(ls, m);
+    for (int l0 = ls; l0 <= lmax; l0 += SPB) {
+        const int n = min(SPB, lmax - l0 + 1), npd = (n + 3) & ~3;
+        if (warp == 0) spin_rows(l0, m, lane, cf, nl, carry);
+        for (int i = lane; i < ROW; i += 32) mine[i] = 0.0;
+        __syncthreads();
+        if (any) {
+            if (par0)
+                anal_block<U, 1>(S, W, npd, mode, cf, mine, lane);
+            else
+                anal_block<U, 0>(S, W, npd, mode, cf, mine, lane);
+        }
+        __syncthreads();
+        for (int i = tid; i < 2 * n; i += NT) {
+            const int row = i >> 1, c = (i & 1) * 2;  // E or B of the row
+            double2 s = make_double2(0.0, 0.0);
+            for (int w = 0; w < NW; ++w) {
+                s.x += red[w * ROW + 4 * row + c];
+                s.y += red[w * ROW + 4 * row + c + 1];
+            }
+            s = cscale(s, nl[row]);
+            double2 *d = (c ? B : E) + alm_idx(lmax, l0 + row, m);
+            if (atomic) {
+                atomicAdd(&d->x, s.x);
+                atomicAdd(&d->y, s.y);
+            } else {
+                *d = s;
             }
         }
         __syncthreads();
-        {
-            const int s = tid / TPS, sub = tid % TPS;
-            T a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-#pragma unroll
-            for (int j = 0; j < TL; ++j) {
-                const W v = red[rb][s][sub + j * TPS];
-                a0 += v.x; a1 += v.y; a2 += v.z; a3 += v.w;
-            }
-#pragma unroll
-            for (int off = TPS / 2; off >= 1; off >>= 1) {
-                a0 += __shfl_xor_sync(0xffffffffu, a0, off);
-                a1 += __shfl_xor_sync(0xffffffffu, a1, off);
-                a2 += __shfl_xor_sync(0xffffffffu, a2, off);
-                a3 += __shfl_xor_sync(0xffffffffu, a3, off);
-            }
-            const int l = lb + s;
-            if (sub == 0 && l <= lmax) {
-                V *de = Eout + alm_idx(lmax, l, m), *db = Bout + alm_idx(lmax, l, m);
-                if (atomic) {
-                    atomicAdd(&de->x, a0); atomicAdd(&de->y, a1);
-                    atomicAdd(&db->x, a2); atomicAdd(&db->y, a3);
-                } else {
-                    *de = mk2(a0, a1);
-                    *db = mk2(a2, a3);
-                }
-            }
-        }
-        rb ^= 1;
-    }
-    // E, B are zero for l < l0 (l < 2 when m < 2)
-    if (chunk == 0 && tid < 2 && m + tid < l0 && m + tid <= lmax) {
-        const int l = m + tid;
-        if (!atomic) {
-            Eout[alm_idx(lmax, l, m)] = mk2((T)0, (T)0);
-            Bout[alm_idx(lmax, l, m)] = mk2((T)0, (T)0);
-        }
     }
 }
 
-template <typename T, int K, int NT>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 4 : 1) spin_synthesis_kernel(GeomDev g, int lmax, int mmax, const c2_t<T> *__restrict__ E,
-                                                            const c2_t<T> *__restrict__ B, int64_t alm_stride,
-                                                            c2_t<T> *__restrict__ QG, c2_t<T> *__restrict__ UG,
-                                                            int64_t gm_stride, const float4 *__restrict__ ckP,
-                                                            const float4 *__restrict__ ckM,
-                                                            const int64_t *__restrict__ blk_ofs) {
-    using V = c2_t<T>;
-    using W = v4_t<T>;
-    __shared__ W coef[SCOEF_CH];
-    __shared__ W aco[SCOEF_CH];  // (A+ = E + iB, A- = E - iB)
-    const int m = blockIdx.x, chunk = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
-    const int l0 = m > 2 ? m : 2;
-    const int par0 = (l0 - m) & 1;
-    const int64_t np = g.npairs;
-    const V *Eb = E + b * alm_stride, *Bb = B + b * alm_stride;
-    V *Qg = QG + b * gm_stride + (int64_t)m * np * 2;
-    V *Ug = UG + b * gm_stride + (int64_t)m * np * 2;
+// ------------------------------------------------------------------ synthesis
+// With A+ = E + iB, A- = E - iB and eps = (-1)^(l-m):
+//   north: Q = -1/2 sum (P A+ + M A-),      U = -i/2 sum (M A- - P A+),
+//   south: Q = -1/2 sum eps (P A- + M A+),  U = -i/2 sum eps (P A- - M A+).
+// The sums of P and M stay apart (their exponents differ), in units of 2^(512 e).
+template <int U> struct Sums {
+    double2 x1[U], x2[U], x3[U], x4[U];  // P A+, M A-, eps P A-, eps M A+
+};
+struct alignas(16) SAlm {
+    double pr, pi, mr, mi;  // N (A+, A-)
+};
+__device__ __forceinline__ void axpy(double2 &s, double v, double r, double i) {
+    s.x = fma(v, r, s.x);
+    s.y = fma(v, i, s.y);
+}
 
-    T P1[K], P2[K], M1[K], M2[K];
-    SXRep<T> x[K];
-    int ep[K], em[K];
-    // X1 = sum P A+, X3 = sum P A-, X2 = sum M A-, X4 = sum M A+, per slot parity
-    V X1[2][K], X2[2][K], X3[2][K], X4[2][K];
-    bool anyneg = false;
+template <int U>
+__device__ __forceinline__ void synth_row(State<U> &S, Sums<U> &A, double2 c, const SAlm &a, bool odd) {
+    spin_step(S, c, [&](int u, double p, double q) {
+        axpy(A.x1[u], p, a.pr, a.pi);
+        axpy(A.x2[u], q, a.mr, a.mi);
+        axpy(A.x3[u], odd ? -p : p, a.mr, a.mi);
+        axpy(A.x4[u], odd ? -q : q, a.pr, a.pi);
+    });
+}
+
+template <int U, int PAR>
+__device__ __forceinline__ void synth_block(State<U> &S, Sums<U> &A, int n, int &mode, const double2 *cf, const SAlm *ac) {
+    int k = 0;
+    while (mode != CLEAN && k < n) {
+        if (mode == DEAD) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const int64_t p = (int64_t)chunk * NT * K + (int64_t)k * NT + tid;
-        P1[k] = M1[k] = (T)0;
-        for (int q = 0; q < 2; ++q) X1[q][k] = X2[q][k] = X3[q][k] = X4[q][k] = mk2((T)0, (T)0);
-        if (p < np) {
-            x[k].load(g, p);
-            spin_start<T>(g, m, p, P2[k], ep[k], M2[k], em[k]);
-            anyneg |= (ep[k] < 0) || (em[k] < 0);
+            for (int s = 0; s < 4; ++s) spin_step(S, cf[k + s], [](int, double, double) {});
         } else {
-            x[k].zero();
-            P2[k] = M2[k] = (T)0;
-            ep[k] = em[k] = 0;
+#pragma unroll
+            for (int s = 0; s < 4; ++s) synth_row(S, A, cf[k + s], ac[k + s], (s + PAR) & 1);
         }
+        k += 4;
+        const auto down = [](double2 &v) { v = cscale(v, 0x1p-512); };
+        const bool up = rescale(
+            S,
+            [&](int u) {
+                down(A.x1[u]);
+                down(A.x3[u]);
+            },
+            [&](int u) {
+                down(A.x2[u]);
+                down(A.x4[u]);
+            });
+        if (up) mode = mode_of(S);
     }
-    for (int lb = l0; lb <= lmax; lb += 4) {
-        const int lrel = lb - l0;
-        if ((lrel % SCOEF_CH) == 0) {
-            __syncthreads();
-            for (int i = tid; i < SCOEF_CH; i += NT) {
-                double a, bb, c;
-                spin_coef(lb + i, m, l0, lmax, a, bb, c);
-                coef[i] = mk4((T)a, (T)bb, (T)c, (T)0);
-                const int l = lb + i;
-                V e = mk2((T)0, (T)0), bv = mk2((T)0, (T)0);
-                if (l <= lmax) {
-                    e = Eb[alm_idx(lmax, l, m)];
-                    bv = Bb[alm_idx(lmax, l, m)];
-                }
-                // E + iB, E - iB
-                aco[i] = mk4(e.x - bv.y, e.y + bv.x, e.x + bv.y, e.y - bv.x);
-            }
-            __syncthreads();
-            if constexpr (sizeof(T) == 4) {
-                if (ckP != nullptr && lrel > 0) {  // re-anchor both recursions on the FP64 states
-                    const int64_t row = (blk_ofs[m] + lrel / SCOEF_CH) * np;
-                    anyneg = false;
+#pragma unroll 1
+    for (; k < n; k += 4) {
 #pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        const int64_t p = (int64_t)chunk * NT * K + (int64_t)k * NT + tid;
-                        if (p < np) {
-                            const float4 cp = ckP[row + p], cm = ckM[row + p];
-                            P1[k] = cp.x; P2[k] = cp.y; M1[k] = cm.x; M2[k] = cm.y;
-                            const int np_ = __float_as_int(cp.z), nm_ = __float_as_int(cm.z);
-                            if (np_ != ep[k]) {  // accumulators are kept in units of 2^(64 e)
-                                const float f = ldexpf(1.0f, 64 * max(-3, ep[k] - np_));
-                                for (int q = 0; q < 2; ++q) { X1[q][k] = cscale(X1[q][k], f); X3[q][k] = cscale(X3[q][k], f); }
-                                ep[k] = np_;
-                            }
-                            if (nm_ != em[k]) {
-                                const float f = ldexpf(1.0f, 64 * max(-3, em[k] - nm_));
-                                for (int q = 0; q < 2; ++q) { X2[q][k] = cscale(X2[q][k], f); X4[q][k] = cscale(X4[q][k], f); }
-                                em[k] = nm_;
-                            }
-                            anyneg |= (ep[k] < 0) || (em[k] < 0);
-                        }
-                    }
-                }
+        for (int s = 0; s < 4; ++s) synth_row(S, A, cf[k + s], ac[k + s], (s + PAR) & 1);
+    }
+}
+
+// One warp per (group of 32 U ring pairs, order, map), as in the scalar synthesis
+template <int U, int MINB>
+__global__ void __launch_bounds__(32, MINB) spin_synthesis64_kernel(GeomDev g, int lmax, const double2 *__restrict__ E,
+                                                                   const double2 *__restrict__ B, int64_t alm_stride,
+                                                                   double2 *__restrict__ QG, double2 *__restrict__ UG,
+                                                                   int64_t gm_stride) {
+    __shared__ double2 cf[SPB];
+    __shared__ double nl[SPB];
+    __shared__ SAlm ac[SPB];
+    const int lane = threadIdx.x, grp = blockIdx.x, m = blockIdx.y;
+    const int ls = m > 2 ? m : 2, par0 = (ls - m) & 1;
+    const int64_t np = g.npairs;
+    const double2 *Eb = E + blockIdx.z * alm_stride, *Bb = B + blockIdx.z * alm_stride;
+    State<U> S;
+    Sums<U> A;
+    start_group(g, m, ls, grp, lane, S);
+#pragma unroll
+    for (int u = 0; u < U; ++u) A.x1[u] = A.x2[u] = A.x3[u] = A.x4[u] = make_double2(0.0, 0.0);
+    int mode = mode_of(S);
+    double carry = spin_a0(ls, m);
+    for (int l0 = ls; l0 <= lmax; l0 += SPB) {
+        const int n = min(SPB, lmax - l0 + 1), npd = (n + 3) & ~3;
+        __syncwarp();
+        spin_rows(l0, m, lane, cf, nl, carry);
+        __syncwarp();
+#pragma unroll
+        for (int k = lane; k < SPB; k += 32) {
+            SAlm v{};
+            if (k < n) {
+                const double2 e = Eb[alm_idx(lmax, l0 + k, m)], bv = Bb[alm_idx(lmax, l0 + k, m)];
+                const double N = nl[k];
+                v = {N * (e.x - bv.y), N * (e.y + bv.x), N * (e.x + bv.y), N * (e.y - bv.x)};
             }
+            ac[k] = v;
         }
-        const int i0 = lrel % SCOEF_CH;
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const W cc = coef[i0 + s], av = aco[i0 + s];
-            const int q = s & 1;
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                T tp = cc.z * P2[k], tm = cc.z * M2[k];
-                T vp = fma(cc.x, x[k].mul(P1[k]), fma(cc.y, P1[k], -tp));
-                T vm = fma(cc.x, x[k].mul(M1[k]), fma(-cc.y, M1[k], -tm));
-                P2[k] = P1[k]; P1[k] = vp;
-                M2[k] = M1[k]; M1[k] = vm;
-                X1[q][k].x = fma(vp, av.x, X1[q][k].x); X1[q][k].y = fma(vp, av.y, X1[q][k].y);
-                X3[q][k].x = fma(vp, av.z, X3[q][k].x); X3[q][k].y = fma(vp, av.w, X3[q][k].y);
-                X2[q][k].x = fma(vm, av.z, X2[q][k].x); X2[q][k].y = fma(vm, av.w, X2[q][k].y);
-                X4[q][k].x = fma(vm, av.x, X4[q][k].x); X4[q][k].y = fma(vm, av.y, X4[q][k].y);
-            }
-        }
-        if (__any_sync(0xffffffffu, anyneg)) {
-            anyneg = false;
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                if (ep[k] < 0 && fabs(P1[k]) > s_huge<T>()) {
-                    P1[k] *= s_down<T>(); P2[k] *= s_down<T>();
-                    for (int q = 0; q < 2; ++q) {
-                        X1[q][k] = cscale(X1[q][k], s_down<T>());
-                        X3[q][k] = cscale(X3[q][k], s_down<T>());
-                    }
-                    ++ep[k];
-                }
-                if (em[k] < 0 && fabs(M1[k]) > s_huge<T>()) {
-                    M1[k] *= s_down<T>(); M2[k] *= s_down<T>();
-                    for (int q = 0; q < 2; ++q) {
-                        X2[q][k] = cscale(X2[q][k], s_down<T>());
-                        X4[q][k] = cscale(X4[q][k], s_down<T>());
-                    }
-                    ++em[k];
-                }
-                anyneg |= (ep[k] < 0) || (em[k] < 0);
-            }
-        }
+        __syncwarp();
+        if (par0)
+            synth_block<U, 1>(S, A, npd, mode, cf, ac);
+        else
+            synth_block<U, 0>(S, A, npd, mode, cf, ac);
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const int64_t p = (int64_t)chunk * NT * K + (int64_t)k * NT + tid;
+    for (int u = 0; u < U; ++u) {
+        const int64_t p = (int64_t)(grp * U + u) * 32 + lane;
         if (p >= np) continue;
-        const T fp = ep[k] == 0 ? (T)1 : (T)ldexp(1.0, SpinCfg<T>::SE * ep[k]);
-        const T fm = em[k] == 0 ? (T)1 : (T)ldexp(1.0, SpinCfg<T>::SE * em[k]);
-        // slot parity q has l-m parity q ^ par0: eps = +1 for even l-m
-        const int qe = par0, qo = par0 ^ 1;
-        V x1e = cscale(X1[qe][k], fp), x1o = cscale(X1[qo][k], fp), x3e = cscale(X3[qe][k], fp), x3o = cscale(X3[qo][k], fp);
-        V x2e = cscale(X2[qe][k], fm), x2o = cscale(X2[qo][k], fm), x4e = cscale(X4[qe][k], fm), x4o = cscale(X4[qo][k], fm);
-        const T h = (T)-0.5;
-        // Q_N = -1/2 sum (X1 + X2); Q_S = -1/2 sum eps (X3 + X4)
-        V qn = cscale(cadd(cadd(x1e, x2e), cadd(x1o, x2o)), h);
-        V qs = cscale(csub(cadd(x3e, x4e), cadd(x3o, x4o)), h);
-        // U_N = -1/2 i sum (X2 - X1); U_S = -1/2 i sum eps (X3 - X4)
-        V dn = cadd(csub(x2e, x1e), csub(x2o, x1o));
-        V ds = csub(csub(x3e, x4e), csub(x3o, x4o));
-        V un = mk2(-h * dn.y, h * dn.x);
-        V us = mk2(-h * ds.y, h * ds.x);
-        Qg[2 * p] = qn;
-        Qg[2 * p + 1] = qs;
-        Ug[2 * p] = un;
-        Ug[2 * p + 1] = us;
+        const double fp = S.ep[u] == 0 ? 1.0 : ldexp(1.0, 512 * S.ep[u]), fm = S.em[u] == 0 ? 1.0 : ldexp(1.0, 512 * S.em[u]);
+        const double2 x1 = cscale(A.x1[u], fp), x3 = cscale(A.x3[u], fp), x2 = cscale(A.x2[u], fm), x4 = cscale(A.x4[u], fm);
+        const double2 dn = csub(x2, x1), ds = csub(x3, x4);
+        const int64_t o = blockIdx.z * gm_stride + ((int64_t)m * np + p) * 2;
+        QG[o] = cscale(cadd(x1, x2), -0.5);
+        QG[o + 1] = cscale(cadd(x3, x4), -0.5);
+        UG[o] = make_double2(0.5 * dn.y, -0.5 * dn.x);  // -i/2 z
+        UG[o + 1] = make_double2(0.5 * ds.y, -0.5 * ds.x);
     }
 }
 
-template <typename T, int K, int NT>
-static int run_spin_analysis(const GeomDev &g, int nmaps, int lmax, int mmax, const c2_t<T> *QF, const c2_t<T> *UF,
-                             c2_t<T> *E, c2_t<T> *B, cudaStream_t st, const float4 *ckP, const float4 *ckM,
-                             const int64_t *bo) {
-    const int64_t per = (int64_t)K * NT;
-    const int nchunks = (int)((g.npairs + per - 1) / per);
-    const int64_t fm_stride = (int64_t)(mmax + 1) * g.npairs * 2;
-    const int64_t alm_stride = alm_size(lmax, mmax);
+// ------------------------------------------------------------------ launches
+template <int U, int NT, int MINB>
+static int run_analysis(const hb_plan *p, int nmaps, const double2 *QF, const double2 *UF, double2 *E, double2 *B, cudaStream_t st) {
+    const int64_t np = p->g->d.npairs, as = alm_size(p->lmax, p->mmax), per = (int64_t)U * NT;
+    const int nchunks = (int)((np + per - 1) / per);
     if (nchunks > 1) {
-        HB_CUDA_TRY(cudaMemsetAsync(E, 0, sizeof(c2_t<T>) * alm_stride * nmaps, st));
-        HB_CUDA_TRY(cudaMemsetAsync(B, 0, sizeof(c2_t<T>) * alm_stride * nmaps, st));
+        HB_CUDA_TRY(cudaMemsetAsync(E, 0, sizeof(double2) * as * nmaps, st));
+        HB_CUDA_TRY(cudaMemsetAsync(B, 0, sizeof(double2) * as * nmaps, st));
     }
-    const int smem = 2 * SpinCfg<T>::TL * NT * (int)sizeof(v4_t<T>);
-    HB_CUDA_TRY(cudaFuncSetAttribute(spin_analysis_kernel<T, K, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    dim3 grid((unsigned)(mmax + 1), (unsigned)nchunks, (unsigned)nmaps);
-    spin_analysis_kernel<T, K, NT><<<grid, NT, smem, st>>>(g, lmax, mmax, QF, UF, fm_stride, E, B, alm_stride,
-                                                            nchunks > 1, ckP, ckM, bo);
+    const int smem = NT / 32 * SPB * 4 * (int)sizeof(double);
+    HB_CUDA_TRY(cudaFuncSetAttribute(spin_analysis64_kernel<U, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    dim3 grid((unsigned)(p->mmax + 1), (unsigned)nchunks, (unsigned)nmaps);
+    spin_analysis64_kernel<U, NT, MINB><<<grid, NT, smem, st>>>(p->g->d, p->lmax, QF, UF, (int64_t)(p->mmax + 1) * np * 2, E, B, as,
+                                                                nchunks > 1);
+    HB_CHECK_LAUNCH();
+    return HB_OK;
+}
+template <int U, int MINB>
+static int run_synthesis(const hb_plan *p, int nmaps, const double2 *E, const double2 *B, double2 *QG, double2 *UG, cudaStream_t st) {
+    const int64_t np = p->g->d.npairs;
+    dim3 grid((unsigned)((np + 32 * U - 1) / (32 * U)), (unsigned)(p->mmax + 1), (unsigned)nmaps);
+    spin_synthesis64_kernel<U, MINB><<<grid, 32, 0, st>>>(p->g->d, p->lmax, E, B, alm_size(p->lmax, p->mmax), QG, UG,
+                                                              (int64_t)(p->mmax + 1) * np * 2);
     HB_CHECK_LAUNCH();
     return HB_OK;
 }
 
-template <typename T, int K, int NT>
-static int run_spin_synthesis(const GeomDev &g, int nmaps, int lmax, int mmax, const c2_t<T> *E, const c2_t<T> *B,
-                              c2_t<T> *QG, c2_t<T> *UG, cudaStream_t st, const float4 *ckP, const float4 *ckM,
-                              const int64_t *bo) {
-    const int64_t per = (int64_t)K * NT;
-    const int nchunks = (int)((g.npairs + per - 1) / per);
-    const int64_t gm_stride = (int64_t)(mmax + 1) * g.npairs * 2;
-    const int64_t alm_stride = alm_size(lmax, mmax);
-    dim3 grid((unsigned)(mmax + 1), (unsigned)nchunks, (unsigned)nmaps);
-    spin_synthesis_kernel<T, K, NT><<<grid, NT, 0, st>>>(g, lmax, mmax, E, B, alm_stride, QG, UG, gm_stride, ckP,
-                                                          ckM, bo);
-    HB_CHECK_LAUNCH();
-    return HB_OK;
+// Pairs per lane: the synthesis reads 48 bytes of coefficients per l and warp from shared memory, as long
+// as the operations of two pairs; four pairs (10 warps per SM) 3.88 ms at nside 1024 where two (16 warps)
+// take 4.09, but 464 us at nside 256, lmax 700 (three maps) where two take 439.  The analysis: four 5.35 ms
+// and 636 us, two 6.06 ms and 667 us.  Below 256 pairs one, to spread over more warps.
+static int spin_analysis64(const hb_plan *p, int nmaps, const double2 *QF, const double2 *UF, double2 *E, double2 *B, cudaStream_t st) {
+    if (p->g->d.npairs >= 256) return run_analysis<4, 128, 3>(p, nmaps, QF, UF, E, B, st);
+    return run_analysis<1, 128, 4>(p, nmaps, QF, UF, E, B, st);
 }
-
-template <typename T>
-static int spin_analysis_t(const GeomDev &g, int nmaps, int lmax, int mmax, const c2_t<T> *QF, const c2_t<T> *UF,
-                           c2_t<T> *E, c2_t<T> *B, cudaStream_t st, const float4 *ckP, const float4 *ckM,
-                           const int64_t *bo) {
-    if (g.npairs >= 256) return run_spin_analysis<T, 2, 128>(g, nmaps, lmax, mmax, QF, UF, E, B, st, ckP, ckM, bo);
-    if (g.npairs >= 128) return run_spin_analysis<T, 2, 64>(g, nmaps, lmax, mmax, QF, UF, E, B, st, ckP, ckM, bo);
-    return run_spin_analysis<T, 1, 64>(g, nmaps, lmax, mmax, QF, UF, E, B, st, ckP, ckM, bo);
-}
-
-template <typename T>
-static int spin_synthesis_t(const GeomDev &g, int nmaps, int lmax, int mmax, const c2_t<T> *E, const c2_t<T> *B,
-                            c2_t<T> *QG, c2_t<T> *UG, cudaStream_t st, const float4 *ckP, const float4 *ckM,
-                            const int64_t *bo) {
-    if (g.npairs >= 256) return run_spin_synthesis<T, 2, 128>(g, nmaps, lmax, mmax, E, B, QG, UG, st, ckP, ckM, bo);
-    if (g.npairs >= 128) return run_spin_synthesis<T, 2, 64>(g, nmaps, lmax, mmax, E, B, QG, UG, st, ckP, ckM, bo);
-    return run_spin_synthesis<T, 1, 64>(g, nmaps, lmax, mmax, E, B, QG, UG, st, ckP, ckM, bo);
+static int spin_synthesis64(const hb_plan *p, int nmaps, const double2 *E, const double2 *B, double2 *QG, double2 *UG, cudaStream_t st) {
+    if (p->g->d.npairs >= 1024) return run_synthesis<4, 10>(p, nmaps, E, B, QG, UG, st);
+    if (p->g->d.npairs >= 256) return run_synthesis<2, 16>(p, nmaps, E, B, QG, UG, st);
+    return run_synthesis<1, 16>(p, nmaps, E, B, QG, UG, st);
 }
 
 int launch_spin_analysis32(const hb_plan *p, int nmaps, const float2 *QF, const float2 *UF, float2 *E, float2 *B, cudaStream_t st);
@@ -494,18 +446,18 @@ int launch_spin_synthesis32(const hb_plan *p, int nmaps, const float2 *E, const 
 
 int launch_spin_analysis(const hb_plan *p, int precision, int nmaps, const void *QFm, const void *UFm, void *E, void *B,
                          cudaStream_t st) {
+    HB_NVTX("spin_analysis");
     if (precision == 32)
         return launch_spin_analysis32(p, nmaps, (const float2 *)QFm, (const float2 *)UFm, (float2 *)E, (float2 *)B, st);
-    return spin_analysis_t<double>(p->g->d, nmaps, p->lmax, p->mmax, (const double2 *)QFm, (const double2 *)UFm, (double2 *)E,
-                                   (double2 *)B, st, nullptr, nullptr, nullptr);
+    return spin_analysis64(p, nmaps, (const double2 *)QFm, (const double2 *)UFm, (double2 *)E, (double2 *)B, st);
 }
 
 int launch_spin_synthesis(const hb_plan *p, int precision, int nmaps, const void *E, const void *B, void *QGm, void *UGm,
                           cudaStream_t st) {
+    HB_NVTX("spin_synthesis");
     if (precision == 32)
         return launch_spin_synthesis32(p, nmaps, (const float2 *)E, (const float2 *)B, (float2 *)QGm, (float2 *)UGm, st);
-    return spin_synthesis_t<double>(p->g->d, nmaps, p->lmax, p->mmax, (const double2 *)E, (const double2 *)B, (double2 *)QGm,
-                                    (double2 *)UGm, st, nullptr, nullptr, nullptr);
+    return spin_synthesis64(p, nmaps, (const double2 *)E, (const double2 *)B, (double2 *)QGm, (double2 *)UGm, st);
 }
 
 }  // namespace hb

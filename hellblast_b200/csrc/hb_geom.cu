@@ -478,7 +478,7 @@ int hb_geom_fft_launches(const hb_geom *g, int precision, int *n) {
     const GeomDev &d = g->d;
     const int ncls = precision == 32 ? d.rest_n_cls : d.n_cls;
     const int nm = precision == 32 ? merged_classes(ncls, d.rest_L, d.rest_first) : merged_classes(ncls, d.cls_L, d.cls_first);
-    *n = (precision == 32 ? d.pk_n_cls : 0) + ncls - (nm > 1 ? nm - 1 : 0);
+    *n = (precision == 32 ? pk_launches(d, 1) : 0) + ncls - (nm > 1 ? nm - 1 : 0);
     return HB_OK;
 }
 

@@ -245,4 +245,6 @@ int launch_pk_synthesis(const GeomDev &g, int nmaps, const float2 *Gm, int mmax,
                         const double *w, bool apply_w, bool mdouble, int flags, cudaStream_t st);
 int launch_pk_analysis(const GeomDev &g, int nmaps, const float *maps, int64_t map_stride, const double *w,
                        float2 *Fm, int mmax, int flags, bool unit_w, bool mdouble, cudaStream_t st, bool mblk);
+// launches the pair-packed classes make per direction for a batch of nmaps
+int pk_launches(const GeomDev &g, int nmaps);
 }  // namespace hb

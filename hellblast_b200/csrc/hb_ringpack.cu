@@ -131,10 +131,10 @@ template <int LOGL> __device__ __forceinline__ float2 pk_table_entry(int i, int 
 // phases exp(i pi e / n) from gph (a Bluestein ring's phase block) or, for n = L, from gtw
 __device__ __forceinline__ float2 pk_ld(const float2 *p) { return __ldg(p); }
 template <int LOGL>
-__device__ __forceinline__ PkTab pk_tables(float2 *base, const float2 *__restrict__ gtw, const float2 *__restrict__ gph) {
+__device__ __forceinline__ PkTab pk_tables(float2 *base, int tid, const float2 *__restrict__ gtw, const float2 *__restrict__ gph) {
     using C = PkCfg<LOGL>;
     float2 *tw1 = base, *tw4 = tw1 + C::TWP, *tws = tw4 + C::TWP, *phf = tws + C::TWS, *phc = phf + 64;
-    for (int i = threadIdx.x; i < C::TAB; i += C::NT) base[i] = pk_ld((gph && i >= C::TWB) ? gph + (i - C::TWB) : gtw + i);
+    for (int i = tid; i < C::TAB; i += C::NT) base[i] = pk_ld((gph && i >= C::TWB) ? gph + (i - C::TWB) : gtw + i);
     return {tw1, tw4, tws, phf, phc};
 }
 
@@ -286,7 +286,7 @@ __device__ __forceinline__ void pk_csum(int k, int n, int s, int mmax, float cha
 // (-1)^(s j) over the aliases m = k + j n; put(k, Z_k) for every k < n (CTA-strided loops of NT
 // threads).  c_m = 1 for m = 0, dbl for m > 0.  P2: n is a power of two.
 template <int NT, bool P2, class Ld, class Put>
-__device__ __forceinline__ void pk_fold(int n, int s, int mmax, float dbl, const PkTab &T, Ld &&ld, Put &&put) {
+__device__ __forceinline__ void pk_fold(int tid, int n, int s, int mmax, float dbl, const PkTab &T, Ld &&ld, Put &&put) {
     const float chalf = 0.5f * dbl;
     const float sg = (s & 1) ? -1.f : 1.f;
     const PkMod mod2n{2 * n, 1.f / (float)(2 * n)};
@@ -298,21 +298,21 @@ __device__ __forceinline__ void pk_fold(int n, int s, int mmax, float dbl, const
     };
     if (mmax < n) {  // at most one harmonic per residue class (the equatorial belt when mmax < 4 nside)
 #pragma unroll 4
-        for (int k = threadIdx.x + 1; k < n / 2; k += NT) {
+        for (int k = tid + 1; k < n / 2; k += NT) {
             const float4 a = k <= mmax ? ld(k) : make_float4(0.f, 0.f, 0.f, 0.f);
             const float4 c = n - k <= mmax ? ld(n - k) : make_float4(0.f, 0.f, 0.f, 0.f);
             put_pair(k, cscale(f4lo(a), chalf), cscale(f4hi(a), chalf), cscale(f4lo(c), chalf),
                      cscale(f4hi(c), chalf));
         }
     } else {
-        for (int k = threadIdx.x + 1; k < n / 2; k += NT) {
+        for (int k = tid + 1; k < n / 2; k += NT) {
             float2 SkN, SkS, SmN, SmS;
             csum(k, SkN, SkS);
             csum(n - k, SmN, SmS);
             put_pair(k, SkN, SkS, SmN, SmS);
         }
     }
-    if (threadIdx.x == 0) {  // bins 0 and n/2: c_m Re(G(m) exp(i m phi0)) of their classes
+    if (tid == 0) {  // bins 0 and n/2: c_m Re(G(m) exp(i m phi0)) of their classes
         float aN = 0.f, aS = 0.f, sj = 1.f;
         for (int m = 0; m <= mmax; m += n) {
             const float4 v = ld(m);
@@ -334,22 +334,21 @@ __device__ __forceinline__ void pk_fold(int n, int s, int mmax, float dbl, const
 // rings of each pair.  c_m = 1 for m = 0 and `dbl` (2: real-field synthesis, 1: adjoint of the
 // weighted analysis) for m > 0; apply_w multiplies ring r by scale 2 pi w_r / n (no 2 pi with
 // HB_F_NO2PI).  BLU: n is not a power of two and L is its Bluestein length.
+// (one pair by NT threads tid over PkCfg::SMEM bytes at pk_smem; every thread of the CTA takes the same
+// barriers)
 template <int LOGL, bool BLU>
-__global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
-    ring_pair_synthesis_kernel(GeomDev g, const int32_t *__restrict__ pairs, const float4 *__restrict__ Gm,
-                               int64_t gm_stride4, int mmax, float *__restrict__ maps, int64_t map_stride,
-                               const double *__restrict__ w, int apply_w, int mdouble, int flags) {
+__device__ __forceinline__ void pair_synthesis(const GeomDev &g, int pair, int bm, int tid, float2 *pk_smem, const float4 *__restrict__ Gm,
+                                               int64_t gm_stride4, int mmax, float *__restrict__ maps, int64_t map_stride,
+                                               const double *__restrict__ w, int apply_w, int mdouble, int flags) {
     using C = PkCfg<LOGL>;
     constexpr int L = C::L, NT = C::NT;
-    extern __shared__ __align__(16) float2 pk_smem[];
     float2 *buf = pk_smem;
-    const int pair = pairs[BLU ? blockIdx.y : blockIdx.x], bm = BLU ? blockIdx.x : blockIdx.y;
     const int rN = g.pair_ring[2 * pair], rS = g.pair_ring[2 * pair + 1];
     const int n = BLU ? g.nphi[rN] : L;
     // Bluestein tables: chirp spectrum bt[0, L), chirp ch[t] = exp(-i pi t^2 / n) for t < n, then
     // the ring's phase block
     const float2 *bt = BLU ? g.pkb_bt + g.pkb_bt_ofs[pair] : nullptr, *ch = BLU ? bt + L : nullptr;
-    const PkTab T = pk_tables<LOGL>(pk_smem + C::BUF, g.pk_tw + g.pk_tw_ofs[LOGL], BLU ? bt + L + L / 2 : nullptr);
+    const PkTab T = pk_tables<LOGL>(pk_smem + C::BUF, tid, g.pk_tw + g.pk_tw_ofs[LOGL], BLU ? bt + L + L / 2 : nullptr);
     const int s = (flags & HB_F_NOPHASE) ? 0 : pk_shift(g.phi0_pi[rN], n);
     const int64_t np = g.npairs;
     const float4 *gin = Gm + bm * gm_stride4 + pair;  // (m, pair) entry at gin[m * np]
@@ -367,9 +366,9 @@ __global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
         if (!hasS) v.z = v.w = 0.f;
         return v;
     };
-    pk_fold<NT, !BLU>(n, s, mmax, dbl, T, ld, put);
+    pk_fold<NT, !BLU>(tid, n, s, mmax, dbl, T, ld, put);
     if (BLU)  // zero padding of the convolution (the first pass reads points below L/2 only)
-        for (int k = n + threadIdx.x; k < L / 2; k += NT) buf[pk_pad(k)] = make_float2(0.f, 0.f);
+        for (int k = n + tid; k < L / 2; k += NT) buf[pk_pad(k)] = make_float2(0.f, 0.f);
     __syncthreads();
     const double sc2 = (flags & HB_F_NO2PI) ? 1.0 : 6.283185307179586476925286766559;
     const float psN = apply_w ? (float)(sc2 * w[rN] / (double)n) : 1.f;
@@ -378,18 +377,18 @@ __global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
     float *fS = hasS ? maps + bm * map_stride + g.ofs[rS] : nullptr;
     auto lds = [&](int, int ip) -> float2 { return buf[ip]; };
     if constexpr (!BLU) {
-        pk_run<LOGL, true, false, false>(buf, T, threadIdx.x, lds, [&](int i, int, float2 v) {
+        pk_run<LOGL, true, false, false>(buf, T, tid, lds, [&](int i, int, float2 v) {
             fN[i] = v.x * psN;
             if (fS) fS[i] = v.y * psS;
         });
     } else {
         // forward FFT_L (input zero from L/2 on), times the chirp spectrum
-        pk_run<LOGL, false, true, false>(buf, T, threadIdx.x, lds, [&](int, int ip, float2 v) { buf[ip] = v; });
+        pk_run<LOGL, false, true, false>(buf, T, tid, lds, [&](int, int ip, float2 v) { buf[ip] = v; });
         __syncthreads();
-        for (int i = threadIdx.x; i < L; i += NT) buf[pk_pad(i)] = cmul(buf[pk_pad(i)], __ldg(bt + i));
+        for (int i = tid; i < L; i += NT) buf[pk_pad(i)] = cmul(buf[pk_pad(i)], __ldg(bt + i));
         __syncthreads();
         // inverse FFT_L, points below L/2 only; times the chirp, conjugated, to the two rings
-        pk_run<LOGL, true, false, true>(buf, T, threadIdx.x, lds, [&](int i, int, float2 v) {
+        pk_run<LOGL, true, false, true>(buf, T, tid, lds, [&](int i, int, float2 v) {
             if (i < n) {
                 const float2 z = cconj(cmul(__ldg(ch + i), v));
                 fN[i] = z.x * psN;
@@ -399,6 +398,16 @@ __global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
     }
 }
 
+template <int LOGL, bool BLU>
+__global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
+    ring_pair_synthesis_kernel(GeomDev g, const int32_t *__restrict__ pairs, const float4 *__restrict__ Gm,
+                               int64_t gm_stride4, int mmax, float *__restrict__ maps, int64_t map_stride,
+                               const double *__restrict__ w, int apply_w, int mdouble, int flags) {
+    extern __shared__ __align__(16) float2 pk_smem[];
+    pair_synthesis<LOGL, BLU>(g, pairs[BLU ? blockIdx.y : blockIdx.x], BLU ? blockIdx.x : blockIdx.y, threadIdx.x, pk_smem, Gm,
+                              gm_stride4, mmax, maps, map_stride, w, apply_w, mdouble, flags);
+}
+
 // The orders of the two rings from the spectrum Z of z = f_N + i f_S (Zf(k), k < n):
 // D_N = (Z[k] + conj Z[n-k]) / 2 and D_S = (Z[k] - conj Z[n-k]) / (2 i), times exp(-i pi s k / n)
 // and the ring scales scN / scS, stored through at(m) for every m <= mlim of residue class k
@@ -406,13 +415,13 @@ __global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
 // with mdouble; the orders mlim < m <= mmax are zero.  CTA-strided loops of NT threads; P2: n is
 // a power of two.
 template <int NT, bool P2, class Zfn, class At>
-__device__ __forceinline__ void pk_emit(int n, int s, int mmax, int mlim, bool mdouble, float scN, float scS,
+__device__ __forceinline__ void pk_emit(int tid, int n, int s, int mmax, int mlim, bool mdouble, float scN, float scS,
                                         const PkTab &T, Zfn &&Zf, At &&at) {
     const PkMod mod2n{2 * n, 1.f / (float)(2 * n)};
     auto pidx = [&](int k) -> int { return P2 ? ((s * k) & (2 * n - 1)) : mod2n(s * k); };
     // HB_F_NOFOLD: the orders the ring does not resolve (m >= n) are zero, not left unwritten
-    for (int m = mlim + 1 + threadIdx.x; m <= mmax; m += NT) at(m) = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = threadIdx.x; k <= n / 2; k += NT) {
+    for (int m = mlim + 1 + tid; m <= mmax; m += NT) at(m) = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = tid; k <= n / 2; k += NT) {
         const float2 zk = Zf(k), zc = k == 0 ? zk : Zf(n - k);
         // D_N = (Z[k] + conj Z[n-k]) / 2, D_S = (Z[k] - conj Z[n-k]) / (2 i)
         const float2 dN = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y - zc.y));
@@ -443,22 +452,18 @@ __device__ __forceinline__ void pk_emit(int n, int s, int mmax, int mlim, bool m
 // (adjoint of the synthesis), else 1; HB_F_NOFOLD keeps m < n.  Lanes take consecutive orders, so
 // in the blocked layout 8 lanes fill one 128-byte line.
 template <int LOGL, bool BLU>
-__global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
-    ring_pair_analysis_kernel(GeomDev g, const int32_t *__restrict__ pairs, const float *__restrict__ maps,
-                              int64_t map_stride, const double *__restrict__ w, float4 *__restrict__ Fm,
-                              int64_t fm_stride4, int mmax, int flags, int unit_w, int mdouble, int mblk) {
+__device__ __forceinline__ void pair_analysis(const GeomDev &g, int pair, int bm, int tid, float2 *pk_smem, const float *__restrict__ maps,
+                                              int64_t map_stride, const double *__restrict__ w, float4 *__restrict__ Fm,
+                                              int64_t fm_stride4, int mmax, int flags, int unit_w, int mdouble, int mblk) {
     using C = PkCfg<LOGL>;
     constexpr int L = C::L, NT = C::NT;
-    extern __shared__ __align__(16) float2 pk_smem[];
     float2 *buf = pk_smem;
-    const bool mf = BLU && mblk;
-    const int pair = pairs[mf ? blockIdx.y : blockIdx.x], bm = mf ? blockIdx.x : blockIdx.y;
     const int rN = g.pair_ring[2 * pair], rS = g.pair_ring[2 * pair + 1];
     const int n = BLU ? g.nphi[rN] : L;
     // Bluestein tables: chirp spectrum bt[0, L), chirp ch[t] = exp(-i pi t^2 / n) for t < n, then
     // the ring's phase block
     const float2 *bt = BLU ? g.pkb_bt + g.pkb_bt_ofs[pair] : nullptr, *ch = BLU ? bt + L : nullptr;
-    const PkTab T = pk_tables<LOGL>(pk_smem + C::BUF, g.pk_tw + g.pk_tw_ofs[LOGL], BLU ? bt + L + L / 2 : nullptr);
+    const PkTab T = pk_tables<LOGL>(pk_smem + C::BUF, tid, g.pk_tw + g.pk_tw_ofs[LOGL], BLU ? bt + L + L / 2 : nullptr);
     const int s = (flags & HB_F_NOPHASE) ? 0 : pk_shift(g.phi0_pi[rN], n);
     const int64_t np = g.npairs;
     const float *fN = maps + bm * map_stride + g.ofs[rN];
@@ -467,17 +472,17 @@ __global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
     auto ring = [&](int i, int = 0) -> float2 { return make_float2(__ldg(fN + i), fS ? __ldg(fS + i) : 0.f); };
     __syncthreads();  // tables
     if constexpr (!BLU) {
-        pk_run<LOGL, false, false, false>(buf, T, threadIdx.x, ring, sts);
+        pk_run<LOGL, false, false, false>(buf, T, tid, ring, sts);
     } else {
         // forward FFT_L of the chirped ring (zero from n on; read below L/2 only), times the chirp
         // spectrum; inverse FFT_L, points below L/2 only
         auto lds = [&](int, int ip) -> float2 { return buf[ip]; };
         auto ld0 = [&](int i, int) -> float2 { return i < n ? cmul(ring(i), __ldg(ch + i)) : make_float2(0.f, 0.f); };
-        pk_run<LOGL, false, true, false>(buf, T, threadIdx.x, ld0, sts);
+        pk_run<LOGL, false, true, false>(buf, T, tid, ld0, sts);
         __syncthreads();
-        for (int i = threadIdx.x; i < L; i += NT) buf[pk_pad(i)] = cmul(buf[pk_pad(i)], __ldg(bt + i));
+        for (int i = tid; i < L; i += NT) buf[pk_pad(i)] = cmul(buf[pk_pad(i)], __ldg(bt + i));
         __syncthreads();
-        pk_run<LOGL, true, false, true>(buf, T, threadIdx.x, lds, sts);
+        pk_run<LOGL, true, false, true>(buf, T, tid, lds, sts);
     }
     __syncthreads();
     auto Zf = [&](int k) -> float2 { return BLU ? cmul(__ldg(ch + k), buf[pk_pad(k)]) : buf[pk_pad(k)]; };
@@ -487,7 +492,76 @@ __global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
     const int mlim = (flags & HB_F_NOFOLD) ? min(mmax, n - 1) : mmax;
     float4 *out = Fm + bm * fm_stride4;
     auto at = [&](int m) -> float4 & { return out[fg_off(m, pair, np, mblk != 0)]; };
-    pk_emit<NT, !BLU>(n, s, mmax, mlim, mdouble != 0, scN, scS, T, Zf, at);
+    pk_emit<NT, !BLU>(tid, n, s, mmax, mlim, mdouble != 0, scN, scS, T, Zf, at);
+}
+
+template <int LOGL, bool BLU>
+__global__ void __launch_bounds__(PkCfg<LOGL>::NT, PkCfg<LOGL>::MINB)
+    ring_pair_analysis_kernel(GeomDev g, const int32_t *__restrict__ pairs, const float *__restrict__ maps,
+                              int64_t map_stride, const double *__restrict__ w, float4 *__restrict__ Fm,
+                              int64_t fm_stride4, int mmax, int flags, int unit_w, int mdouble, int mblk) {
+    extern __shared__ __align__(16) float2 pk_smem[];
+    const bool mf = BLU && mblk;
+    pair_analysis<LOGL, BLU>(g, pairs[mf ? blockIdx.y : blockIdx.x], mf ? blockIdx.x : blockIdx.y, threadIdx.x, pk_smem, maps,
+                             map_stride, w, Fm, fm_stride4, mmax, flags, unit_w, mdouble, mblk);
+}
+
+// ------------------------------------------------------------------------ merged classes
+// One launch for the classes up to L = 2^12, up to PM_WORK items (pk_merge).  A CTA has PM_NT threads, as
+// many pairs of one class side by side as their L/16 threads fit (its last CTA repeats the class's last
+// pair, with the same values), so a class whose own launch would be one short wave of 32- to 256-thread
+// CTAs, bound by the latency of its strided G reads and of its 3 to 4 passes, shares the GPU with the
+// others.  Longest classes first.  One FP32 map at nside 1024 (8 classes): synthesis 255 us in 8 launches
+// -> 108 us in one, analysis 149 -> 73 us; at nside 128 (3 classes) 30 -> 16 us each.
+constexpr int PM_NT = 256, PM_LOG = 12;
+struct PkMerged {
+    int n;
+    int key[2 * (PM_LOG - PK_MIN_LOG + 1)];  // log2 L | Bluestein << 8
+    int block[2 * (PM_LOG - PK_MIN_LOG + 1) + 1];  // first CTA of each class
+    int first[2 * (PM_LOG - PK_MIN_LOG + 1)], count[2 * (PM_LOG - PK_MIN_LOG + 1)];  // its pairs
+};
+template <int LOGL> constexpr int pm_smem_of() { return PM_NT / PkCfg<LOGL>::NT * PkCfg<LOGL>::SMEM; }
+constexpr int pm_max(int a, int b) { return a > b ? a : b; }
+constexpr int PM_SMEM = pm_max(pm_max(pm_smem_of<9>(), pm_smem_of<10>()), pm_max(pm_smem_of<11>(), pm_smem_of<12>()));
+
+// calls body(integral constants LOGL, BLU, thread, shared slice, pair) for this CTA's class
+template <class Body> __device__ __forceinline__ void pm_dispatch(const PkMerged &M, const int32_t *pairs, float2 *sm, Body body) {
+    int c = 0;
+    while (c + 1 < M.n && (int)blockIdx.x >= M.block[c + 1]) ++c;
+    const auto run = [&](auto logl, auto blu) {
+        constexpr int LOGL = decltype(logl)::value, NT = PkCfg<LOGL>::NT;
+        const int sub = threadIdx.x / NT;
+        const int i = min(((int)blockIdx.x - M.block[c]) * (PM_NT / NT) + sub, M.count[c] - 1);
+        body(logl, blu, (int)(threadIdx.x % NT), sm + sub * (PkCfg<LOGL>::SMEM / (int)sizeof(float2)), pairs[M.first[c] + i]);
+    };
+    switch (M.key[c]) {
+#define HB_PM_CASE(LG)                                                                                             \
+    case LG: run(std::integral_constant<int, LG>(), std::false_type()); break;                                     \
+    case LG | 256: run(std::integral_constant<int, LG>(), std::true_type()); break;
+        HB_PM_CASE(9) HB_PM_CASE(10) HB_PM_CASE(11) HB_PM_CASE(12)
+#undef HB_PM_CASE
+    }
+}
+
+__global__ void __launch_bounds__(PM_NT, 4)
+    ring_merged_synthesis_kernel(GeomDev g, PkMerged M, const float4 *__restrict__ Gm, int64_t gm_stride4, int mmax,
+                                 float *__restrict__ maps, int64_t map_stride, const double *__restrict__ w, int apply_w, int mdouble,
+                                 int flags) {
+    extern __shared__ __align__(16) float2 pk_smem[];
+    pm_dispatch(M, g.pk_pairs, pk_smem, [&](auto logl, auto blu, int tid, float2 *sm, int pair) {
+        pair_synthesis<decltype(logl)::value, decltype(blu)::value>(g, pair, blockIdx.y, tid, sm, Gm, gm_stride4, mmax, maps, map_stride,
+                                                                    w, apply_w, mdouble, flags);
+    });
+}
+
+__global__ void __launch_bounds__(PM_NT, 4)
+    ring_merged_analysis_kernel(GeomDev g, PkMerged M, const float *__restrict__ maps, int64_t map_stride, const double *__restrict__ w,
+                                float4 *__restrict__ Fm, int64_t fm_stride4, int mmax, int flags, int unit_w, int mdouble, int mblk) {
+    extern __shared__ __align__(16) float2 pk_smem[];
+    pm_dispatch(M, g.pk_pairs, pk_smem, [&](auto logl, auto blu, int tid, float2 *sm, int pair) {
+        pair_analysis<decltype(logl)::value, decltype(blu)::value>(g, pair, blockIdx.y, tid, sm, maps, map_stride, w, Fm, fm_stride4,
+                                                                   mmax, flags, unit_w, mdouble, mblk);
+    });
 }
 
 // ------------------------------------------------------------------------ quad-split Bluestein
@@ -622,7 +696,7 @@ __global__ void __launch_bounds__(QkCfg<LOGQ>::NT, QkCfg<LOGQ>::MINB)
     } else {
         tc::cp_async_wait<0>();
         __syncthreads();  // tables
-        pk_fold<NT, false>(n, s, mmax, dbl, T, ld, put);
+        pk_fold<NT, false>(threadIdx.x, n, s, mmax, dbl, T, ld, put);
     }
     __syncthreads();
     // radix-4 step: V^b_r c_r into sub-buffer b at r (zero for q <= r < LQ/2)
@@ -759,7 +833,7 @@ __global__ void __launch_bounds__(QkCfg<LOGQ>::NT, QkCfg<LOGQ>::MINB)
     const int mlim = (flags & HB_F_NOFOLD) ? min(mmax, n - 1) : mmax;
     float4 *out = Fm + bm * fm_stride4;
     auto at = [&](int m) -> float4 & { return out[fg_off(m, pair, np, mblk != 0)]; };
-    pk_emit<NT, false>(n, s, mmax, mlim, mdouble != 0, scN, scS, T, [&](int k) { return buf[qk_slot<LOGQ>(k, q)]; },
+    pk_emit<NT, false>(threadIdx.x, n, s, mmax, mlim, mdouble != 0, scN, scS, T, [&](int k) { return buf[qk_slot<LOGQ>(k, q)]; },
                        at);
 }
 
@@ -934,10 +1008,70 @@ static int pk_dispatch(const GeomDev &g, int logL, const int32_t *pp, int64_t cn
     }
 }
 
+// the classes that share a launch: those up to 2^PM_LOG
+static bool pk_mergeable(int key) { return (key & 0xff) <= PM_LOG && !((key >> 9) & 1); }
+// Whether they do: with up to PM_WORK (pair, map) items among them.  Both directions of all ring FFTs, one
+// launch per class against the shared one, in us: nside 128 x 1 98 -> 67, 512 x 5 482 -> 314, 1024 x 1
+// 573 -> 350, 1024 x 8 (12k items) 1665 -> 1505, 512 x 32 (30k) 1513 -> 1392, 1024 x 64 (94k) 10751 -> 10976:
+// from there on each class fills the GPU by itself, with its own register and shared-memory footprint.
+constexpr int64_t PM_WORK = 32768;
+static bool pk_merge(const GeomDev &g, int nmaps) {
+    int64_t items = 0;
+    int classes = 0;
+    for (int c = 0; c < g.pk_n_cls; ++c)
+        if (pk_mergeable(g.pk_logn[c])) {
+            items += (g.pk_first[c + 1] - g.pk_first[c]) * nmaps;
+            ++classes;
+        }
+    return classes > 1 && items <= PM_WORK && nmaps <= 65535;
+}
+int pk_launches(const GeomDev &g, int nmaps) {
+    int shared = 0;
+    for (int c = 0; c < g.pk_n_cls; ++c) shared += pk_mergeable(g.pk_logn[c]) ? 1 : 0;
+    return g.pk_n_cls - (pk_merge(g, nmaps) ? shared - 1 : 0);
+}
+
+static int pm_launch(const GeomDev &g, const PkMerged &M, const dim3 &grid, const PkSynArgs &a, cudaStream_t st) {
+    HB_CUDA_TRY(cudaFuncSetAttribute(ring_merged_synthesis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PM_SMEM));
+    ring_merged_synthesis_kernel<<<grid, PM_NT, PM_SMEM, st>>>(
+        g, M, reinterpret_cast<const float4 *>(a.Gm), (int64_t)(a.mmax + 1) * g.npairs, a.mmax, a.maps, a.map_stride, a.w,
+        a.apply_w ? 1 : 0, a.mdouble ? 1 : 0, a.flags);
+    HB_CHECK_LAUNCH();
+    return HB_OK;
+}
+static int pm_launch(const GeomDev &g, const PkMerged &M, const dim3 &grid, const PkAnaArgs &a, cudaStream_t st) {
+    HB_CUDA_TRY(cudaFuncSetAttribute(ring_merged_analysis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PM_SMEM));
+    ring_merged_analysis_kernel<<<grid, PM_NT, PM_SMEM, st>>>(
+        g, M, a.maps, a.map_stride, a.w, reinterpret_cast<float4 *>(a.Fm), fg_rows(a.mmax, a.mblk) * g.npairs, a.mmax, a.flags,
+        a.unit_w ? 1 : 0, a.mdouble ? 1 : 0, a.mblk ? 1 : 0);
+    HB_CHECK_LAUNCH();
+    return HB_OK;
+}
+
 template <class A> static int pk_all(const GeomDev &g, const A &a, cudaStream_t st) {
+    const bool merge = pk_merge(g, a.nmaps);
+    if (merge) {
+        PkMerged M{};
+        int blocks = 0;
+        for (int lg = PM_LOG; lg >= PK_MIN_LOG; --lg)
+            for (int c = 0; c < g.pk_n_cls; ++c) {
+                if (!pk_mergeable(g.pk_logn[c]) || (g.pk_logn[c] & 0xff) != lg) continue;
+                const int cnt = (int)(g.pk_first[c + 1] - g.pk_first[c]), per = PM_NT / ((1 << lg) / 16);
+                if (cnt <= 0) continue;
+                M.key[M.n] = g.pk_logn[c] & 0x1ff;
+                M.block[M.n] = blocks;
+                M.first[M.n] = (int)g.pk_first[c];
+                M.count[M.n] = cnt;
+                blocks += (cnt + per - 1) / per;
+                ++M.n;
+            }
+        M.block[M.n] = blocks;
+        if (blocks > 0)
+            if (int rc = pm_launch(g, M, dim3((unsigned)blocks, (unsigned)a.nmaps), a, st)) return rc;
+    }
     for (int c = 0; c < g.pk_n_cls; ++c) {
         const int64_t first = g.pk_first[c], cnt = g.pk_first[c + 1] - first;
-        if (cnt <= 0) continue;
+        if (cnt <= 0 || (merge && pk_mergeable(g.pk_logn[c]))) continue;
         const int lg = g.pk_logn[c] & 0xff;
         const bool blu = (g.pk_logn[c] >> 8) & 1, quad = (g.pk_logn[c] >> 9) & 1;
         int rc = quad  ? qk_dispatch(g, lg, g.pk_pairs + first, cnt, a, st)

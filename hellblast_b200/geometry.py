@@ -42,7 +42,7 @@ class Geometry:
             _registry[self.gid] = self
 
     def fft_launches(self, precision: int = 32) -> int:
-        """Ring-FFT kernel launches per direction (one per transform-length class)."""
+        """Ring-FFT kernel launches per direction for one map (short length classes share launches)."""
         n = ctypes.c_int(0)
         L.call("hb_geom_fft_launches", self.handle, int(precision), ctypes.byref(n))
         return n.value

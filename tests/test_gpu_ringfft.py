@@ -127,3 +127,29 @@ def test_unpaired_south_slot_garbage_is_ignored(hb, oracle):
         outs.append(out.cpu().numpy())
     assert np.all(np.isfinite(outs[1]))
     assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("nside,lmax,nmaps,phi0", [(128, 200, 176, "healpix"), (256, 37, 80, "reference"),
+                                                  (1024, 300, 24, "healpix")])
+def test_few_maps_match_large_batch(hb, nside, lmax, nmaps, phi0):
+    """The short pair-packed classes of a call on few maps run in one launch, those of a large batch in
+    one each (the line is at 32768 (pair, map) items): the same operations, so the same bits."""
+    from hellblast_b200 import _lib as L
+    from hellblast_b200 import geometry as G
+    g = G.healpix(nside, phi0=phi0)
+    p = G.plan(g, lmax, precision=64)
+    gen = torch.Generator(device="cuda").manual_seed(nside)
+    few = 3
+    nphi = np.asarray(g.nphi)[:g.npairs]
+    shared = int(np.sum((nphi > 256) & ((nphi <= 2048) | (nphi == 4096))))
+    assert shared * few <= 4800 and shared * nmaps > 32768
+    Gm = torch.view_as_complex(torch.randn(nmaps, lmax + 1, g.npairs, 2, 2, device="cuda", generator=gen))
+    st = torch.cuda.current_stream().cuda_stream
+    maps = {n: torch.full((n, g.npix), float("nan"), device="cuda") for n in (few, nmaps)}
+    for n, out in maps.items():
+        L.call("hb_ring_synthesis", p.handle, 32, n, Gm.data_ptr(), out.data_ptr(), 0, st)
+    assert torch.equal(maps[few], maps[nmaps][:few])
+    F = {n: torch.full((n, lmax + 1, g.npairs, 2), float("nan"), dtype=torch.complex64, device="cuda") for n in (few, nmaps)}
+    for n, out in F.items():
+        L.call("hb_ring_analysis", p.handle, 32, n, maps[nmaps].data_ptr(), None, out.data_ptr(), 0, st)
+    assert torch.equal(torch.view_as_real(F[few]), torch.view_as_real(F[nmaps][:few]))

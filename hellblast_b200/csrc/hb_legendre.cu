@@ -31,7 +31,7 @@
 //
 // What bounds the kernels: the FP64 pipe (62 FMA per clock and SM measured); the analysis adds a
 // warp reduction per l.  One map at nside 1024, lmax 2047: synthesis 2063 -> 1160 us, analysis
-// 2826 -> 1820 us (one-step form with a shared-memory reduction per l before).
+// 2826 -> 1706 us (one-step form with a shared-memory reduction per l before); two maps 1.8 times one.
 #include <cmath>
 
 #include "hb_internal.cuh"
@@ -195,100 +195,105 @@ __device__ __forceinline__ void anal_block(State<U> &S, const Weights<NB, U> &W,
     for (; k < nk; k += TL) anal_chunk<ZONE, false, U, NB, TL>(S, W, cf + k, red + k * NB * 4, lane);
 }
 
-// One CTA per (order, chunk of ring pairs, NB maps), every warp keeping one group of 32 U pairs in
-// registers over all l.  Per block of 256 l the warps' rows are summed by zone and combined to
+// One CTA per (order, chunk of ring pairs or all of them in turn, NB maps), every warp keeping one group of
+// 32 U pairs in registers over all l.  Per block of 256 l the warps' rows are summed by zone and combined to
 //     a_l = N_k eps_{l+1} c_k + N_{k-1} eps_l c_{k-1} + M_l e_k,   a_{l+1} = N_k o_k + M_{l+1} o'_k.
-template <int U, int NB, int TL, int NT>
-__global__ void __launch_bounds__(NT) leg_analysis64_kernel(GeomDev g, LegTab tb, int lmax, int mmax,
-                                                            const double2 *__restrict__ Fm, int64_t fm_stride,
-                                                            double2 *__restrict__ alm, int64_t alm_stride, int atomic,
-                                                            const int32_t *__restrict__ mlist) {
+template <int U, int NB, int TL, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) leg_analysis64_kernel(GeomDev g, LegTab tb, int lmax, int mmax,
+                                                                  const double2 *__restrict__ Fm, int64_t fm_stride,
+                                                                  double2 *__restrict__ alm, int64_t alm_stride, int nchunks,
+                                                                  const int32_t *__restrict__ mlist) {
     constexpr int NW = NT / 32, ROW = LKB * NB * 4;
     __shared__ double2 ca[LKB], cb[LKB];
     __shared__ double cprev[2 * NB];
     __shared__ int wzone[NW];
     extern __shared__ double red[];  // [NW][LKB][NB][4], then the sums [zone][LKB][NB][4]
     double *sum = red + NW * ROW;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = blockIdx.y * NW + warp;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // F row blockIdx.x holds order m (all orders, or the orders of mlist in list order)
     const int m = mlist ? mlist[blockIdx.x] : blockIdx.x;
     if (m < 0 || m > mmax) return;  // a listed order outside the plan: nothing read or written
     const int64_t np = g.npairs;
     const double2 *F = Fm + (int64_t)blockIdx.z * NB * fm_stride + (int64_t)blockIdx.x * np * 2;
-    const double *tab = tb.row(m, 0);
-    const bool any = (int64_t)grp * U * 32 < np;
-    State<U> S;
-    Weights<NB, U> W;
-    const int zone = start_group(g, tab, m, grp, lane, S);
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int64_t p = unit_pair<U>(grp, u, lane);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            W.er[b][u] = W.ei[b][u] = W.qr[b][u] = W.qi[b][u] = 0.0;
-            if (p < np) {
-                const double2 fn = F[b * fm_stride + 2 * p], fs = F[b * fm_stride + 2 * p + 1];
-                const double x = zone == ZPOLE ? g.pair_x[p] : 1.0;
-                W.er[b][u] = fn.x + fs.x;
-                W.ei[b][u] = fn.y + fs.y;
-                W.qr[b][u] = (fn.x - fs.x) * x;
-                W.qi[b][u] = (fn.y - fs.y) * x;
-            }
-        }
-    }
-    int mode = mode_of(S);
     double *mine = red + warp * ROW;
-    if (lane == 0) wzone[warp] = any ? zone : -1;
-    for (int l0 = m; l0 <= lmax; l0 += 2 * LKB, tab += LKB * LT_N) {
-        const int nk = min(LKB, (lmax - l0) / 2 + 1), nkp = (nk + TL - 1) / TL * TL;
-        for (int i = tid; i < LKB; i += NT) {
-            const double4 z = make_double4(0.0, 0.0, 0.0, 0.0);
-            const double4 a = i < nk ? four(tab + (int64_t)i * LT_N + LT_A) : z, b = i < nk ? four(tab + (int64_t)i * LT_N + LT_B0) : z;
-            ca[i] = make_double2(a.x, a.y);
-            cb[i] = make_double2(b.x, b.y);
-        }
-        for (int i = lane; i < ROW; i += 32) mine[i] = 0.0;
-        __syncthreads();
-        if (any) {
-            if (zone == ZPOLE)
-                anal_block<ZPOLE, U, NB, TL>(S, W, nkp, mode, ca, mine, lane);
-            else
-                anal_block<ZEQ, U, NB, TL>(S, W, nkp, mode, cb, mine, lane);
-        }
-        __syncthreads();
-        for (int i = tid; i < 2 * nk * NB * 4; i += NT) {
-            const int z = i >= nk * NB * 4, o = i - z * nk * NB * 4;
-            double s = 0.0;
-            for (int w = 0; w < NW; ++w)
-                if (wzone[w] == z) s += red[w * ROW + o];
-            sum[z * ROW + o] = s;
-        }
-        __syncthreads();
-        for (int i = tid; i < nk * NB; i += NT) {
-            const int k = i % nk, b = i / nk, l = l0 + 2 * k;
-            const double *A = sum + (k * NB + b) * 4, *B = A + ROW, *t = tab + (int64_t)k * LT_N;
-            double2 q = make_double2(0.0, 0.0);
-            if (l > m) {
-                const double *c = k > 0 ? A - NB * 4 : cprev + 2 * b;
-                q = make_double2(t[LT_Q - LT_N] * c[0], t[LT_Q - LT_N] * c[1]);
-            }
-            const double2 v0 = make_double2(t[LT_P] * A[0] + t[LT_M0] * B[0] + q.x, t[LT_P] * A[1] + t[LT_M0] * B[1] + q.y);
-            const double2 v1 = make_double2(t[LT_NX] * A[2] + t[LT_M1] * B[2], t[LT_NX] * A[3] + t[LT_M1] * B[3]);
-            double2 *dst = alm + ((int64_t)blockIdx.z * NB + b) * alm_stride + alm_idx(lmax, l, m);
-            if (atomic) {
-                atomicAdd(&dst[0].x, v0.x);
-                atomicAdd(&dst[0].y, v0.y);
-                if (l < lmax) {
-                    atomicAdd(&dst[1].x, v1.x);
-                    atomicAdd(&dst[1].y, v1.y);
+    const bool atomic = gridDim.y > 1;
+    for (int chunk = blockIdx.y; chunk < nchunks; chunk += gridDim.y) {
+        const int grp = chunk * NW + warp;
+        const double *tab = tb.row(m, 0);
+        const bool any = (int64_t)grp * U * 32 < np;
+        State<U> S;
+        Weights<NB, U> W;
+        const int zone = start_group(g, tab, m, grp, lane, S);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t p = unit_pair<U>(grp, u, lane);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                W.er[b][u] = W.ei[b][u] = W.qr[b][u] = W.qi[b][u] = 0.0;
+                if (p < np) {
+                    const double2 fn = F[b * fm_stride + 2 * p], fs = F[b * fm_stride + 2 * p + 1];
+                    const double x = zone == ZPOLE ? g.pair_x[p] : 1.0;
+                    W.er[b][u] = fn.x + fs.x;
+                    W.ei[b][u] = fn.y + fs.y;
+                    W.qr[b][u] = (fn.x - fs.x) * x;
+                    W.qi[b][u] = (fn.y - fs.y) * x;
                 }
-            } else {
-                dst[0] = v0;
-                if (l < lmax) dst[1] = v1;
             }
         }
+        int mode = mode_of(S);
+        if (lane == 0) wzone[warp] = any ? zone : -1;
+        for (int l0 = m; l0 <= lmax; l0 += 2 * LKB, tab += LKB * LT_N) {
+            const int nk = min(LKB, (lmax - l0) / 2 + 1), nkp = (nk + TL - 1) / TL * TL;
+            for (int i = tid; i < LKB; i += NT) {
+                const double4 z = make_double4(0.0, 0.0, 0.0, 0.0);
+                const double4 a = i < nk ? four(tab + (int64_t)i * LT_N + LT_A) : z, b = i < nk ? four(tab + (int64_t)i * LT_N + LT_B0) : z;
+                ca[i] = make_double2(a.x, a.y);
+                cb[i] = make_double2(b.x, b.y);
+            }
+            for (int i = lane; i < ROW; i += 32) mine[i] = 0.0;
+            __syncthreads();
+            if (any) {
+                if (zone == ZPOLE)
+                    anal_block<ZPOLE, U, NB, TL>(S, W, nkp, mode, ca, mine, lane);
+                else
+                    anal_block<ZEQ, U, NB, TL>(S, W, nkp, mode, cb, mine, lane);
+            }
+            __syncthreads();
+            for (int i = tid; i < 2 * nk * NB * 4; i += NT) {
+                const int z = i >= nk * NB * 4, o = i - z * nk * NB * 4;
+                double s = 0.0;
+                for (int w = 0; w < NW; ++w)
+                    if (wzone[w] == z) s += red[w * ROW + o];
+                sum[z * ROW + o] = s;
+            }
+            __syncthreads();
+            for (int i = tid; i < nk * NB; i += NT) {
+                const int k = i % nk, b = i / nk, l = l0 + 2 * k;
+                const double *A = sum + (k * NB + b) * 4, *B = A + ROW, *t = tab + (int64_t)k * LT_N;
+                double2 q = make_double2(0.0, 0.0);
+                if (l > m) {
+                    const double *c = k > 0 ? A - NB * 4 : cprev + 2 * b;
+                    q = make_double2(t[LT_Q - LT_N] * c[0], t[LT_Q - LT_N] * c[1]);
+                }
+                const double2 v0 = make_double2(t[LT_P] * A[0] + t[LT_M0] * B[0] + q.x, t[LT_P] * A[1] + t[LT_M0] * B[1] + q.y);
+                const double2 v1 = make_double2(t[LT_NX] * A[2] + t[LT_M1] * B[2], t[LT_NX] * A[3] + t[LT_M1] * B[3]);
+                double2 *dst = alm + ((int64_t)blockIdx.z * NB + b) * alm_stride + alm_idx(lmax, l, m);
+                if (atomic) {
+                    atomicAdd(&dst[0].x, v0.x);
+                    atomicAdd(&dst[0].y, v0.y);
+                    if (l < lmax) {
+                        atomicAdd(&dst[1].x, v1.x);
+                        atomicAdd(&dst[1].y, v1.y);
+                    }
+                } else {  // the chunks before this one were added by this thread
+                    dst[0] = chunk ? cadd(dst[0], v0) : v0;
+                    if (l < lmax) dst[1] = chunk ? cadd(dst[1], v1) : v1;
+                }
+            }
+            __syncthreads();
+            if (tid < 2 * NB) cprev[tid] = sum[((LKB - 1) * NB + tid / 2) * 4 + tid % 2];
+        }
         __syncthreads();
-        if (tid < 2 * NB) cprev[tid] = sum[((LKB - 1) * NB + tid / 2) * 4 + tid % 2];
     }
 }
 
@@ -429,15 +434,17 @@ struct LegArgs {
     int64_t a_stride() const { return alm_size(p->lmax, p->mmax); }
 };
 
-template <int U, int NB, int TL, int NT> static int run_analysis(const LegArgs &L, int nz, const double2 *F, double2 *alm) {
+template <int U, int NB, int TL, int NT, int MINB, bool IN_TURN>
+static int run_analysis(const LegArgs &L, int nz, const double2 *F, double2 *alm) {
     const int64_t per = (int64_t)U * NT;
-    const int nchunks = (int)((L.np() + per - 1) / per);
-    if (nchunks > 1) HB_CUDA_TRY(cudaMemsetAsync(alm, 0, sizeof(double2) * L.a_stride() * NB * nz, L.st));
+    const int nchunks = (int)((L.np() + per - 1) / per), ny = IN_TURN ? 1 : nchunks;
+    if (ny > 1) HB_CUDA_TRY(cudaMemsetAsync(alm, 0, sizeof(double2) * L.a_stride() * NB * nz, L.st));
     const int smem = (NT / 32 + 2) * LKB * NB * 4 * (int)sizeof(double);
-    HB_CUDA_TRY(cudaFuncSetAttribute(leg_analysis64_kernel<U, NB, TL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    dim3 grid((unsigned)L.rows, (unsigned)nchunks, (unsigned)nz);
-    leg_analysis64_kernel<U, NB, TL, NT><<<grid, NT, smem, L.st>>>(L.p->g->d, L.p->leg, L.p->lmax, L.p->mmax, F, L.f_stride(),
-                                                                   alm, L.a_stride(), nchunks > 1, L.mlist);
+    const auto kernel = leg_analysis64_kernel<U, NB, TL, NT, MINB>;
+    HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    dim3 grid((unsigned)L.rows, (unsigned)ny, (unsigned)nz);
+    kernel<<<grid, NT, smem, L.st>>>(L.p->g->d, L.p->leg, L.p->lmax, L.p->mmax, F, L.f_stride(), alm, L.a_stride(), nchunks,
+                                     L.mlist);
     HB_CHECK_LAUNCH();
     return HB_OK;
 }
@@ -452,10 +459,22 @@ template <int U, int NB, int MINB> static int run_synthesis(const LegArgs &L, in
 // Pairs per lane and warps per CTA: large grids amortise the warp reduction (analysis) and the
 // coefficient loads (synthesis) over U = 4 pairs per lane; grids below 1024 pairs spread their few
 // pairs over more warps, since they do not fill the GPU.
+// Analysis of large grids: every block of 256 l ends in a barrier of the CTA, where warps whose pairs are
+// still evanescent wait for the others.  With IN_TURN a CTA has 4 warps and takes the chunks of an order
+// one after the other (a fixed sum, no atomics), and the 3 or 4 CTAs of an SM fill each other's waits.  That
+// takes enough orders (in_turn) and each of them once, which a list of orders does not promise; else one
+// map's pairs run side by side, 16 warps a CTA.  In us, wide / in turn: nside 1024, one map, lmax 2047
+// 1836 / 1706, 1100 562 / 540, 900 378 / 401.  Two maps in pairs, 8 warps wide / in turn: lmax 2047 4295 / 3077,
+// 700 562 / 439, 500 291 / 280.
+static bool in_turn(const LegArgs &L, int nb, int64_t nz) {
+    return L.np() >= 1024 && !L.mlist && L.rows * nz >= (nb == 1 ? 1024 : 512);
+}
 template <int NB> static int analysis_nb(const LegArgs &L, int nz, const double2 *F, double2 *alm) {
-    if (L.np() >= 1024) return run_analysis<4, NB, NB == 1 ? 4 : 2, NB == 1 ? 512 : 256>(L, nz, F, alm);
-    if (L.np() >= 256) return run_analysis<2, NB, NB == 1 ? 4 : 2, 256>(L, nz, F, alm);
-    return run_analysis<1, NB, NB == 1 ? 4 : 2, 128>(L, nz, F, alm);
+    constexpr int TL = NB == 1 ? 4 : 2;
+    if ((NB == 2 && L.np() >= 1024) || in_turn(L, NB, nz)) return run_analysis<4, NB, TL, 128, NB == 1 ? 4 : 3, true>(L, nz, F, alm);
+    if (NB == 1 && L.np() >= 1024) return run_analysis<4, 1, 4, 512, 0, false>(L, nz, F, alm);
+    if (L.np() >= 256) return run_analysis<2, NB, TL, 256, 0, false>(L, nz, F, alm);
+    return run_analysis<1, NB, TL, 128, 0, false>(L, nz, F, alm);
 }
 template <int NB> static int synthesis_nb(const LegArgs &L, int nz, const double2 *alm, double2 *G) {
     if (L.np() >= 1024) return run_synthesis<NB == 1 ? 4 : 2, NB, NB == 1 ? 16 : 14>(L, nz, alm, G);
@@ -463,10 +482,10 @@ template <int NB> static int synthesis_nb(const LegArgs &L, int nz, const double
 }
 
 // Maps in pairs that share one recursion: 11 operations per (two l, ring pair) for two maps, 7 for one.
-// Below 256 pairs one launch of single maps: these are bound by latency (3 maps at nside 64, lmax 100:
+// Below 256 ring pairs one launch of single maps: these are bound by latency (3 maps at nside 64, lmax 100:
 // 6 us, 9 us as a pair and a single).
-template <typename Fn2, typename Fn1> static int by_two(int nmaps, int64_t np, Fn2 f2, Fn1 f1) {
-    const int n2 = np >= 256 ? nmaps / 2 : 0;
+template <typename Fn2, typename Fn1> static int by_two(int nmaps, bool pairs, Fn2 f2, Fn1 f1) {
+    const int n2 = pairs ? nmaps / 2 : 0;
     if (n2)
         if (int rc = f2(n2, 0)) return rc;
     return nmaps > 2 * n2 ? f1(nmaps - 2 * n2, 2 * n2) : HB_OK;
@@ -476,7 +495,8 @@ int launch_leg_analysis64(const hb_plan *p, int nmaps, const double2 *F, double2
                           const int32_t *mlist) {
     const LegArgs L{p, mlist ? nm : p->mmax + 1, mlist, st};
     const int64_t fs = L.f_stride(), as = L.a_stride();
-    return by_two(nmaps, L.np(), [&](int nz, int b) { return analysis_nb<2>(L, nz, F + b * fs, alm + b * as); },
+    const bool pairs = L.np() >= 1024 ? in_turn(L, 2, nmaps / 2) : L.np() >= 256;
+    return by_two(nmaps, pairs, [&](int nz, int b) { return analysis_nb<2>(L, nz, F + b * fs, alm + b * as); },
                   [&](int nz, int b) { return analysis_nb<1>(L, nz, F + b * fs, alm + b * as); });
 }
 
@@ -484,7 +504,7 @@ int launch_leg_synthesis64(const hb_plan *p, int nmaps, const double2 *alm, doub
                            const int32_t *mlist) {
     const LegArgs L{p, mlist ? nm : p->mmax + 1, mlist, st};
     const int64_t fs = L.f_stride(), as = L.a_stride();
-    return by_two(nmaps, L.np(), [&](int nz, int b) { return synthesis_nb<2>(L, nz, alm + b * as, G + b * fs); },
+    return by_two(nmaps, L.np() >= 256, [&](int nz, int b) { return synthesis_nb<2>(L, nz, alm + b * as, G + b * fs); },
                   [&](int nz, int b) { return synthesis_nb<1>(L, nz, alm + b * as, G + b * fs); });
 }
 

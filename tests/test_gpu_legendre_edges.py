@@ -77,3 +77,33 @@ def test_spin_sizes(hb, oracle, nside, lmax, mmax, nmaps):
         for i in range(2):
             assert rel2(got[i].double().cpu().numpy(), np.stack([r[i] for r in ref_map])) < tol, (prec, "map")
             assert rel2(back[i].to(torch.complex128).cpu().numpy(), np.stack([r[i] for r in ref_alm])) < tol, (prec, "alm")
+
+
+@pytest.mark.parametrize("nrings,lmax,nmaps", [(2047, 1023, 1), (2051, 1025, 3), (2048, 511, 2), (4097, 1100, 1)])
+def test_orders_in_turn_match_a_list(hb, nrings, lmax, nmaps):
+    """FP64 analysis on 1024 and more ring pairs: with many orders a CTA takes an order's chunks of pairs in
+    turn (and maps in pairs), a list of orders has each order's pairs side by side.  The same products
+    summed in another order, at most 2049 per value: 1e-12 relative (L2) is 2049 eps with room."""
+    from hellblast_b200 import _lib as L
+    from hellblast_b200 import geometry as G
+    th = np.linspace(0.0007, np.pi / 2, (nrings + 1) // 2 + (nrings % 2 == 0))[:(nrings + 1) // 2]
+    th = np.concatenate([th, np.pi - th[:nrings // 2][::-1]])
+    g = G.generic(th, np.full(nrings, 4, dtype=np.int32), np.full(nrings, 2.0 / nrings))
+    assert g.npairs == (nrings + 1) // 2 >= 1024
+    p = G.plan(g, lmax, precision=64)
+    gen = torch.Generator(device="cuda").manual_seed(nrings)
+    F = torch.view_as_complex(torch.randn(nmaps, lmax + 1, g.npairs, 2, 2, device="cuda", generator=gen, dtype=torch.float64))
+    nalm = L.lib().hb_alm_size(lmax, lmax)
+    st = torch.cuda.current_stream().cuda_stream
+    full = torch.full((nmaps, nalm), float("nan"), dtype=torch.complex128, device="cuda")
+    L.call("hb_legendre_analysis", p.handle, 64, nmaps, F.data_ptr(), full.data_ptr(), st)
+    orders = [0, 1, 2, lmax // 2, lmax - 1, lmax]
+    lst = torch.tensor(orders, dtype=torch.int32, device="cuda")
+    some = torch.zeros_like(full)
+    L.call("hb_legendre_analysis_ms", p.handle, 64, nmaps, len(orders), lst.data_ptr(), F[:, orders].contiguous().data_ptr(),
+           some.data_ptr(), st)
+    assert torch.isfinite(torch.view_as_real(full)).all()
+    for m in orders:
+        i = m * (2 * lmax + 1 - m) // 2
+        a, b = full[:, i + m:i + lmax + 1].cpu().numpy(), some[:, i + m:i + lmax + 1].cpu().numpy()
+        assert rel2(a, b) < 1e-12, m

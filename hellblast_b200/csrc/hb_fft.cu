@@ -368,8 +368,8 @@ template <> __device__ __forceinline__ void store_ns<double2>(double2 *dst, doub
     dst[1] = s;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
+template <typename T, int MINB>
+__global__ void __launch_bounds__(256, MINB)
     ring_analysis_kernel(GeomDev g, const int32_t *__restrict__ pairs, const T *__restrict__ maps, int64_t map_stride,
                          const double *__restrict__ w, c2_t<T> *__restrict__ Fm, int64_t fm_stride, int mmax,
                          int flags, int unit_w, int mdouble, int Lcls, int stage_n, int mblk) {
@@ -464,8 +464,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
 }
 
 // ------------------------------------------------------------------------------ synthesis
-template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1)
+template <typename T, int MINB>
+__global__ void __launch_bounds__(256, MINB)
     ring_synthesis_kernel(GeomDev g, const int32_t *__restrict__ pairs, const c2_t<T> *__restrict__ Gm,
                           int64_t gm_stride, int mmax, T *__restrict__ maps, int64_t map_stride,
                           const double *__restrict__ w, int apply_w, int mdouble, int flags, int Lcls, int stage_t) {
@@ -773,6 +773,31 @@ int merged_classes(int ncls, const int *L, const int64_t *first) {
     return n;
 }
 
+// CTAs of 256 threads per SM that the kernels' registers leave room for: FP32 3; FP64 1 (230 registers) for
+// calls whose launches hold no more threads than one such CTA per SM, bound by the latency of one CTA, else 2
+// (128 registers, 16 bytes spilled).  All launches of a call take the same one: changing the kernel between
+// them costs 6 us of instruction fetches.  FP64, 1 / 2 in us, synthesis + analysis: nside 1024 508 + 388 /
+// 372 + 308, 3 maps 1313 + 989 / 991 + 783; 512 109 + 100 / 86 + 79; 64 17 + 16 / 18 + 17.5.
+template <typename T> static int min_ctas(int ncls, int nmerge, const int *L, const int64_t *first, int nmaps) {
+    if (sizeof(T) == 4) return 3;
+    int64_t threads = 0;
+    for (int c = nmerge ? nmerge - 1 : 0; c < ncls; ++c)
+        threads = std::max(threads, (first[c + 1] - (c < nmerge ? 0 : first[c])) * nmaps * class_threads(L[c]));
+    return threads <= 256 * (int64_t)sm_count() ? 1 : 2;
+}
+template <typename T> static auto analysis_kernel(int minb) {
+    if constexpr (sizeof(T) == 4)
+        return ring_analysis_kernel<T, 3>;
+    else
+        return minb == 1 ? ring_analysis_kernel<T, 1> : ring_analysis_kernel<T, 2>;
+}
+template <typename T> static auto synthesis_kernel(int minb) {
+    if constexpr (sizeof(T) == 4)
+        return ring_synthesis_kernel<T, 3>;
+    else
+        return minb == 1 ? ring_synthesis_kernel<T, 1> : ring_synthesis_kernel<T, 2>;
+}
+
 template <typename T>
 static int check_smem(const GeomDev &g, int mmax) {
     for (int c = 0; c < g.n_cls; ++c) {
@@ -804,6 +829,7 @@ static int launch_analysis_t(const GeomDev &g, int nmaps, const T *maps, int64_t
     const int64_t *clsF = f32 ? g.rest_first : g.cls_first;
     const int32_t *clsP = f32 ? g.rest_pairs : g.cls_pairs;
     const int nmerge = merged_classes(ncls, clsL, clsF);
+    const auto kernel = analysis_kernel<T>(min_ctas<T>(ncls, nmerge, clsL, clsF, nmaps));
     for (int c = nmerge ? nmerge - 1 : 0; c < ncls; ++c) {
         const int L = clsL[c];
         const int64_t first = c < nmerge ? 0 : clsF[c], cnt = clsF[c + 1] - first;
@@ -812,14 +838,12 @@ static int launch_analysis_t(const GeomDev &g, int nmaps, const T *maps, int64_t
         const int ctas0 = ctas_by_smem(base_smem), ctas1 = ctas_by_smem(base_smem + stage_bytes);
         const bool stage_n = base_smem + stage_bytes <= (size_t)max_smem_optin() && ctas1 >= std::min(2, ctas0);
         const int smem = (int)(base_smem + (stage_n ? stage_bytes : 0));
-        HB_CUDA_TRY(cudaFuncSetAttribute(ring_analysis_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        HB_CUDA_TRY(cudaFuncSetAttribute(ring_analysis_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared));
         dim3 grid((unsigned)cnt, (unsigned)nmaps);
-        ring_analysis_kernel<T><<<grid, class_threads(L), smem, st>>>(g, clsP + first, maps, map_stride,
-                                                                       w ? w : g.w, Fm, fm_stride, mmax, flags,
-                                                                       unit_w ? 1 : 0, mdouble ? 1 : 0, L,
-                                                                       stage_n ? 1 : 0, mblk ? 1 : 0);
+        kernel<<<grid, class_threads(L), smem, st>>>(g, clsP + first, maps, map_stride, w ? w : g.w, Fm, fm_stride, mmax, flags,
+                                                     unit_w ? 1 : 0, mdouble ? 1 : 0, L, stage_n ? 1 : 0, mblk ? 1 : 0);
         HB_CHECK_LAUNCH();
     }
     return HB_OK;
@@ -844,22 +868,22 @@ static int launch_synthesis_t(const GeomDev &g, int nmaps, const c2_t<T> *Gm, in
     const int64_t *clsF = f32 ? g.rest_first : g.cls_first;
     const int32_t *clsP = f32 ? g.rest_pairs : g.cls_pairs;
     const int nmerge = merged_classes(ncls, clsL, clsF);
+    const auto kernel = synthesis_kernel<T>(min_ctas<T>(ncls, nmerge, clsL, clsF, nmaps));
     for (int c = nmerge ? nmerge - 1 : 0; c < ncls; ++c) {
         const int L = clsL[c];
         const int64_t first = c < nmerge ? 0 : clsF[c], cnt = clsF[c + 1] - first;
         const bool stage_t = class_smem_syn<T>(L, mmax, true) <= (size_t)max_smem_optin();
         const int smem = (int)class_smem_syn<T>(L, mmax, stage_t), nt = class_threads(L);
-        HB_CUDA_TRY(cudaFuncSetAttribute(ring_synthesis_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        HB_CUDA_TRY(cudaFuncSetAttribute(ring_synthesis_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared));
         // asynchronous staging when the grid is under two waves of resident CTAs
         int occ = 1;
-        HB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ring_synthesis_kernel<T>, nt, smem));
+        HB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, nt, smem));
         const bool async_t = stage_t && cnt * (int64_t)nmaps < 2 * (int64_t)sm_count() * std::max(occ, 1);
         dim3 grid((unsigned)cnt, (unsigned)nmaps);
-        ring_synthesis_kernel<T><<<grid, nt, smem, st>>>(g, clsP + first, Gm, gm_stride, mmax, maps, map_stride,
-                                                         w ? w : g.w, apply_w ? 1 : 0, mdouble ? 1 : 0, flags, L,
-                                                         stage_t ? (async_t ? 2 : 1) : 0);
+        kernel<<<grid, nt, smem, st>>>(g, clsP + first, Gm, gm_stride, mmax, maps, map_stride, w ? w : g.w, apply_w ? 1 : 0,
+                                       mdouble ? 1 : 0, flags, L, stage_t ? (async_t ? 2 : 1) : 0);
         HB_CHECK_LAUNCH();
     }
     return HB_OK;

@@ -153,3 +153,26 @@ def test_few_maps_match_large_batch(hb, nside, lmax, nmaps, phi0):
     for n, out in F.items():
         L.call("hb_ring_analysis", p.handle, 32, n, maps[nmaps].data_ptr(), None, out.data_ptr(), 0, st)
     assert torch.equal(torch.view_as_real(F[few]), torch.view_as_real(F[nmaps][:few]))
+
+
+@pytest.mark.parametrize("nside,lmax", [(32, 100), (256, 300), (512, 40)])
+def test_fp64_one_map_matches_many(hb, nside, lmax):
+    """FP64 ring FFTs of small and of large calls are separate builds of the kernels, with more and with fewer
+    registers per thread: the same formulas, so 1e-13 relative (L2) between them (FFT rounding is below 1e-14)."""
+    from hellblast_b200 import _lib as L
+    from hellblast_b200 import geometry as G
+    g = G.healpix(nside)
+    p = G.plan(g, lmax, precision=64)
+    many = max(2, 80000 // (64 * g.npairs) + 1)
+    gen = torch.Generator(device="cuda").manual_seed(nside)
+    Gm = torch.view_as_complex(torch.randn(many, lmax + 1, g.npairs, 2, 2, device="cuda", generator=gen, dtype=torch.float64))
+    st = torch.cuda.current_stream().cuda_stream
+    maps, F = {}, {}
+    for n in (1, many):
+        maps[n] = torch.full((n, g.npix), float("nan"), device="cuda", dtype=torch.float64)
+        L.call("hb_ring_synthesis", p.handle, 64, n, Gm.data_ptr(), maps[n].data_ptr(), 0, st)
+    for n in (1, many):
+        F[n] = torch.full((n, lmax + 1, g.npairs, 2), float("nan"), dtype=torch.complex128, device="cuda")
+        L.call("hb_ring_analysis", p.handle, 64, n, maps[many].data_ptr(), None, F[n].data_ptr(), 0, st)
+    assert rel2(maps[1][0].cpu().numpy(), maps[many][0].cpu().numpy()) < 1e-13
+    assert rel2(F[1][0].cpu().numpy(), F[many][0].cpu().numpy()) < 1e-13

@@ -126,47 +126,65 @@ static int alm2map_spin_impl(const hb_plan *p, int nmaps, const void *E, const v
                                  st);
 }
 
-// alm2cl (alm_ops.py:19-32): a CTA owns 32 consecutive l of one map (the lanes) and its 8 warps
-// split the m range (m = warp mod 8), so every warp load reads 32 consecutive l of one healpy
+// alm2cl (alm_ops.py:19-32): a CTA owns 32 consecutive l of one map (the lanes) and its 32 warps
+// (fewer for small spectra) split the m range, so every warp load reads 32 consecutive l of one healpy
 // m-column (256 B); FP64 accumulation, one shared-memory reduction over the warps, no atomics.
-template <typename V>
-__global__ void __launch_bounds__(256) alm2cl_kernel(int lmax, int mmax, const V *__restrict__ a1,
-                                                     const V *__restrict__ a2, int64_t stride, double *__restrict__ cl) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// HBM-bound for a batch; a single alm has only lmax / 32 CTAs and is bound by the latency of a warp's chain
+// of loads, so a CTA has all the warps it may and a warp 8 loads in flight.  Against 8 warps with 4 m each
+// in flight and every alm loaded twice, complex64, us: lmax 2047 26.9 -> 13.5, 16 of them 86 -> 70, 64 of
+// lmax 4095 887 -> 748; two alm, lmax 2047 27.9 -> 18.2.
+// AUTO: the spectrum of one alm with itself.
+constexpr int CL_WARPS = 32;
+template <typename V, bool AUTO>
+__global__ void __launch_bounds__(32 * CL_WARPS) alm2cl_kernel(int lmax, int mmax, const V *__restrict__ a1,
+                                                              const V *__restrict__ a2, int64_t stride, double *__restrict__ cl) {
+    constexpr int D = AUTO ? 8 : 4;  // m per round: 8 loads
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int l = blockIdx.x * 32 + lane, b = blockIdx.y;
-    const V *p1 = a1 + b * stride, *p2 = (a2 ? a2 : a1) + b * stride;
-    const int mtop = l < mmax ? l : mmax;
-    auto term = [&](int m) -> double {
-        const int64_t k = alm_idx(lmax, l, m);
-        const V u = p1[k], v = p2[k];
-        return (m == 0 ? 1.0 : 2.0) * ((double)u.x * (double)v.x + (double)u.y * (double)v.y);
-    };
+    const V *p1 = a1 + b * stride, *p2 = a2 + b * stride;
+    const int mtop = l > lmax ? -1 : (l < mmax ? l : mmax);
     double acc = 0.0;
-    if (l <= lmax) {
-        int m = warp;
-        for (; m + 24 <= mtop; m += 32) {  // four independent loads in flight per thread
-            const double t0 = term(m), t1 = term(m + 8), t2 = term(m + 16), t3 = term(m + 24);
-            acc += (t0 + t1) + (t2 + t3);
+    for (int m0 = warp; m0 <= mtop; m0 += D * nw) {
+        V u[D], v[AUTO ? 1 : D];
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            const int m = m0 + i * nw;
+            const int64_t k = alm_idx(lmax, l, m <= mtop ? m : m0);
+            u[i] = p1[k];
+            if (!AUTO) v[i] = p2[k];
         }
-        for (; m <= mtop; m += 8) acc += term(m);
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            const int m = m0 + i * nw;
+            const V w = AUTO ? u[i] : v[AUTO ? 0 : i];
+            if (m <= mtop) acc += (m == 0 ? 1.0 : 2.0) * ((double)u[i].x * (double)w.x + (double)u[i].y * (double)w.y);
+        }
     }
-    __shared__ double red[8][33];
+    __shared__ double red[CL_WARPS][33];
     red[warp][lane] = acc;
     __syncthreads();
     if (warp == 0 && l <= lmax) {
         double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) s += red[w][lane];
+#pragma unroll 8
+        for (int w = 0; w < nw; ++w) s += red[w][lane];
         cl[(int64_t)b * (lmax + 1) + l] = s / (2.0 * l + 1.0);
     }
 }
 
+// Warps that find work, at mmax 20 / 64 / 128 / 256 / 2047 in us: 8 warps 2.0 / 2.4 / 3.0 / 4.4 / 23.9, 16 warps 2.2 /
+// 2.1 / 2.7 / 3.6 / 16.1, 32 warps 2.5 / 2.8 / 3.3 / 3.5 / 13.5; where CTAs queue (64 alm of lmax 4095) 16 warps
+// 748, 32 warps 844.
+static int cl_warps(int mmax, int64_t ctas) { return mmax < 40 ? 8 : (mmax < 256 || ctas >= 4096 ? 16 : CL_WARPS); }
 template <typename V>
 static int alm2cl_impl(int lmax, int mmax, int nmaps, const V *a1, const V *a2, double *cl, cudaStream_t st) {
     if (lmax < 0 || mmax < 0 || mmax > lmax || nmaps <= 0 || nmaps > 65535 || !a1 || !cl)
         return fail(HB_ERR_INVALID, "hb_alm2cl: bad arguments");
     dim3 grid((unsigned)((lmax + 32) / 32), (unsigned)nmaps);
-    alm2cl_kernel<V><<<grid, 256, 0, st>>>(lmax, mmax, a1, a2, alm_size(lmax, mmax), cl);
+    const int nw = cl_warps(mmax, (int64_t)grid.x * nmaps);
+    if (!a2 || a2 == a1)
+        alm2cl_kernel<V, true><<<grid, 32 * nw, 0, st>>>(lmax, mmax, a1, a1, alm_size(lmax, mmax), cl);
+    else
+        alm2cl_kernel<V, false><<<grid, 32 * nw, 0, st>>>(lmax, mmax, a1, a2, alm_size(lmax, mmax), cl);
     HB_CHECK_LAUNCH();
     return HB_OK;
 }

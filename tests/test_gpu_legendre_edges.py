@@ -107,3 +107,29 @@ def test_orders_in_turn_match_a_list(hb, nrings, lmax, nmaps):
         i = m * (2 * lmax + 1 - m) // 2
         a, b = full[:, i + m:i + lmax + 1].cpu().numpy(), some[:, i + m:i + lmax + 1].cpu().numpy()
         assert rel2(a, b) < 1e-12, m
+
+
+@pytest.mark.parametrize("lmax,mmax,nmaps", [(0, 0, 1), (31, 31, 2), (33, 39, 1), (64, 40, 3), (255, 255, 1), (256, 256, 1), (300, 5, 2),
+                                             (517, 300, 1), (256, 256, 456)])
+@pytest.mark.parametrize("cross", [False, True])
+def test_alm2cl_sizes(hb, lmax, mmax, nmaps, cross):
+    """alm2cl around the sizes where its CTAs change their number of warps, with order cut-offs; against NumPy in
+    64 bits: at most 2 * 517 products per value, 1e-13 of the largest |a||b| / (2l+1)."""
+    from hellblast_b200 import ops
+    mmax = min(mmax, lmax)
+    nalm = (mmax + 1) * (2 * lmax + 2 - mmax) // 2
+    for dt in (torch.complex64, torch.complex128):
+        gen = torch.Generator(device="cuda").manual_seed(lmax)
+        a = torch.randn(nmaps, nalm, dtype=dt, device="cuda", generator=gen)
+        b = torch.randn(nmaps, nalm, dtype=dt, device="cuda", generator=gen) if cross else None
+        A = a.to(torch.complex128).cpu().numpy()
+        B = A if b is None else b.to(torch.complex128).cpu().numpy()
+        want, size = np.zeros((2, nmaps, lmax + 1))
+        for m in range(mmax + 1):
+            i = m * (2 * lmax + 1 - m) // 2
+            p, q = A[:, i + m:i + lmax + 1], B[:, i + m:i + lmax + 1]
+            want[:, m:] += (1 if m == 0 else 2) * (p * q.conj()).real
+            size[:, m:] += 2 * np.abs(p) * np.abs(q)
+        deg = 2 * np.arange(lmax + 1) + 1.0
+        got = ops.alm2cl(a, b, lmax, mmax).cpu().numpy()
+        assert np.all(np.abs(got - want / deg) <= 1e-13 * size / deg)

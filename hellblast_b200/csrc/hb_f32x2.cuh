@@ -37,4 +37,9 @@ __device__ __forceinline__ unsigned bits_or(unsigned acc, f32x2 v) { return acc 
 __device__ __forceinline__ bool maybe_big(unsigned acc) { return (acc & 0x7f800000u) >= 0x4f800000u; }
 constexpr float F32_UP = 4294967296.0f;                 // 2^32: a state past this moves to the next exponent
 constexpr float F32_DOWN = 5.42101086242752217e-20f;    // 2^-64: one exponent step
+// factor that takes sums in units of 2^(64 e0) to units of 2^(64 e1).  Exponents rise from block to block, but for a
+// first block's e1 < 0 against the 0 of empty sums: one step up is then as good as any, and stays finite.
+__device__ __forceinline__ float sums_to_unit(int e0, int e1) {
+    return e0 == e1 ? 1.f : ldexpf(1.f, 64 * max(-3, min(1, e0 - e1)));
+}
 }  // namespace hb

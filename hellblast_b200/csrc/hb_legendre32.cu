@@ -56,12 +56,8 @@ __device__ __forceinline__ void block_state(const GeomDev &g, int m, int j, int6
     }
 }
 
-// whether a pair that starts a block with e < 0 keeps e < 0 through it, by the next block's checkpoint row:
-// both of its values below 2^-32 (one alone can be near zero on an oscillating pair)
-__device__ __forceinline__ bool stays_dead(const float4 *next, int64_t p) {
-    const float4 c = next[p];
-    return __float_as_int(c.z) < 0 && fabsf(c.y) < F32_UP;
-}
+// whether a pair that starts a block with e < 0 keeps e < 0 through it, by the next block's checkpoint row
+__device__ __forceinline__ bool stays_dead(const float4 *next, int64_t p) { return __float_as_int(next[p].z) < 0; }
 
 struct alignas(16) Coef2 {  // (A_l, B_l), each in both halves
     f32x2 a, b;
@@ -381,8 +377,7 @@ __global__ void __launch_bounds__(32, MINB) leg_synthesis32_kernel(GeomDev g, in
             for (int i = 0; i < 2; ++i) {
                 int e;
                 block_state(g, m, j, (int64_t)(grp * U + u) * 64 + 2 * lane + i, ck + blk * np, l1[i], l2[i], e);
-                // e never falls from block to block, except from the 0 of empty sums
-                f[i] = e > S.e[u][i] ? ldexpf(1.0f, 64 * max(-3, S.e[u][i] - e)) : 1.f;
+                f[i] = sums_to_unit(S.e[u][i], e);
                 S.e[u][i] = e;
                 neg |= e < 0;
             }

@@ -32,9 +32,11 @@ __device__ __forceinline__ void ck_scalar_coef(int l, int m, double &A, double &
     B = (l - 1 > m) ? -A * sqrt(((ll - 1.0 - mm) * (ll - 1.0 + mm)) / (4.0 * (ll - 1.0) * (ll - 1.0) - 1.0)) : 0.0;
 }
 
-// Convert an FP64 scaled state (v1, v2) * 2^(512 e) to the FP32 format (mu1, mu2) * 2^(64 ef).
+// Convert an FP64 scaled state (v1, v2) * 2^(512 e) to the FP32 format (mu1, mu2) * 2^(64 ef).  The exponent
+// is that of the larger value: one alone can be near zero on an oscillating pair (every second value on a
+// ring at the equator), and such a pair is live.
 __device__ __forceinline__ float4 to_f32_state(double v1, double v2, int e) {
-    double ref = (v1 != 0.0) ? v1 : v2;
+    const double ref = fmax(fabs(v1), fabs(v2));
     if (ref == 0.0) return make_float4(0.f, 0.f, __int_as_float(0), 0.f);
     int ex;
     frexp(ref, &ex);  // |ref| in [2^(ex-1), 2^ex)
@@ -159,8 +161,7 @@ __global__ void __launch_bounds__(CK_NT) ck_scalar_kernel(GeomDev g, int lmax, c
             }
         }
         if (flags) {
-            // by the larger of the last two values: one alone can be near zero on an oscillating pair
-            if (live && __float_as_int(to_f32_state(fmax(fabs(l1), fabs(l2)), 0.0, e).z) >= 0) any_live[threadIdx.x / 64] = 1;
+            if (live && __float_as_int(to_f32_state(l1, l2, e).z) >= 0) any_live[threadIdx.x / 64] = 1;
             __syncthreads();
             write_flags(flags, blk_ofs[m] + (l0 - m) / CKR, np, any_neg, any_live);
         }
@@ -239,8 +240,7 @@ __global__ void __launch_bounds__(CK_NT) ck_spin_kernel(GeomDev g, int lmax, con
             if (ep < 0 && fabs(P1) > 0x1p256) { P1 *= 0x1p-512; P2 *= 0x1p-512; ++ep; }
             if (em < 0 && fabs(M1) > 0x1p256) { M1 *= 0x1p-512; M2 *= 0x1p-512; ++em; }
         }
-        if (live && (__float_as_int(to_f32_state(fmax(fabs(P1), fabs(P2)), 0.0, ep).z) >= 0 ||
-                     __float_as_int(to_f32_state(fmax(fabs(M1), fabs(M2)), 0.0, em).z) >= 0))
+        if (live && (__float_as_int(to_f32_state(P1, P2, ep).z) >= 0 || __float_as_int(to_f32_state(M1, M2, em).z) >= 0))
             any_live[threadIdx.x / 64] = 1;
         __syncthreads();
         write_flags(flags, blk_ofs[m] + (lb - l0s) / CKR, np, any_neg, any_live);

@@ -347,10 +347,8 @@ __global__ void __launch_bounds__(32, MINB) spin_synthesis32_kernel(GeomDev g, i
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const SpinPair s = spin_state(g, m, j, (int64_t)(grp * U + u) * 32 + lane, ckP + blk * np, ckM + blk * np);
-            // the sums are in units of 2^(64 e); e never falls from block to block, except from the 0 of empty sums
-            const float fp = s.ep > S.ep[u] ? ldexpf(1.f, 64 * max(-3, S.ep[u] - s.ep)) : 1.f;
-            const float fm = s.em > S.em[u] ? ldexpf(1.f, 64 * max(-3, S.em[u] - s.em)) : 1.f;
-            spin_scale(S, u, pk(fp, fm));
+            // the sums are in units of 2^(64 e)
+            spin_scale(S, u, pk(sums_to_unit(S.ep[u], s.ep), sums_to_unit(S.em[u], s.em)));
             S.ep[u] = s.ep;
             S.em[u] = s.em;
             S.v1[u] = pk(s.p1, s.m1);

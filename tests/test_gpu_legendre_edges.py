@@ -133,3 +133,64 @@ def test_alm2cl_sizes(hb, lmax, mmax, nmaps, cross):
         deg = 2 * np.arange(lmax + 1) + 1.0
         got = ops.alm2cl(a, b, lmax, mmax).cpu().numpy()
         assert np.all(np.abs(got - want / deg) <= 1e-13 * size / deg)
+
+
+def _odd_grid(oracle, nrings, nphi):
+    """Rings symmetric about the middle one, which lies at theta = pi/2 (cos = 6e-17, not zero)."""
+    th = np.linspace(0.02, np.pi - 0.02, nrings)
+    th[nrings // 2] = np.pi / 2
+    n = np.full(nrings, nphi, dtype=np.int32)
+    w = np.random.default_rng(nrings).uniform(0.5, 1.5, nrings) * 2.0 / nrings
+    return th, n, w, oracle.generic_geometry(th, n, weights=w), slice((nrings // 2) * nphi, (nrings // 2 + 1) * nphi)
+
+
+@pytest.mark.parametrize("nrings,lmax,mmax", [(129, 700, 700), (33, 600, 3), (2051, 520, 2)])
+def test_equator_ring(hb, oracle, nrings, lmax, mmax):
+    """On a ring at theta = pi/2 every second lambda_lm is near zero, also at the starts of the 256-l blocks: the
+    ring by itself, in both directions (1e-5 relative (L2) in FP32, 1e-10 in FP64, as above)."""
+    th, nphi, w, g, eq = _odd_grid(oracle, nrings, 16)
+    rng = np.random.default_rng(lmax)
+    a = _alm(oracle, rng, 1, lmax, mmax)[0]
+    mp = np.zeros(g["npix"])
+    mp[eq] = rng.standard_normal(16)
+    ref_map, ref_alm = oracle.alm2map(a, g, lmax, mmax)[eq], oracle.map2alm(mp, g, lmax, mmax)
+    G = hb.geometry.generic(th, nphi, w)
+    for prec, tol in (("fp64", 1e-10), ("fp32", 1e-5)):
+        got = hb.transforms.alm2map(torch.from_numpy(a).cuda(), G, lmax, mmax, precision=prec).double().cpu().numpy()[eq]
+        assert rel2(got, ref_map) < tol, (prec, "map")
+        got = hb.transforms.map2alm(torch.from_numpy(mp).cuda(), G, lmax, mmax, precision=prec).cpu().numpy()
+        assert rel2(got, ref_alm) < tol, (prec, "alm")
+
+
+@pytest.mark.parametrize("nrings,lmax,mmax", [(129, 700, 700), (33, 600, 3)])
+def test_equator_ring_spin(hb, oracle, nrings, lmax, mmax):
+    """The same for spin 2 (at m = 0 its functions have a definite parity, so one of two is near zero)."""
+    th, nphi, w, g, eq = _odd_grid(oracle, nrings, 16)
+    rng = np.random.default_rng(lmax)
+    a = _alm(oracle, rng, 2, lmax, mmax)
+    q = np.zeros((2, g["npix"]))
+    q[:, eq] = rng.standard_normal((2, 16))
+    ref_map = [x[eq] for x in oracle.alm2map_spin2(a[0], a[1], g, lmax, mmax)]
+    ref_alm = oracle.map2alm_spin2(q[0], q[1], g, lmax, mmax)
+    G = hb.geometry.generic(th, nphi, w)
+    for prec, tol in (("fp64", 1e-10), ("fp32", 1e-5)):
+        got = hb.transforms.alm2map_spin2(*(torch.from_numpy(x).cuda() for x in a), G, lmax, mmax, precision=prec)
+        back = hb.transforms.map2alm_spin2(*(torch.from_numpy(x).cuda() for x in q), G, lmax, mmax, precision=prec)
+        for i in range(2):
+            assert rel2(got[i].double().cpu().numpy()[eq], ref_map[i]) < tol, (prec, "map")
+            assert rel2(back[i].cpu().numpy(), ref_alm[i]) < tol, (prec, "alm")
+
+
+def test_equator_ring_batched(hb, oracle):
+    """The tensor-core path starts from the same checkpoints: the equator ring by itself (1e-5 relative (L2))."""
+    lmax, mmax, n = 600, 600, 3
+    th, nphi, w, g, eq = _odd_grid(oracle, 129, 16)
+    rng = np.random.default_rng(n)
+    a = _alm(oracle, rng, n, lmax, mmax)
+    mp = np.zeros((n, g["npix"]), dtype=np.float32)
+    mp[:, eq] = rng.standard_normal((n, 16))
+    bp = hb.batched.BatchedPlan([(hb.geometry.generic(th, nphi, w), lmax, mmax, n)])
+    got = bp.alm2map(torch.from_numpy(a).to("cuda", torch.complex64)).reshape(n, -1)[:, eq].double().cpu().numpy()
+    assert rel2(got, np.stack([oracle.alm2map(x, g, lmax, mmax)[eq] for x in a])) < 1e-5
+    got = bp.map2alm(torch.from_numpy(mp).cuda()).reshape(n, -1).to(torch.complex128).cpu().numpy()
+    assert rel2(got, np.stack([oracle.map2alm(x, g, lmax, mmax) for x in mp.astype(np.float64)])) < 1e-5

@@ -64,10 +64,12 @@ def _op(name: str, fn):
 
 
 def _plain(args) -> bool:
-    """Whether nothing but the computation can happen in a call: ordinary tensors outside autograd,
-    and no tracer, mode, transform (vmap, forward AD) or profiler that has to see the operator."""
+    """Whether nothing but the computation can happen in a call: ordinary tensors outside autograd, whose
+    storage holds their values (the dispatcher conjugates and negates lazy ones on the way to the operator), and
+    no tracer, mode, transform (vmap, forward AD) or profiler that has to see the operator."""
     for a in args:
-        if isinstance(a, torch.Tensor) and (type(a) is not torch.Tensor or (a.requires_grad and torch.is_grad_enabled())):
+        if isinstance(a, torch.Tensor) and (type(a) is not torch.Tensor or (a.requires_grad and torch.is_grad_enabled())
+                                            or a.is_conj() or a.is_neg()):
             return False
     return not (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
                 or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None

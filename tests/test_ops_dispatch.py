@@ -76,3 +76,67 @@ def test_same_result_and_same_autograd_behaviour():
     assert a.requires_grad
     with pytest.raises(RuntimeError):  # no gradient formula on this entry point: an error, not zeros
         a.abs().sum().backward()
+
+
+def _lazy(t):
+    """Tensors whose storage is not their value: still to be conjugated or negated."""
+    z = torch.complex(t, t + 1)
+    return {"conj": z.conj(), "neg": torch._neg_view(t)}
+
+
+@pytest.mark.parametrize("kind", ["conj", "neg"])
+def test_lazy_tensors_use_the_operator(kind):
+    from hellblast_b200 import ops
+    x = _lazy(torch.ones(2, 3))[kind]
+    assert not ops._plain((x, 3, None))
+    assert not ops._plain((torch.ones(2), 3, x))
+
+
+@pytest.mark.gpu
+def test_conjugated_inputs():
+    import hellblast_b200 as hb
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    lmax, nside = 40, 16
+    a, b = (torch.randn(2, hb.alm_ops.alm_size(lmax), dtype=torch.complex128, device="cuda", generator=gen) for _ in range(2))
+    for dt in (torch.complex128, torch.complex64):
+        x, y = a.to(dt), b.to(dt)
+        xc, yc = x.conj().resolve_conj(), y.conj().resolve_conj()
+        assert torch.equal(hb.hp_compat.alm2map(x.conj(), nside), hb.hp_compat.alm2map(xc, nside))
+        for got, want in zip(hb.hp_compat.alm2map_spin(x.conj(), y.conj(), 2, nside), hb.hp_compat.alm2map_spin(xc, yc, 2, nside)):
+            assert torch.equal(got, want)
+        want = hb.hp_compat.alm2cl(xc, y)
+        assert not torch.equal(want, hb.hp_compat.alm2cl(x, y))
+        assert torch.equal(hb.hp_compat.alm2cl(x.conj(), y), want)
+        assert torch.equal(hb.hp_compat.alm2cl(xc, yc.conj()), want)
+
+
+@pytest.mark.gpu
+def test_gradients_that_arrive_conjugated():
+    """autograd hands a backward pass lazily conjugated gradients: against a dense transform whose rows are the
+    transforms of the unit maps (1e-12 relative: FP64 sums of 48 terms)."""
+    import hellblast_b200 as hb
+    nside, lmax = 2, 4
+    npix = 12 * nside * nside
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    n = hb.alm_ops.alm_size(lmax)
+    w, v = (torch.randn(1, n, dtype=torch.complex128, device="cuda", generator=gen) for _ in range(2))
+    eye, none = torch.eye(npix, dtype=torch.float64, device="cuda"), torch.zeros(npix, npix, dtype=torch.float64, device="cuda")
+
+    def check(x, transform, dense, loss):
+        grads = []
+        for f in (transform, dense):
+            y = [t.clone().requires_grad_(True) for t in x]
+            loss(f(*y)).backward()
+            grads.append([t.grad for t in y])
+        for g, want in zip(*grads):
+            assert torch.linalg.norm(g - want) < 1e-12 * torch.linalg.norm(want)
+
+    def loss(alms):
+        return sum((a.conj() * k).sum().abs() for a, k in zip(alms, (w, v)))
+
+    m = torch.randn(2, 1, npix, dtype=torch.float64, device="cuda", generator=gen)
+    Y = hb.autograd.map2alm(eye, nside, lmax)
+    check([m[0]], lambda t: [hb.autograd.map2alm(t, nside, lmax)], lambda t: [t.to(Y.dtype) @ Y], loss)
+    (EQ, BQ), (EU, BU) = hb.autograd.map2alm_spin(eye, none, nside, lmax), hb.autograd.map2alm_spin(none, eye, nside, lmax)
+    check([m[0], m[1]], lambda q, u: hb.autograd.map2alm_spin(q, u, nside, lmax),
+          lambda q, u: (q.to(EQ.dtype) @ EQ + u.to(EU.dtype) @ EU, q.to(BQ.dtype) @ BQ + u.to(BU.dtype) @ BU), loss)

@@ -15,6 +15,7 @@ import torch
 from . import _lib as L
 from . import geometry as G
 from .ops import alm_size
+from .util import stored
 
 _cache: dict[tuple, "BatchedPlan"] = {}
 _lock = threading.Lock()
@@ -41,7 +42,7 @@ class BatchedPlan:
         self.total_alm = sum(alm_size(l, m) * k for _, l, m, k in self.specs)
 
     def alm2map(self, alm: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-        alm = alm.reshape(-1).contiguous()
+        alm = stored(alm.reshape(-1))
         if alm.dtype != torch.complex64 or alm.numel() != self.total_alm or not alm.is_cuda:
             raise ValueError(f"alm must be a CUDA complex64 tensor of {self.total_alm} elements")
         out = torch.empty(self.total_pix, dtype=torch.float32, device=alm.device) if out is None else out
@@ -52,12 +53,12 @@ class BatchedPlan:
     def map2alm(self, maps: torch.Tensor, out: torch.Tensor | None = None, fl: torch.Tensor | None = None) -> torch.Tensor:
         """maps -> alm; with ``fl`` (a per-l filter, >= max lmax + 1 values) every alm(l, m) is
         multiplied by fl[l] in the tensor-core kernel's store (almxfl fused)."""
-        maps = maps.reshape(-1).contiguous()
+        maps = stored(maps.reshape(-1))
         if maps.dtype != torch.float32 or maps.numel() != self.total_pix or not maps.is_cuda:
             raise ValueError(f"maps must be a CUDA float32 tensor of {self.total_pix} elements")
         out = torch.empty(self.total_alm, dtype=torch.complex64, device=maps.device) if out is None else out
         if fl is not None:
-            fl = torch.as_tensor(fl, dtype=torch.float32, device=maps.device).contiguous()
+            fl = stored(torch.as_tensor(fl, dtype=torch.float32, device=maps.device))
             if fl.numel() < max(s[1] for s in self.specs) + 1:
                 raise ValueError("fl needs at least lmax + 1 entries")
         L.call("hb_batched_map2alm_fl", self.handle, maps.data_ptr(), out.data_ptr(),

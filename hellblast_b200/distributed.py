@@ -17,6 +17,8 @@ from typing import Callable
 import torch
 import torch.distributed as dist
 
+from .util import stored
+
 
 def shard_range(n: int, rank: int, world: int) -> tuple[int, int]:
     """Contiguous, balanced shard [start, stop) of n items for ``rank`` of ``world``; the first
@@ -269,7 +271,7 @@ class MShardedSHT:
         nmaps = x_local.shape[0]
         F = torch.zeros(nmaps, self.mmax + 1, self.layout.npl(self.rank), 2, dtype=self.ct, device=self.device)
         if self.npix_local:
-            x = x_local.to(self.rt).contiguous()
+            x = stored(x_local.to(self.rt))
             L.call("hb_ring_analysis", self.lplan.handle, self.prec, nmaps, x.data_ptr(), None, F.data_ptr(), 0,
                    self._stream())
         return F
@@ -277,7 +279,7 @@ class MShardedSHT:
     def legendre_analysis(self, Fm: torch.Tensor) -> torch.Tensor:
         """[nmaps, |M_r|, npairs, 2] -> [nmaps, nalm] with this rank's orders filled."""
         from . import _lib as L
-        Fm = Fm.to(self.ct).contiguous()
+        Fm = stored(Fm.to(self.ct))
         nmaps = Fm.shape[0]
         alm = torch.zeros(nmaps, L.lib().hb_alm_size(self.lmax, self.mmax), dtype=self.ct, device=self.device)
         if self.mlist.numel():
@@ -288,7 +290,7 @@ class MShardedSHT:
     def legendre_synthesis(self, alm: torch.Tensor) -> torch.Tensor:
         """alm [nmaps, nalm] (this rank's orders read) -> [nmaps, |M_r|, npairs, 2]."""
         from . import _lib as L
-        a = alm.to(self.ct).contiguous()
+        a = stored(alm.to(self.ct))
         nmaps = a.shape[0]
         Gm = torch.zeros(nmaps, int(self.mlist.numel()), self.g.npairs, 2, dtype=self.ct, device=self.device)
         if self.mlist.numel():
@@ -299,7 +301,7 @@ class MShardedSHT:
     def ring_synthesis(self, G_local: torch.Tensor) -> torch.Tensor:
         """[nmaps, mmax+1, npl, 2] -> [nmaps, npix_local]: ring FFTs of this rank's pairs."""
         from . import _lib as L
-        Gl = G_local.to(self.ct).contiguous()
+        Gl = stored(G_local.to(self.ct))
         nmaps = Gl.shape[0]
         out = torch.empty(nmaps, self.npix_local, dtype=self.rt, device=self.device)
         if self.npix_local:

@@ -19,7 +19,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from .util import as_tensor, like_input
+from .util import as_tensor, like_input, stored
 
 
 def _dev(x=None):
@@ -42,7 +42,7 @@ def _i64(x, dev):
 
 
 def _f64(x, dev):
-    return as_tensor(x, torch.float64).to(device=dev, dtype=torch.float64).reshape(-1).contiguous()
+    return stored(as_tensor(x, torch.float64).to(device=dev, dtype=torch.float64).reshape(-1))
 
 
 def ring2nest(nside: int, ipix):
@@ -133,7 +133,7 @@ def reorder(map_in, r2n: bool = False, n2r: bool = False):
     x = t.reshape(-1, t.shape[-1]).to(dev)
     if x.dtype not in (torch.float32, torch.float64):
         x = x.to(torch.float64)
-    x = x.contiguous()
+    x = stored(x)
     npix = x.shape[-1]
     nside = int(round((npix / 12) ** 0.5))
     if 12 * nside * nside != npix:

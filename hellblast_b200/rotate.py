@@ -23,7 +23,7 @@ import torch
 
 from . import _lib as L
 from . import alm_ops
-from .util import as_tensor, like_input
+from .util import as_tensor, like_input, stored
 
 
 def _to_healpy(alm, lmax, alm_layout):
@@ -45,7 +45,7 @@ def rotate_alm_euler(alm, alpha, beta, gamma, lmax=None, *, alm_layout="healpy")
     """[nalm] or [nmaps, nalm] complex alm rotated by Euler angles (ZYZ)."""
     t, lmax = _to_healpy(alm, lmax, alm_layout)
     squeeze = t.dim() == 1
-    x = t.reshape(-1, t.shape[-1]).contiguous()
+    x = stored(t.reshape(-1, t.shape[-1]))
     if not x.is_cuda:
         raise ValueError("rotate_alm_euler needs CUDA tensors (there is no CPU path)")
     out = torch.empty_like(x)
@@ -69,7 +69,7 @@ def rotate_alm_z(alm, alpha, lmax=None, *, alm_layout="healpy"):
 
 def wigner_d_full(beta, l: int, batch: int = 1):
     """d^l_{mm'}(beta_b) for m, m' = -l..l: [B, 2l+1, 2l+1] float64 (wigner_fast.py:15-25)."""
-    b = as_tensor(beta, torch.float64).to(torch.float64).reshape(-1).contiguous()
+    b = stored(as_tensor(beta, torch.float64).reshape(-1))
     if not b.is_cuda:
         b = b.cuda()
     out = torch.empty(b.numel(), 2 * l + 1, 2 * l + 1, dtype=torch.float64, device=b.device)

@@ -27,6 +27,11 @@ def as_tensor(x, dtype=None) -> torch.Tensor:
     return t
 
 
+def stored(t: torch.Tensor) -> torch.Tensor:
+    """t contiguous, with a lazy conjugation or negation carried out: what a kernel may read at data_ptr()."""
+    return t.resolve_conj().resolve_neg().contiguous()
+
+
 def like_input(t: torch.Tensor, ref):
     """Return t as a CuPy array (DLPack) when ref was one, else as a torch tensor."""
     if _is_cupy(ref):

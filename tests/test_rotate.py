@@ -142,3 +142,22 @@ def test_gpu_rotation_inverse(lmax):
     a[: lmax + 1] = a[: lmax + 1].real.to(a.dtype)
     b = rotate.rotate_alm_euler(rotate.rotate_alm_euler(a, 0.3, 1.1, -0.7), 0.7, -1.1, -0.3)
     assert float(torch.linalg.norm(a - b) / torch.linalg.norm(a)) < 1e-10
+
+
+@pytest.mark.gpu
+def test_gpu_conjugated_alm():
+    """Lazily conjugated alm (torch's conj()) into the entry points that take no custom operator."""
+    import torch
+    import hellblast_b200 as hb
+    from hellblast_b200 import rotate
+    lmax, nside, n = 40, 16, 4
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    a = torch.randn(n, hb.alm_ops.alm_size(lmax), generator=gen, device="cuda", dtype=torch.complex128)
+    c = a.conj().resolve_conj()
+    got, want = rotate.rotate_alm_euler(a.conj(), 0.3, 0.4, -0.7), rotate.rotate_alm_euler(c, 0.3, 0.4, -0.7)
+    assert torch.linalg.norm(got - want) < 1e-12 * torch.linalg.norm(want)
+    a, c = a.to(torch.complex64), c.to(torch.complex64)
+    assert torch.equal(hb.batched.alm2map(a.conj(), nside, lmax), hb.batched.alm2map(c, nside, lmax))
+    m = torch.randn(n, 12 * nside * nside, generator=gen, device="cuda")
+    assert torch.equal(hb.batched.map2alm(torch._neg_view(m), nside, lmax), hb.batched.map2alm(-m, nside, lmax))
+    assert torch.equal(hb.pixelfunc.reorder(torch._neg_view(m), r2n=True), hb.pixelfunc.reorder(-m, r2n=True))

@@ -31,7 +31,7 @@
 //
 // What bounds the kernels: the FP64 pipe (62 FMA per clock and SM measured); the analysis adds a
 // warp reduction per l.  One map at nside 1024, lmax 2047: synthesis 2063 -> 1160 us, analysis
-// 2826 -> 1706 us (one-step form with a shared-memory reduction per l before); two maps 1.8 times one.
+// 2826 -> 1729 us (one-step form with a shared-memory reduction per l before); two maps 1.8 times one.
 #include <cmath>
 
 #include "hb_internal.cuh"
@@ -175,12 +175,12 @@ __device__ __forceinline__ void anal_chunk(State<U> &S, const Weights<NB, U> &W,
         red[lane >> 1] += s;
 }
 
-// a block's steps [0, nk) (nk a multiple of TL; past lmax the coefficients are zero); groups that
-// are evanescent as a whole run the recursion alone
+// a block's steps from k to nk (nk a multiple of TL; past lmax the coefficients are zero); groups that
+// are evanescent as a whole run the recursion alone.  Returns the next step: nk, or with held weights (held) the
+// one after a change of exponents.
 template <int ZONE, int U, int NB, int TL>
-__device__ __forceinline__ void anal_block(State<U> &S, const Weights<NB, U> &W, int nk, int &mode, const double2 *cf, double *red,
-                                           int lane) {
-    int k = 0;
+__device__ __forceinline__ int anal_block(State<U> &S, const Weights<NB, U> &W, int k, int nk, int &mode, const double2 *cf, double *red,
+                                          int lane, bool held) {
     while (mode != CLEAN && k < nk) {
         if (mode == DEAD) {
 #pragma unroll
@@ -189,10 +189,14 @@ __device__ __forceinline__ void anal_block(State<U> &S, const Weights<NB, U> &W,
             anal_chunk<ZONE, true, U, NB, TL>(S, W, cf + k, red + k * NB * 4, lane);
         }
         k += TL;
-        if (rescale(S, [](int) {})) mode = mode_of(S);
+        if (rescale(S, [](int) {})) {
+            mode = mode_of(S);
+            if (held) return k;
+        }
     }
 #pragma unroll 1
     for (; k < nk; k += TL) anal_chunk<ZONE, false, U, NB, TL>(S, W, cf + k, red + k * NB * 4, lane);
+    return k;
 }
 
 // One CTA per (order, chunk of ring pairs or all of them in turn, NB maps), every warp keeping one group of
@@ -224,9 +228,13 @@ __global__ void __launch_bounds__(NT, MINB) leg_analysis64_kernel(GeomDev g, Leg
         State<U> S;
         Weights<NB, U> W;
         const int zone = start_group(g, tab, m, grp, lane, S);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
+        // Weights of pair u.  Infinite or NaN ones are held back (zero, bit u of hold) while e < 0: the gate zeroes the
+        // values, and 0 times these is NaN.
+        unsigned hold = 0;
+        const auto weigh = [&](int u) {
             const int64_t p = unit_pair<U>(grp, u, lane);
+            double z = 0.0;  // stays zero with finite samples
+            hold &= ~(1u << u);
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 W.er[b][u] = W.ei[b][u] = W.qr[b][u] = W.qi[b][u] = 0.0;
@@ -237,9 +245,18 @@ __global__ void __launch_bounds__(NT, MINB) leg_analysis64_kernel(GeomDev g, Leg
                     W.ei[b][u] = fn.y + fs.y;
                     W.qr[b][u] = (fn.x - fs.x) * x;
                     W.qi[b][u] = (fn.y - fs.y) * x;
+                    z += 0.0 * W.er[b][u] + 0.0 * W.ei[b][u];
+                    z += 0.0 * W.qr[b][u] + 0.0 * W.qi[b][u];
                 }
             }
-        }
+            if (z != 0.0 && S.e[u] < 0) {
+                hold |= 1u << u;
+#pragma unroll
+                for (int b = 0; b < NB; ++b) W.er[b][u] = W.ei[b][u] = W.qr[b][u] = W.qi[b][u] = 0.0;
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < U; ++u) weigh(u);
         int mode = mode_of(S);
         if (lane == 0) wzone[warp] = any ? zone : -1;
         for (int l0 = m; l0 <= lmax; l0 += 2 * LKB, tab += LKB * LT_N) {
@@ -252,11 +269,16 @@ __global__ void __launch_bounds__(NT, MINB) leg_analysis64_kernel(GeomDev g, Leg
             }
             for (int i = lane; i < ROW; i += 32) mine[i] = 0.0;
             __syncthreads();
-            if (any) {
+            for (int k = any ? 0 : nkp; k < nkp;) {
+                const bool held = __any_sync(0xffffffffu, hold);
                 if (zone == ZPOLE)
-                    anal_block<ZPOLE, U, NB, TL>(S, W, nkp, mode, ca, mine, lane);
+                    k = anal_block<ZPOLE, U, NB, TL>(S, W, k, nkp, mode, ca, mine, lane, held);
                 else
-                    anal_block<ZEQ, U, NB, TL>(S, W, nkp, mode, cb, mine, lane);
+                    k = anal_block<ZEQ, U, NB, TL>(S, W, k, nkp, mode, cb, mine, lane, held);
+                if (!held) break;
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if ((hold >> u & 1) && S.e[u] >= 0) weigh(u);
             }
             __syncthreads();
             for (int i = tid; i < 2 * nk * NB * 4; i += NT) {

@@ -194,3 +194,39 @@ def test_equator_ring_batched(hb, oracle):
     assert rel2(got, np.stack([oracle.alm2map(x, g, lmax, mmax)[eq] for x in a])) < 1e-5
     got = bp.map2alm(torch.from_numpy(mp).cuda()).reshape(n, -1).to(torch.complex128).cpu().numpy()
     assert rel2(got, np.stack([oracle.map2alm(x, g, lmax, mmax) for x in mp.astype(np.float64)])) < 1e-5
+
+
+def _orders(alm, lmax, mmax, m0):
+    """The coefficients of the orders m0 .. mmax."""
+    return alm[..., m0 * (2 * lmax + 1 - m0) // 2 + m0:]
+
+
+@pytest.mark.parametrize("nside,lmax,nmaps,m0", [(64, 130, 1, 90), (128, 200, 2, 90), (512, 1100, 1, 90), (512, 600, 2, 90)])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_nan_stays_where_the_ring_contributes(hb, nside, lmax, nmaps, m0, prec):
+    """A NaN pixel on the ring next to the pole (theta < 0.013, l theta < 1.8): for m >= 90 the ring's lambda is
+    below 2^-256 at every l, (l theta / 2)^m / m! < 2^-400, and a ring that counts as zero adds nothing, be its
+    value finite or not."""
+    gen = torch.Generator(device="cuda").manual_seed(nside)
+    mp = torch.randn(nmaps, 12 * nside * nside, device="cuda", generator=gen, dtype=torch.float64)
+    bad = mp.clone()
+    mp[:, 1], bad[:, 1] = 0.0, float("nan")
+    a, b = (hb.hp_compat.map2alm(x, lmax=lmax, precision=prec) for x in (mp, bad))
+    assert torch.isnan(torch.view_as_real(b)).any()
+    assert torch.equal(torch.view_as_real(_orders(a, lmax, lmax, m0)), torch.view_as_real(_orders(b, lmax, lmax, m0)))
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("nmaps", [1, 2])
+def test_nan_reaches_the_orders_of_its_ring(hb, oracle, value, nmaps):
+    """The same ring (theta = 0.0128) where it counts, in FP64: lambda is past 2^-256 at every l of m <= 30, at m = 45
+    from some l on (2^-283 at l = 45, 2^-198 at l = 130)."""
+    nside, lmax = 64, 130
+    mp = torch.ones(nmaps, 12 * nside * nside, device="cuda", dtype=torch.float64)
+    mp[-1, 1] = value
+    a = hb.hp_compat.map2alm(mp, lmax=lmax)[-1].cpu().numpy()
+    at = lambda l, m: a[oracle.alm_index(lmax, l, m)]
+    assert not any(np.isfinite(at(l, m)) for m in (0, 1, 2, 30) for l in range(m, lmax + 1))
+    assert np.isfinite(at(45, 45)) and not np.isfinite(at(lmax, 45))
+    if nmaps > 1:
+        assert torch.isfinite(torch.view_as_real(hb.hp_compat.map2alm(mp, lmax=lmax)[0])).all()

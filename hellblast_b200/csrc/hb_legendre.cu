@@ -31,7 +31,7 @@
 //
 // What bounds the kernels: the FP64 pipe (62 FMA per clock and SM measured); the analysis adds a
 // warp reduction per l.  One map at nside 1024, lmax 2047: synthesis 2063 -> 1160 us, analysis
-// 2826 -> 1729 us (one-step form with a shared-memory reduction per l before); two maps 1.8 times one.
+// 2826 -> 1680 us (one-step form with a shared-memory reduction per l before); two maps 1.8 times one.
 #include <cmath>
 
 #include "hb_internal.cuh"
@@ -147,7 +147,9 @@ template <int NB, int U> struct Weights {
 };
 
 // TL two-l steps: values times weights summed over the group's pairs, added to the warp's row
-// red[(step * NB + map) * 4 + (E re, E im, O re, O im)]; values with e < 0 count as zero
+// red[(step * NB + map) * 4 + (E re, E im, O re, O im)].  GATED: pairs with e < 0 take no part.  Their terms are
+// predicated off: a zero value in their place would turn an infinite or NaN weight into NaN, and costs more
+// (nside 1024, lmax 2047: one map 1680 us, 1705 with zeroed values; two 3021, 3082).
 template <int ZONE, bool GATED, int U, int NB, int TL>
 __device__ __forceinline__ void anal_chunk(State<U> &S, const Weights<NB, U> &W, const double2 *cf, double *red, int lane) {
     double v[TL * NB * 4];
@@ -155,8 +157,20 @@ __device__ __forceinline__ void anal_chunk(State<U> &S, const Weights<NB, U> &W,
     for (int s = 0; s < TL; ++s) {
         two_step<ZONE>(S, cf[s], [&](int u, double ve, double vo) {
             if (GATED) {
-                ve = S.e[u] < 0 ? 0.0 : ve;
-                vo = S.e[u] < 0 ? 0.0 : vo;
+#pragma unroll
+                for (int i = 0; i < NB * 4; ++i)
+                    if (u == 0) v[s * NB * 4 + i] = 0.0;
+                if (S.e[u] >= 0) {
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        double *a = v + (s * NB + b) * 4;
+                        a[0] = fma(ve, W.er[b][u], a[0]);
+                        a[1] = fma(ve, W.ei[b][u], a[1]);
+                        a[2] = fma(vo, W.qr[b][u], a[2]);
+                        a[3] = fma(vo, W.qi[b][u], a[3]);
+                    }
+                }
+                return;
             }
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
@@ -175,12 +189,12 @@ __device__ __forceinline__ void anal_chunk(State<U> &S, const Weights<NB, U> &W,
         red[lane >> 1] += s;
 }
 
-// a block's steps from k to nk (nk a multiple of TL; past lmax the coefficients are zero); groups that
-// are evanescent as a whole run the recursion alone.  Returns the next step: nk, or with held weights (held) the
-// one after a change of exponents.
+// a block's steps [0, nk) (nk a multiple of TL; past lmax the coefficients are zero); groups that
+// are evanescent as a whole run the recursion alone
 template <int ZONE, int U, int NB, int TL>
-__device__ __forceinline__ int anal_block(State<U> &S, const Weights<NB, U> &W, int k, int nk, int &mode, const double2 *cf, double *red,
-                                          int lane, bool held) {
+__device__ __forceinline__ void anal_block(State<U> &S, const Weights<NB, U> &W, int nk, int &mode, const double2 *cf, double *red,
+                                           int lane) {
+    int k = 0;
     while (mode != CLEAN && k < nk) {
         if (mode == DEAD) {
 #pragma unroll
@@ -189,14 +203,10 @@ __device__ __forceinline__ int anal_block(State<U> &S, const Weights<NB, U> &W, 
             anal_chunk<ZONE, true, U, NB, TL>(S, W, cf + k, red + k * NB * 4, lane);
         }
         k += TL;
-        if (rescale(S, [](int) {})) {
-            mode = mode_of(S);
-            if (held) return k;
-        }
+        if (rescale(S, [](int) {})) mode = mode_of(S);
     }
 #pragma unroll 1
     for (; k < nk; k += TL) anal_chunk<ZONE, false, U, NB, TL>(S, W, cf + k, red + k * NB * 4, lane);
-    return k;
 }
 
 // One CTA per (order, chunk of ring pairs or all of them in turn, NB maps), every warp keeping one group of
@@ -228,13 +238,9 @@ __global__ void __launch_bounds__(NT, MINB) leg_analysis64_kernel(GeomDev g, Leg
         State<U> S;
         Weights<NB, U> W;
         const int zone = start_group(g, tab, m, grp, lane, S);
-        // Weights of pair u.  Infinite or NaN ones are held back (zero, bit u of hold) while e < 0: the gate zeroes the
-        // values, and 0 times these is NaN.
-        unsigned hold = 0;
-        const auto weigh = [&](int u) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
             const int64_t p = unit_pair<U>(grp, u, lane);
-            double z = 0.0;  // stays zero with finite samples
-            hold &= ~(1u << u);
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 W.er[b][u] = W.ei[b][u] = W.qr[b][u] = W.qi[b][u] = 0.0;
@@ -245,18 +251,9 @@ __global__ void __launch_bounds__(NT, MINB) leg_analysis64_kernel(GeomDev g, Leg
                     W.ei[b][u] = fn.y + fs.y;
                     W.qr[b][u] = (fn.x - fs.x) * x;
                     W.qi[b][u] = (fn.y - fs.y) * x;
-                    z += 0.0 * W.er[b][u] + 0.0 * W.ei[b][u];
-                    z += 0.0 * W.qr[b][u] + 0.0 * W.qi[b][u];
                 }
             }
-            if (z != 0.0 && S.e[u] < 0) {
-                hold |= 1u << u;
-#pragma unroll
-                for (int b = 0; b < NB; ++b) W.er[b][u] = W.ei[b][u] = W.qr[b][u] = W.qi[b][u] = 0.0;
-            }
-        };
-#pragma unroll
-        for (int u = 0; u < U; ++u) weigh(u);
+        }
         int mode = mode_of(S);
         if (lane == 0) wzone[warp] = any ? zone : -1;
         for (int l0 = m; l0 <= lmax; l0 += 2 * LKB, tab += LKB * LT_N) {
@@ -269,16 +266,11 @@ __global__ void __launch_bounds__(NT, MINB) leg_analysis64_kernel(GeomDev g, Leg
             }
             for (int i = lane; i < ROW; i += 32) mine[i] = 0.0;
             __syncthreads();
-            for (int k = any ? 0 : nkp; k < nkp;) {
-                const bool held = __any_sync(0xffffffffu, hold);
+            if (any) {
                 if (zone == ZPOLE)
-                    k = anal_block<ZPOLE, U, NB, TL>(S, W, k, nkp, mode, ca, mine, lane, held);
+                    anal_block<ZPOLE, U, NB, TL>(S, W, nkp, mode, ca, mine, lane);
                 else
-                    k = anal_block<ZEQ, U, NB, TL>(S, W, k, nkp, mode, cb, mine, lane, held);
-                if (!held) break;
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-                    if ((hold >> u & 1) && S.e[u] >= 0) weigh(u);
+                    anal_block<ZEQ, U, NB, TL>(S, W, nkp, mode, cb, mine, lane);
             }
             __syncthreads();
             for (int i = tid; i < 2 * nk * NB * 4; i += NT) {

@@ -25,7 +25,7 @@
 //
 // What bounds the kernels: the FP64 pipe, 4 operations per (l, ring pair) for the recursions and 8 per map
 // for the contraction, and in the analysis the warp reductions.  Three Q/U maps at nside 256, lmax 700:
-// synthesis 523 -> 440 us, analysis 1261 -> 636 us.
+// synthesis 523 -> 440 us, analysis 1261 -> 593 us.
 #include <cmath>
 
 #include "hb_internal.cuh"
@@ -170,7 +170,9 @@ template <int U> struct Weights {
     double2 w[2][U], v[2][U];  // [l - m even, odd]
 };
 
-// TL rows: sums over the group's pairs, added to the warp's row red[row * 4 + (E re, E im, B re, B im)]
+// Four rows: sums over the group's pairs, added to the warp's row red[row * 4 + (E re, E im, B re, B im)].  GATED:
+// P and M with e < 0 take no part, their terms predicated off (as in the scalar analysis; three maps at nside 256,
+// lmax 700, whole call 734 us, 764 with zeroed values; one at nside 1024, lmax 2047 5882, 5957).
 template <bool GATED, int U, int PAR>
 __device__ __forceinline__ void anal_chunk(State<U> &S, const Weights<U> &W, const double2 *cf, double *red, int lane) {
     double a[16];
@@ -178,12 +180,24 @@ __device__ __forceinline__ void anal_chunk(State<U> &S, const Weights<U> &W, con
     for (int s = 0; s < 4; ++s) {
         const int k = (s + PAR) & 1;
         spin_step(S, cf[s], [&](int u, double p, double q) {
-            if (GATED) {
-                p = S.ep[u] < 0 ? 0.0 : p;
-                q = S.em[u] < 0 ? 0.0 : q;
-            }
             const double2 w = W.w[k][u], v = W.v[k][u], wo = W.w[k ^ 1][u], vo = W.v[k ^ 1][u];
             double *o = a + 4 * s;
+            if (GATED) {
+                if (u == 0) o[0] = o[1] = o[2] = o[3] = 0.0;
+                if (S.em[u] >= 0) {
+                    o[0] = fma(q, v.x, o[0]);
+                    o[1] = fma(q, v.y, o[1]);
+                    o[2] = fma(-q, vo.y, o[2]);
+                    o[3] = fma(q, vo.x, o[3]);
+                }
+                if (S.ep[u] >= 0) {
+                    o[0] = fma(p, w.x, o[0]);
+                    o[1] = fma(p, w.y, o[1]);
+                    o[2] = fma(p, wo.y, o[2]);
+                    o[3] = fma(-p, wo.x, o[3]);
+                }
+                return;
+            }
             o[0] = fma(p, w.x, u ? fma(q, v.x, o[0]) : q * v.x);
             o[1] = fma(p, w.y, u ? fma(q, v.y, o[1]) : q * v.y);
             o[2] = fma(p, wo.y, u ? fma(-q, vo.y, o[2]) : -q * vo.y);
@@ -429,8 +443,8 @@ static int run_synthesis(const hb_plan *p, int nmaps, const double2 *E, const do
 
 // Pairs per lane: the synthesis reads 48 bytes of coefficients per l and warp from shared memory, as long
 // as the operations of two pairs; four pairs (10 warps per SM) 3.88 ms at nside 1024 where two (16 warps)
-// take 4.09, but 464 us at nside 256, lmax 700 (three maps) where two take 439.  The analysis: four 5.35 ms
-// and 636 us, two 6.06 ms and 667 us.  Below 256 pairs one, to spread over more warps.
+// take 4.09, but 464 us at nside 256, lmax 700 (three maps) where two take 439.  The analysis: four 5.25 ms
+// and 593 us, two (with the gate on the values) 6.06 ms and 667 us.  Below 256 pairs one, to spread over more warps.
 static int spin_analysis64(const hb_plan *p, int nmaps, const double2 *QF, const double2 *UF, double2 *E, double2 *B, cudaStream_t st) {
     if (p->g->d.npairs >= 256) return run_analysis<4, 128, 3>(p, nmaps, QF, UF, E, B, st);
     return run_analysis<1, 128, 4>(p, nmaps, QF, UF, E, B, st);

@@ -230,3 +230,30 @@ def test_nan_reaches_the_orders_of_its_ring(hb, oracle, value, nmaps):
     assert np.isfinite(at(45, 45)) and not np.isfinite(at(lmax, 45))
     if nmaps > 1:
         assert torch.isfinite(torch.view_as_real(hb.hp_compat.map2alm(mp, lmax=lmax)[0])).all()
+
+
+@pytest.mark.parametrize("nside,lmax", [(64, 130), (256, 300)])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_nan_stays_where_the_ring_contributes_spin(hb, nside, lmax, prec):
+    """The same for spin 2, whose functions are of order m - 2 in theta."""
+    gen = torch.Generator(device="cuda").manual_seed(nside)
+    q = torch.randn(2, 12 * nside * nside, device="cuda", generator=gen, dtype=torch.float64)
+    bad = q.clone()
+    q[:, 1], bad[:, 1] = 0.0, float("nan")
+    a, b = (hb.hp_compat.map2alm_spin(x[0], x[1], 2, lmax=lmax, precision=prec) for x in (q, bad))
+    for x, y in zip(a, b):
+        assert torch.isnan(torch.view_as_real(y)).any()
+        assert torch.equal(torch.view_as_real(_orders(x, lmax, lmax, 96)), torch.view_as_real(_orders(y, lmax, lmax, 96)))
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_nan_reaches_the_orders_of_its_ring_spin(hb, oracle, value):
+    """Spin 2 counts from 2^-256 too, in FP64: P and M are of order m + 2 and m - 2 in theta."""
+    nside, lmax = 64, 130
+    q = torch.ones(2, 12 * nside * nside, device="cuda", dtype=torch.float64)
+    q[0, 1] = value
+    for a in hb.hp_compat.map2alm_spin(q[0], q[1], 2, lmax=lmax):
+        a = a.cpu().numpy()
+        at = lambda l, m: a[oracle.alm_index(lmax, l, m)]
+        assert not any(np.isfinite(at(l, m)) for m in (0, 1, 2, 30) for l in range(max(m, 2), lmax + 1))
+        assert np.isfinite(at(48, 48)) and not np.isfinite(at(lmax, 47))

@@ -24,7 +24,7 @@
 // (a step with two roots and a division took over 100 per (l, m, m')), then the sum
 // over m': TL l at a time by a transposing warp reduction (16 values per lane), one shared atomic each.
 // CTAs hold chunks of 256 orders m' and add to the output with global atomics when there are
-// several.  One set of alm at lmax 767: 2880 -> 635 us.
+// several.  One set of alm at lmax 767: 2880 -> 609 us.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -244,7 +244,6 @@ __global__ void __launch_bounds__(ROT_NT, 2) rotate_alm_kernel(int lmax, const d
 #pragma unroll
             for (int i = 0; i < MM; ++i) {
                 const int m = mb + i, k = (CLEAN ? l : min(l, lmax)) - mb;
-                double p, q;
                 if (CLEAN || (on && l > max(m, mp))) {
                     const double2 f = TAB ? fc[k * MM + i] : rot_factors(l, m);
                     const double g = f.x * i1, c = f.y * r, mm = (double)m * (double)mp;
@@ -252,16 +251,19 @@ __global__ void __launch_bounds__(ROT_NT, 2) rotate_alm_kernel(int lmax, const d
                     P[i].template step<CLEAN>(!CLEAN && l == 1 && m == 0 && mp == 0 ? x : (X - mm) * g, c);
                     Q[i].template step<CLEAN>((X + mm) * g, c);
                 }
+                double *o = v + (s * MM + i) * 2;
                 if (CLEAN) {
-                    p = P[i].d1;
-                    q = qs * Q[i].d1;
-                } else {
-                    const bool in = on && l >= m;
-                    p = in ? P[i].value() : 0.0;
-                    q = in ? qs * Q[i].value() : 0.0;
+                    const double q = qs * Q[i].d1;
+                    o[0] = (P[i].d1 + q) * zr;
+                    o[1] = (P[i].d1 - q) * zi;
+                } else {  // an input whose d is out of range does not count, infinite and NaN ones neither
+                    o[0] = o[1] = 0.0;
+                    if (on && l >= m && max(P[i].e, Q[i].e) == 0) {
+                        const double p = P[i].value(), q = qs * Q[i].value();
+                        o[0] = (p + q) * zr;
+                        o[1] = (p - q) * zi;
+                    }
                 }
-                v[(s * MM + i) * 2] = (p + q) * zr;
-                v[(s * MM + i) * 2 + 1] = (p - q) * zi;
             }
         }
         const double t = warp_sums<ROT_V>(v, lane);
@@ -338,7 +340,8 @@ int hb_rotate_alm(int lmax, int nmaps, const void *alm_in, void *alm_out, double
     const auto *in = (const double2 *)alm_in;
     auto *out = (double2 *)alm_out;
     // Two orders per CTA while the tables fit (lmax <= 2800), else one, without tables where they do not
-    // fit either.  At lmax 767 two orders take 635 us, four 676 us (both at two CTAs per SM).
+    // fit either.  At lmax 767 two orders take 609 us; compared with four orders, 635 against 676 us (both at two
+    // CTAs per SM, before the input's gate was predicated).
     const auto st = (cudaStream_t)s;
     if (rot_smem<2, true>(lmax) <= 220 * 1024) return run_rotate<2, true>(lmax, nmaps, in, out, alpha, br, gamma, st);
     if (rot_smem<1, true>(lmax) <= 220 * 1024) return run_rotate<1, true>(lmax, nmaps, in, out, alpha, br, gamma, st);

@@ -161,3 +161,27 @@ def test_gpu_conjugated_alm():
     m = torch.randn(n, 12 * nside * nside, generator=gen, device="cuda")
     assert torch.equal(hb.batched.map2alm(torch._neg_view(m), nside, lmax), hb.batched.map2alm(-m, nside, lmax))
     assert torch.equal(hb.pixelfunc.reorder(torch._neg_view(m), r2n=True), hb.pixelfunc.reorder(-m, r2n=True))
+
+
+@pytest.mark.gpu
+def test_gpu_rotation_nan_stays_where_it_contributes():
+    """A NaN at (l, m') reaches the (l, m) whose d^l_{m m'} is in range.  d^300_{m, +-300}(0.1) <= C(600, 300 + m)^1/2
+    sin(0.05)^(300 - m) is below 2^-128 for m <= 200 (2^300 2^-432): those add nothing, be the value finite or not."""
+    import torch
+    from hellblast_b200 import alm_ops, rotate
+    lmax = 301
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.randn(alm_ops.alm_size(lmax), generator=gen, device="cuda", dtype=torch.complex128)
+    a[: lmax + 1] = a[: lmax + 1].real.to(a.dtype)
+    hit = alm_ops.alm_index(lmax, 300, 300)
+    bad = a.clone()
+    a[hit], bad[hit] = 0.0, float("nan")
+    x, y = (rotate.rotate_alm_euler(t, 0.3, 0.1, -0.7) for t in (a, bad))
+    m = np.arange(lmax + 1)
+    at = torch.from_numpy(alm_ops.alm_index(lmax, 300, m[:301])).cuda()
+    assert torch.isnan(y[at[300]].real)
+    finite = torch.isfinite(torch.view_as_real(y)).all(-1)
+    assert finite[at[:201]].all()
+    same = torch.ones(a.numel(), dtype=torch.bool, device="cuda")
+    same[at[201:]] = False
+    assert torch.linalg.norm((x - y)[same]) < 1e-12 * torch.linalg.norm(x)

@@ -64,16 +64,19 @@ def _op(name: str, fn):
 
 
 def _plain(args) -> bool:
-    """Whether nothing but the computation can happen in a call: ordinary tensors outside autograd, whose
-    storage holds their values (the dispatcher conjugates and negates lazy ones on the way to the operator), and
-    no tracer, mode, transform (vmap, forward AD) or profiler that has to see the operator."""
+    """Whether nothing but the computation can happen in a call: no tracer, mode, transform (vmap, forward AD) or
+    profiler that has to see the operator, and ordinary tensors outside autograd whose storage holds their values
+    (not meta or all-zero tensors, which have none, nor lazily conjugated or negated ones, which the dispatcher
+    resolves on the way to the operator)."""
+    if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
+            or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None
+            or torch.autograd.forward_ad._current_level >= 0 or torch.autograd._profiler_enabled()):
+        return False
     for a in args:
         if isinstance(a, torch.Tensor) and (type(a) is not torch.Tensor or (a.requires_grad and torch.is_grad_enabled())
-                                            or a.is_conj() or a.is_neg()):
+                                            or a.is_conj() or a.is_neg() or a.data_ptr() == 0):
             return False
-    return not (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
-                or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None
-                or torch.autograd.forward_ad._current_level >= 0 or torch.autograd._profiler_enabled())
+    return True
 
 
 def call(op, *args):

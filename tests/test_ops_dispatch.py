@@ -140,3 +140,18 @@ def test_gradients_that_arrive_conjugated():
     (EQ, BQ), (EU, BU) = hb.autograd.map2alm_spin(eye, none, nside, lmax), hb.autograd.map2alm_spin(none, eye, nside, lmax)
     check([m[0], m[1]], lambda q, u: hb.autograd.map2alm_spin(q, u, nside, lmax),
           lambda q, u: (q.to(EQ.dtype) @ EQ + u.to(EU.dtype) @ EU, q.to(BQ.dtype) @ BQ + u.to(BU.dtype) @ BU), loss)
+
+
+@pytest.mark.parametrize("kind", ["meta", "zero"])
+def test_tensors_without_storage_use_the_operator(kind):
+    from hellblast_b200 import ops
+    x = torch.ones(2, 3, device="meta") if kind == "meta" else torch._efficientzerotensor((2, 3))
+    assert not ops._plain((x, 3, None))
+    assert not ops._plain((torch.ones(2), 3, x))
+
+
+@pytest.mark.gpu
+def test_meta_tensors_give_shapes():
+    import hellblast_b200 as hb
+    a = hb.hp_compat.map2alm(torch.empty(3, 12 * 16 * 16, device="meta"), lmax=20)
+    assert a.is_meta and a.shape == (3, hb.alm_ops.alm_size(20)) and a.dtype == torch.complex64

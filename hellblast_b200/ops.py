@@ -24,7 +24,10 @@ def _prec(dtype: torch.dtype) -> int:
 
 
 def _stream(dev: torch.device) -> int:
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if dev.index is None else dev.index)
+    try:
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if dev.index is None else dev.index)
+    except AttributeError:  # a torch without this shortcut (2 us of host time)
+        return torch.cuda.current_stream(dev).cuda_stream
 
 
 def _check_cuda(*ts):
@@ -67,10 +70,13 @@ def _plain(args) -> bool:
     """Whether nothing but the computation can happen in a call: no tracer, mode, transform (vmap, forward AD) or
     profiler that has to see the operator, and ordinary tensors outside autograd whose storage holds their values
     (not meta or all-zero tensors, which have none, nor lazily conjugated or negated ones, which the dispatcher
-    resolves on the way to the operator)."""
-    if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
-            or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None
-            or torch.autograd.forward_ad._current_level >= 0 or torch.autograd._profiler_enabled()):
+    resolves on the way to the operator).  A torch that lacks one of these internal queries has no plain calls."""
+    try:
+        if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
+                or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None
+                or torch.autograd.forward_ad._current_level >= 0 or torch.autograd._profiler_enabled()):
+            return False
+    except AttributeError:
         return False
     for a in args:
         if isinstance(a, torch.Tensor) and (type(a) is not torch.Tensor or (a.requires_grad and torch.is_grad_enabled())

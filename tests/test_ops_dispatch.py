@@ -155,3 +155,30 @@ def test_meta_tensors_give_shapes():
     import hellblast_b200 as hb
     a = hb.hp_compat.map2alm(torch.empty(3, 12 * 16 * 16, device="meta"), lmax=20)
     assert a.is_meta and a.shape == (3, hb.alm_ops.alm_size(20)) and a.dtype == torch.complex64
+
+
+@pytest.mark.parametrize("owner,name", [
+    (torch._C, "_len_torch_dispatch_stack"), (torch._C, "_len_torch_function_stack"), (torch._C._functorch, "peek_interpreter_stack"),
+    (torch._C, "_get_tracing_state"), (torch.autograd.forward_ad, "_current_level"), (torch.autograd, "_profiler_enabled")],
+    ids=lambda v: v if isinstance(v, str) else "")
+def test_a_torch_without_an_internal_query_uses_the_operator(monkeypatch, owner, name):
+    from hellblast_b200 import ops
+    t = torch.ones(2)
+    assert ops._plain((t,))
+    with monkeypatch.context() as m:
+        m.delattr(owner, name)
+        plain = ops._plain((t,))
+    assert not plain
+
+
+@pytest.mark.gpu
+def test_stream_without_the_shortcut(monkeypatch):
+    from hellblast_b200 import ops
+    dev = torch.device("cuda", 0)
+    with torch.cuda.stream(torch.cuda.Stream(dev)):
+        want = torch.cuda.current_stream(dev).cuda_stream
+        assert ops._stream(dev) == want
+        with monkeypatch.context() as m:
+            m.delattr(torch._C, "_cuda_getCurrentRawStream")
+            got = ops._stream(dev)
+    assert got == want

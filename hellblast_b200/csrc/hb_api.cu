@@ -126,13 +126,13 @@ static int alm2map_spin_impl(const hb_plan *p, int nmaps, const void *E, const v
                                  st);
 }
 
-// alm2cl (alm_ops.py:19-32): a CTA owns 32 consecutive l of one map (the lanes) and its 32 warps
-// (fewer for small spectra) split the m range, so every warp load reads 32 consecutive l of one healpy
+// alm2cl (alm_ops.py:19-32): a CTA owns 32 consecutive l of one map (the lanes) and its 4 to 32 warps
+// (cl_warps) split the m range, so every warp load reads 32 consecutive l of one healpy
 // m-column (256 B); FP64 accumulation, one shared-memory reduction over the warps, no atomics.
 // HBM-bound for a batch; a single alm has only lmax / 32 CTAs and is bound by the latency of a warp's chain
 // of loads, so a CTA has all the warps it may and a warp 8 loads in flight.  Against 8 warps with 4 m each
-// in flight and every alm loaded twice, complex64, us: lmax 2047 26.9 -> 13.5, 16 of them 86 -> 70, 64 of
-// lmax 4095 887 -> 748; two alm, lmax 2047 27.9 -> 18.2.
+// in flight and every alm loaded twice, complex64, us: lmax 2047 26.9 -> 13.5, 64 of lmax 4095
+// 887 -> 692; two alm, lmax 2047 27.9 -> 18.2.
 // AUTO: the spectrum of one alm with itself.
 constexpr int CL_WARPS = 32;
 template <typename V, bool AUTO>
@@ -171,16 +171,25 @@ __global__ void __launch_bounds__(32 * CL_WARPS) alm2cl_kernel(int lmax, int mma
     }
 }
 
-// Warps that find work, at mmax 20 / 64 / 128 / 256 / 2047 in us: 8 warps 2.0 / 2.4 / 3.0 / 4.4 / 23.9, 16 warps 2.2 /
-// 2.1 / 2.7 / 3.6 / 16.1, 32 warps 2.5 / 2.8 / 3.3 / 3.5 / 13.5; where CTAs queue (64 alm of lmax 4095) 16 warps
-// 748, 32 warps 844.
-static int cl_warps(int mmax, int64_t ctas) { return mmax < 40 ? 8 : (mmax < 256 || ctas >= 4096 ? 16 : CL_WARPS); }
+// Warps per CTA.  Few CTAs: all that find work, since a warp waits on its chain of loads.  CTAs that fill the GPU: 8, as
+// a CTA's start and the sum over its warps cost more than they give; in between 16, longer for complex128, whose
+// loads are twice the bytes.  us with 8 / 16 / 32 warps, complex64 auto spectra: 1 alm of lmax 2047 (64 CTAs) 25.2 /
+// 18.6 / 14.8, 8 (512 CTAs) 44.5 / 40.7 / 41.4, 64 (4096) 191 / 208 / 246; lmax 300, 8 alm 6.4 / 5.8 / 6.4, 64 (640)
+// 10.4 / 12.2 / 15.3, 512 46 / 62 / 96; lmax 60, 5000 alm 29 / 58 / 139, lmax 10, 5000 alm 15 / 25 / 47 (4 warps 10).
+// complex128: lmax 400, 64 alm crossed (832 CTAs) 36.5 / 32.9 / 32.9, lmax 1300, 16 crossed (656) 83 / 79 / 72.
+static int cl_warps(int mmax, int64_t ctas, bool fp64) {
+    if (mmax < 24) return 4;
+    if (mmax < 40) return 8;
+    if (mmax < 256) return ctas <= 296 ? 16 : 8;
+    if (ctas <= (mmax >= 1000 ? (fp64 ? 4096 : 592) : mmax >= 700 ? 256 : 148)) return CL_WARPS;
+    return ctas <= (fp64 ? 8192 : mmax >= 512 ? 4096 : 592) ? 16 : 8;
+}
 template <typename V>
 static int alm2cl_impl(int lmax, int mmax, int nmaps, const V *a1, const V *a2, double *cl, cudaStream_t st) {
     if (lmax < 0 || mmax < 0 || mmax > lmax || nmaps <= 0 || nmaps > 65535 || !a1 || !cl)
         return fail(HB_ERR_INVALID, "hb_alm2cl: bad arguments");
     dim3 grid((unsigned)((lmax + 32) / 32), (unsigned)nmaps);
-    const int nw = cl_warps(mmax, (int64_t)grid.x * nmaps);
+    const int nw = cl_warps(mmax, (int64_t)grid.x * nmaps, sizeof(V) == 16);
     if (!a2 || a2 == a1)
         alm2cl_kernel<V, true><<<grid, 32 * nw, 0, st>>>(lmax, mmax, a1, a1, alm_size(lmax, mmax), cl);
     else

@@ -257,3 +257,21 @@ def test_nan_reaches_the_orders_of_its_ring_spin(hb, oracle, value):
         at = lambda l, m: a[oracle.alm_index(lmax, l, m)]
         assert not any(np.isfinite(at(l, m)) for m in (0, 1, 2, 30) for l in range(max(m, 2), lmax + 1))
         assert np.isfinite(at(48, 48)) and not np.isfinite(at(lmax, 47))
+
+
+@pytest.mark.parametrize("lmax,nmaps", [(22, 3), (23, 2), (24, 1), (39, 1), (40, 2), (100, 74), (100, 75), (256, 16), (256, 17), (256, 66),
+                                        (511, 37), (511, 38), (512, 9), (1000, 19), (600, 216)])
+def test_alm2cl_warps(hb, oracle, lmax, nmaps):
+    """alm2cl where its CTAs change their number of warps with the number of CTAs; the first and the last spectrum
+    (tolerance as in test_alm2cl_sizes: at most 2 * 1001 products per value)."""
+    from hellblast_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(lmax)
+    for dt in (torch.complex64, torch.complex128):
+        a, b = (torch.randn(nmaps, oracle.alm_size(lmax), dtype=dt, device="cuda", generator=gen) for _ in range(2))
+        for other in (None, b):
+            got = ops.alm2cl(a, other, lmax, lmax)
+            for i in (0, nmaps - 1):
+                x, y = (t[i].to(torch.complex128).cpu().numpy() for t in (a, a if other is None else b))
+                want = oracle.alm2cl(x, lmax, alm2=y)
+                size = oracle.alm2cl(np.abs(x).astype(complex), lmax, alm2=np.abs(y).astype(complex))
+                assert np.all(np.abs(got[i].cpu().numpy() - want) <= 1e-13 * size)

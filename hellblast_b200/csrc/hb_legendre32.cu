@@ -465,12 +465,14 @@ template <int U, int NB, int MINB> static int run_synthesis(const Leg32 &L, int 
     return HB_OK;
 }
 
-// The number of pairs decides how the analysis orders its sum (columns of K pairs, NT columns): 2048
-// pairs per chunk from 1024 pairs on (above 1024; the K = 4 form is the same sum when the second half
-// is empty), 512 from 256 on, then 128 and 64.  K NB stays at 8 where registers hold it.
+// The number of pairs decides how the analysis orders its sum (columns of K pairs, NT columns): one chunk of 512
+// up to 512 pairs and of 1024 up to 1024, chunks of 2048 above, of 128 and 64 below 256 pairs.  In us, chunks of 512 /
+// 1024 / 2048, lmax equal to the pairs: 600 pairs, one map 100 / 88 / 134, two 142 / 119 / 252; 1000, 226 / 232 / 344, two
+// 334 / 317 / 670; lmax 1.5 times the pairs: 600, 182 / 182 / 274; 1000, 442 / 495 / 733; 2048, 2940 / 3237 / 2794.  Chunks of
+// 2048 leave no registers for a second map's weights, so their maps run singly.
 template <int NB> static int analysis_nb(const Leg32 &L, int nz, const float2 *F, float2 *alm) {
     if (L.np() > 1024) return run_analysis<8, 8, 256, 1, 2>(L, nz * NB, F, alm);
-    if (L.np() == 1024) return run_analysis<4, 4, 256, NB, 2>(L, nz, F, alm);
+    if (L.np() > 512) return run_analysis<4, 4, 256, NB, 2>(L, nz, F, alm);
     if (L.np() >= 256) return run_analysis<4, 4, 128, NB, 5>(L, nz, F, alm);
     if (L.np() >= 64) return run_analysis<2, 2, 64, NB, 10>(L, nz, F, alm);
     return run_analysis<2, 1, 64, NB, 10>(L, nz, F, alm);

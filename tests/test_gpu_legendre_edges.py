@@ -275,3 +275,34 @@ def test_alm2cl_warps(hb, oracle, lmax, nmaps):
                 want = oracle.alm2cl(x, lmax, alm2=y)
                 size = oracle.alm2cl(np.abs(x).astype(complex), lmax, alm2=np.abs(y).astype(complex))
                 assert np.all(np.abs(got[i].cpu().numpy() - want) <= 1e-13 * size)
+
+
+@pytest.mark.parametrize("npairs", [255, 256, 511, 513, 700, 1000, 1023, 1024, 1025, 2049])
+def test_fp32_analysis_pair_counts(hb, npairs):
+    """Numbers of ring pairs around those at which the FP32 analysis changes its chunks of pairs.  With one pair not zero
+    no sum rounds, so alm has the bits that the pair gives in a grid of its own; and maps that share a recursion have the
+    bits of single ones."""
+    from hellblast_b200 import _lib as L
+    from hellblast_b200 import geometry as G
+    lmax, mmax, nrings = 300, 6, 2 * npairs - 1
+    th = (np.arange(nrings) + 0.5) * np.pi / nrings
+    st = torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device="cuda").manual_seed(npairs)
+    nalm = L.lib().hb_alm_size(lmax, mmax)
+
+    def analysis(theta, F):
+        g = G.generic(theta, np.full(len(theta), 4, np.int32), np.ones(len(theta)))
+        assert g.npairs == F.shape[2]
+        alm = torch.full((F.shape[0], nalm), float("nan"), dtype=torch.complex64, device="cuda")
+        L.call("hb_legendre_analysis", G.plan(g, lmax, mmax, precision=32).handle, 32, F.shape[0], F.data_ptr(), alm.data_ptr(), st)
+        return torch.view_as_real(alm)
+
+    full = torch.view_as_complex(torch.randn(3, mmax + 1, npairs, 2, 2, device="cuda", generator=gen))
+    alone = analysis(th, full[:1].contiguous())
+    assert torch.isfinite(alone).all()
+    assert torch.equal(analysis(th, full)[0], alone[0]) and torch.equal(analysis(th, full[:2].contiguous())[0], alone[0])
+    for p in {0, 63, 64, 127, 128, 255, 256, 511, 512, 1023, 1024, 2047, 2048, npairs - 2}:
+        if p < npairs - 1:  # (the last pair is the equator, which has no south ring)
+            F = torch.zeros_like(full[:1])
+            F[:, :, p] = full[:1, :, p]
+            assert torch.equal(analysis(th, F), analysis(th[[p, nrings - 1 - p]], full[:1, :, p:p + 1].contiguous())), p

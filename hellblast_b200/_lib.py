@@ -96,6 +96,7 @@ SIGNATURES["hb_map2alm_f32_noalloc"] = (i32, [vp, i32, vp, vp, vp, i32, vp])
 
 HB_PLAN_FP32 = 1
 HB_PLAN_SPIN2_FP32 = 2
+HB_PLAN_NO_FP64 = 4
 HB_BATCHED_BF16 = 1
 HB_BATCHED_WIDE = 2
 

@@ -9,11 +9,14 @@
 
 namespace hb {
 
+// prec: of the Legendre stage, or 0 for the ring stages, which need no tables of the plan
 static int check_plan(const hb_plan *p, int nmaps, int prec, bool spin, const char *who) {
     if (!p || !p->g) return fail(HB_ERR_INVALID, std::string(who) + ": null plan");
     if (nmaps <= 0 || nmaps > 65535) return fail(HB_ERR_INVALID, std::string(who) + ": nmaps must lie in [1, 65535]");
     if (prec == 32 && !spin && !p->ck)
         return fail(HB_ERR_INVALID, std::string(who) + ": FP32 transforms need a plan created with HB_PLAN_FP32");
+    if (prec == 64 && !spin && !p->leg.base)
+        return fail(HB_ERR_INVALID, std::string(who) + ": FP64 scalar transforms need a plan created without HB_PLAN_NO_FP64");
     if (prec == 32 && spin && !p->ckP)
         return fail(HB_ERR_INVALID,
                     std::string(who) + ": FP32 spin-2 transforms need a plan created with HB_PLAN_SPIN2_FP32");
@@ -304,13 +307,13 @@ int hb_map2alm_spin2_adjoint_f64(const hb_plan *p, int nmaps, const double *gE, 
 int hb_ring_analysis(const hb_plan *p, int prec, int nmaps, const void *maps, const double *w, void *F, int flags,
                      hb_stream_t s) {
     if ((prec != 32 && prec != 64) || !maps || !F) return fail(HB_ERR_INVALID, "hb_ring_analysis: bad args");
-    int rc = check_plan(p, nmaps, 64, false, "hb_ring_analysis");
+    int rc = check_plan(p, nmaps, 0, false, "hb_ring_analysis");
     if (rc) return rc;
     return launch_ring_analysis(p->g->d, prec, nmaps, maps, p->g->d.npix, w, F, p->mmax, flags, false, false, ST(s));
 }
 int hb_ring_synthesis(const hb_plan *p, int prec, int nmaps, const void *G, void *maps, int flags, hb_stream_t s) {
     if ((prec != 32 && prec != 64) || !maps || !G) return fail(HB_ERR_INVALID, "hb_ring_synthesis: bad args");
-    int rc = check_plan(p, nmaps, 64, false, "hb_ring_synthesis");
+    int rc = check_plan(p, nmaps, 0, false, "hb_ring_synthesis");
     if (rc) return rc;
     return launch_ring_synthesis(p->g->d, prec, nmaps, G, p->mmax, maps, p->g->d.npix, nullptr, false, true, flags,
                                  ST(s));

@@ -174,7 +174,7 @@ struct hb_plan {
     size_t bytes;
     int64_t *blk_ofs;       // [mmax+2] first checkpoint block of each m (scalar)
     int64_t *blk_ofs_spin;  // [mmax+2] same for the spin-2 recursions (blocks from max(m,2))
-    hb::LegTab leg;
+    hb::LegTab leg;         // leg.base null with HB_PLAN_NO_FP64
     float2 *leg32;          // FP32 plans: (A_l, B_l) of the one-step recursion, [blk_ofs[m] * 256 + l - m]
     float4 *ck;             // scalar checkpoints, or null
     uint8_t *ck_flags;      // [blocks][flag_stride] FL_CLEAN: the 64 pairs start the block with e = 0, FL_MIXED: some

@@ -15,9 +15,10 @@
 // Each row of the scalar table has a flag byte per 64 pairs (hb_internal.cuh) by which the FP32
 // kernels skip blocks that stay evanescent.
 //
-// Every plan also holds the FP64 coefficient tables of the scalar recursions (LegTab): their scale
-// factors are products over l, which a kernel would have to rebuild per CTA (48 bytes per (l, m),
-// 0.4 GB at lmax 4095).  FP32 plans hold the one-step coefficients (8 bytes per (l, m)).
+// Plans for FP64 calls (all without HB_PLAN_NO_FP64) hold the FP64 coefficient tables of the scalar
+// recursions (LegTab): their scale factors are products over l, which a kernel would have to rebuild per
+// CTA (48 bytes per (l, m), 0.4 GB at lmax 4095).  FP32 plans hold the one-step coefficients (8 bytes per
+// (l, m)).
 #include <cmath>
 #include <vector>
 
@@ -280,11 +281,11 @@ int hb_plan_create(const hb_geom *g, int lmax, int mmax, int flags, hb_plan **ou
         ofs_s[m + 1] = ofs_s[m] + nblk(lmax, m > 2 ? m : 2);
         ofs_t[m + 1] = ofs_t[m] + (lmax - m) / 2 + 1;
     }
-    const bool scalar = (flags & HB_PLAN_FP32) != 0, spin = (flags & HB_PLAN_SPIN2_FP32) != 0;
+    const bool scalar = (flags & HB_PLAN_FP32) != 0, spin = (flags & HB_PLAN_SPIN2_FP32) != 0, fp64 = !(flags & HB_PLAN_NO_FP64);
     size_t bytes = 0;
     auto carve = [&](size_t b) { size_t o = bytes; bytes += (b + 255) & ~(size_t)255; return o; };
     size_t o_ofs = carve(8 * (mmax + 2)), o_ofss = carve(8 * (mmax + 2)), o_ofst = carve(8 * (mmax + 2));
-    const size_t o_leg = carve(8 * LT_N * (size_t)ofs_t[mmax + 1]);
+    const size_t o_leg = fp64 ? carve(8 * LT_N * (size_t)ofs_t[mmax + 1]) : 0;
     const size_t o_flags = scalar ? carve((size_t)ofs[mmax + 1] * flag_stride(np)) : 0;
     const size_t o_leg32 = scalar ? carve(8 * (size_t)ofs[mmax + 1] * CKR) : 0;
     size_t o_ck = scalar ? carve(16 * (size_t)ofs[mmax + 1] * np) : 0;
@@ -302,7 +303,7 @@ int hb_plan_create(const hb_geom *g, int lmax, int mmax, int flags, hb_plan **ou
     p->bytes = bytes;
     p->blk_ofs = (int64_t *)(base + o_ofs);
     p->blk_ofs_spin = (int64_t *)(base + o_ofss);
-    p->leg = {(double *)(base + o_leg), (int64_t *)(base + o_ofst)};
+    p->leg = {fp64 ? (double *)(base + o_leg) : nullptr, (int64_t *)(base + o_ofst)};
     p->leg32 = scalar ? (float2 *)(base + o_leg32) : nullptr;
     p->ck_flags = scalar ? (uint8_t *)(base + o_flags) : nullptr;
     p->ck = scalar ? (float4 *)(base + o_ck) : nullptr;
@@ -317,7 +318,7 @@ int hb_plan_create(const hb_geom *g, int lmax, int mmax, int flags, hb_plan **ou
         rc = fail(HB_ERR_CUDA, "hb_plan_create: upload failed");
     dim3 grid((unsigned)(mmax + 1), (unsigned)((np + CK_NT - 1) / CK_NT));
     if (rc == HB_OK) {
-        leg_table_kernel<<<(unsigned)(mmax / 32 + 1), 32>>>(lmax, mmax, p->leg);
+        if (fp64) leg_table_kernel<<<(unsigned)(mmax / 32 + 1), 32>>>(lmax, mmax, p->leg);
         if (scalar) leg32_coef_kernel<<<(unsigned)(mmax + 1), 256>>>(lmax, p->blk_ofs, p->leg32);
         if (cudaGetLastError() != cudaSuccess) rc = fail(HB_ERR_CUDA, "hb_plan_create: table kernel launch");
     }

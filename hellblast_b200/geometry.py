@@ -100,13 +100,20 @@ def get_plan(pid: int) -> Plan:
     return _plans[pid]
 
 
+def scalar_plan(pid: int, precision: int) -> Plan:
+    """Plan ``pid`` for a scalar transform: FP64 calls on a plan without the FP64 tables take the FP64 plan of the same
+    geometry, lmax and mmax."""
+    p = get_plan(pid)
+    return plan(p.geom, p.lmax, p.mmax) if precision == 64 and p.flags & L.HB_PLAN_NO_FP64 else p
+
+
 def plan(geom: Geometry, lmax: int, mmax: int | None = None, precision: int = 64, spin: bool = False) -> Plan:
     """Cached plan for (geometry, lmax, mmax); FP32 plans carry the checkpoint tables (scalar, or
-    spin-2 with ``spin=True``)."""
+    spin-2 with ``spin=True``), FP64 plans the scalar recursion's tables."""
     mmax = lmax if mmax is None else mmax
     flags = 0
     if precision == 32:
-        flags = L.HB_PLAN_SPIN2_FP32 if spin else L.HB_PLAN_FP32
+        flags = (L.HB_PLAN_SPIN2_FP32 if spin else L.HB_PLAN_FP32) | L.HB_PLAN_NO_FP64
     key = ("plan", geom.gid, int(lmax), int(mmax), flags)
     with _lock:
         p = _cache.get(key)

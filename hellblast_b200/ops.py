@@ -94,7 +94,7 @@ def call(op, *args):
 
 def _map2alm(maps: torch.Tensor, pid: int, weights: Optional[torch.Tensor], flags: int) -> torch.Tensor:
     _check_cuda(maps, weights)
-    p = G.get_plan(pid)
+    p = G.scalar_plan(pid, _prec(maps.dtype))
     maps = maps.contiguous()
     nmaps, prec = maps.shape[0], _prec(maps.dtype)
     out = torch.empty(nmaps, alm_size(p.lmax, p.mmax), dtype=_ctype(prec), device=maps.device)
@@ -115,7 +115,7 @@ def _(maps, pid, weights, flags):
 
 def _alm2map(alm: torch.Tensor, pid: int, flags: int) -> torch.Tensor:
     _check_cuda(alm)
-    p = G.get_plan(pid)
+    p = G.scalar_plan(pid, _prec(alm.dtype))
     alm = alm.contiguous()
     nmaps, prec = alm.shape[0], _prec(alm.dtype)
     out = torch.empty(nmaps, p.npix, dtype=_rtype(prec), device=alm.device)
@@ -135,7 +135,7 @@ def _(alm, pid, flags):
 
 def _alm2map_adjoint(maps: torch.Tensor, pid: int, flags: int) -> torch.Tensor:
     _check_cuda(maps)
-    p = G.get_plan(pid)
+    p = G.scalar_plan(pid, _prec(maps.dtype))
     maps = maps.contiguous()
     nmaps, prec = maps.shape[0], _prec(maps.dtype)
     out = torch.empty(nmaps, alm_size(p.lmax, p.mmax), dtype=_ctype(prec), device=maps.device)
@@ -156,7 +156,7 @@ def _(maps, pid, flags):
 
 def _map2alm_adjoint(alm: torch.Tensor, pid: int, weights: Optional[torch.Tensor], flags: int) -> torch.Tensor:
     _check_cuda(alm, weights)
-    p = G.get_plan(pid)
+    p = G.scalar_plan(pid, _prec(alm.dtype))
     alm = alm.contiguous()
     nmaps, prec = alm.shape[0], _prec(alm.dtype)
     out = torch.empty(nmaps, p.npix, dtype=_rtype(prec), device=alm.device)

@@ -105,12 +105,14 @@ HB_API int hb_geom_fft_launches(const hb_geom *g, int precision, int *n);
 
 /* Transform plans: a geometry plus (lmax, mmax) plus the FP64-computed checkpoints that
  * re-anchor the FP32 Legendre recursions every 256 l (FP32 transforms need them to stay within
- * 1e-5 of FP64 at lmax ~ 4000; FP64 transforms do not use them).  Creating a plan allocates
- * (about 16 bytes per (m, 256-block of l, ring pair) per table) and runs one FP64 pass; plans
- * are immutable afterwards and may be shared across threads and streams.  The geometry must
+ * 1e-5 of FP64 at lmax ~ 4000; FP64 transforms do not use them), and the coefficient tables of
+ * the FP64 scalar recursions.  Creating a plan allocates (about 16 bytes per (m, 256-block of l,
+ * ring pair) per FP32 table, 48 bytes per (l, m) for FP64) and runs one FP64 pass.
+ * HB_PLAN_NO_FP64 leaves the FP64 tables out: Legendre stages and scalar transforms in FP64 then
+ * return HB_ERR_INVALID (ring stages and spin-2 do not need them).  Plans are immutable afterwards and may be shared across threads and streams.  The geometry must
  * outlive the plan. */
 typedef struct hb_plan hb_plan;
-enum { HB_PLAN_FP32 = 1, HB_PLAN_SPIN2_FP32 = 2 };
+enum { HB_PLAN_FP32 = 1, HB_PLAN_SPIN2_FP32 = 2, HB_PLAN_NO_FP64 = 4 };
 HB_API int hb_plan_create(const hb_geom *g, int lmax, int mmax, int flags, hb_plan **out);
 HB_API int hb_plan_destroy(hb_plan *p);
 HB_API size_t hb_plan_bytes(const hb_plan *p);

@@ -233,3 +233,32 @@ def test_fp32_pair_accuracy_at_full_size(hb, nside):
     err_map = float(torch.linalg.norm(m32.double() - m64) / torch.linalg.norm(m64))
     err_alm = float(torch.linalg.norm(b32.to(torch.complex128) - b64) / torch.linalg.norm(b64))
     assert err_map < TOL32 and err_alm < TOL32, (err_map, err_alm)
+
+
+def test_plan_tables_follow_their_use(hb):
+    """FP32 plans hold no FP64 tables (48 bytes per two (l, m)-rows: 12 doubles); FP64 data through the operators takes the
+    FP64 plan then, a C call at precision 64 is refused; a plan made without the flag serves both."""
+    from hellblast_b200 import _lib as L
+    from hellblast_b200 import geometry as G
+    from hellblast_b200 import ops
+    nside, lmax, mmax = 16, 45, 40
+    g = G.healpix(nside)
+    tables = sum(((lmax - m) // 2 + 1) * 96 for m in range(mmax + 1))
+    p32, p64, both = G.plan(g, lmax, mmax, precision=32), G.plan(g, lmax, mmax), G.Plan(g, lmax, mmax, L.HB_PLAN_FP32)
+    assert 0 <= both.nbytes - p32.nbytes - tables < 256 and p64.nbytes >= tables
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    m = torch.randn(2, g.npix, dtype=torch.float64, device="cuda", generator=gen)
+    a = ops.map2alm(m, p64.pid, None, 0)
+    st = torch.cuda.current_stream().cuda_stream
+    for pid in (p32.pid, both.pid):
+        assert torch.equal(ops.map2alm(m, pid, None, 0), a)
+        assert torch.equal(ops.alm2map(a, pid, 0), ops.alm2map(a, p64.pid, 0))
+        assert torch.equal(ops.alm2map_adjoint(m, pid, 0), ops.alm2map_adjoint(m, p64.pid, 0))
+        assert torch.equal(ops.map2alm_adjoint(a, pid, None, 0), ops.map2alm_adjoint(a, p64.pid, None, 0))
+    F = torch.zeros(2, mmax + 1, g.npairs, 2, dtype=torch.complex128, device="cuda")
+    L.call("hb_ring_analysis", p32.handle, 64, 2, m.data_ptr(), None, F.data_ptr(), 0, st)
+    out = torch.zeros_like(a)
+    with pytest.raises(ValueError, match="NO_FP64"):
+        L.call("hb_legendre_analysis", p32.handle, 64, 2, F.data_ptr(), out.data_ptr(), st)
+    L.call("hb_legendre_analysis", both.handle, 64, 2, F.data_ptr(), out.data_ptr(), st)
+    assert torch.equal(out, a)

@@ -44,7 +44,7 @@ struct TcGroup {
     const int64_t *blk_ofs;
     const float4 *ckh;       // checkpoints at l0 + 128 of every block (same indexing as ck)
     const float4 *ckq1, *ckq3;  // ... at l0 + 64 and l0 + 192 (analysis l-quarters)
-    const float2 *coef;      // recursion coefficients (A_l, B_l): [(blk_ofs[m] + b) * 256 + i], l = m + 256 b + i
+    const float2 *coef;      // the plan's (A_l, B_l): [(blk_ofs[m] + b) * 256 + i], l = m + 256 b + i
     // synthesis
     const uint4 *alm_tiles;  // [chunk][K-step half][4][N x 16] 16-bit, chunk = tile_ofs[m] + c
     const int64_t *alm_tile_ofs;
@@ -379,25 +379,6 @@ __device__ __forceinline__ void gen16(Rec &R, const float2 *cf, float (&ev)[8], 
             if (t & 1) R.check();
         }
     }
-}
-
-__device__ __forceinline__ void coef_scalar(int l, int m, int lmax, float2 &out) {
-    double A = 0.0, B = 0.0;
-    if (l == m) {
-        B = 1.0;
-    } else if (l <= lmax) {
-        const double ll = l, mm = m;
-        A = sqrt((4.0 * ll * ll - 1.0) / ((ll - mm) * (ll + mm)));
-        B = (l - 1 > m) ? -A * sqrt(((ll - 1.0 - mm) * (ll - 1.0 + mm)) / (4.0 * (ll - 1.0) * (ll - 1.0) - 1.0)) : 0.0;
-    }
-    out = make_float2((float)A, (float)B);
-}
-
-// (A_l, B_l) of every (m, l), in the plan's 256-l block layout, zero past lmax; one CTA per m.
-__global__ void coef_table_kernel(int lmax, const int64_t *__restrict__ blk_ofs, float2 *__restrict__ tab) {
-    const int m = blockIdx.x;
-    const int64_t b0 = blk_ofs[m], nb = blk_ofs[m + 1] - b0;
-    for (int64_t i = threadIdx.x; i < nb * 256; i += blockDim.x) coef_scalar(m + (int)i, m, lmax, tab[b0 * 256 + i]);
 }
 
 // Evanescent skip ranges.  Below its turning point the plan's checkpoint state of a ring pair
@@ -1122,7 +1103,6 @@ struct hb_batched_plan {
         float2 *GF;
         int64_t gf_stride, ff_stride;
         int64_t *tile_ofs;            // device [mmax+1] alm chunk offsets
-        float2 *coef;                 // recursion coefficient table (coef_table_kernel)
         float4 *ckh;                  // mid-block recursion checkpoints (launch_ck_mid)
         float4 *ckq1, *ckq3;          // quarter-block checkpoints (l0 + 64, l0 + 192)
     };
@@ -1233,7 +1213,7 @@ int hb_batched_plan_create(const hb_plan *const *plans, const int *nmaps, int np
     // sizes and layout of the single allocation
     size_t total = 0;
     auto carve = [&](size_t b) { size_t o = total; total += (b + 255) & ~(size_t)255; return o; };
-    struct Off { size_t gf, tofs, tiles_a, tiles_g, scales, coef, ckh, ckq1, ckq3; };
+    struct Off { size_t gf, tofs, tiles_a, tiles_g, scales, ckh, ckq1, ckq3; };
     std::vector<Off> offs(nplans);
     std::vector<std::vector<int64_t>> tile_ofs(nplans);
     std::vector<int64_t> chunks_a(nplans);
@@ -1254,7 +1234,6 @@ int hb_batched_plan_create(const hb_plan *const *plans, const int *nmaps, int np
         offs[i].scales = carve((size_t)ng * 4 * (p->mmax + 1) * (N / 2));
         int64_t nblocks = 0;  // 256-l blocks over all m, the plan's checkpoint layout
         for (int m = 0; m <= p->mmax; ++m) nblocks += (p->lmax - m) / 256 + 1;
-        offs[i].coef = carve((size_t)nblocks * 256 * sizeof(float2));
         offs[i].ckh = carve((size_t)nblocks * np * sizeof(float4));
         offs[i].ckq1 = carve((size_t)nblocks * np * sizeof(float4));
         offs[i].ckq3 = carve((size_t)nblocks * np * sizeof(float4));
@@ -1319,7 +1298,6 @@ int hb_batched_plan_create(const hb_plan *const *plans, const int *nmaps, int np
         part.gf_stride = fg_rows(part.p->mmax, false) * part.p->g->d.npairs * 2;
         part.ff_stride = fg_rows(part.p->mmax, true) * part.p->g->d.npairs * 2;
         part.tile_ofs = (int64_t *)(base + offs[i].tofs);
-        part.coef = (float2 *)(base + offs[i].coef);
         part.ckh = (float4 *)(base + offs[i].ckh);
         part.ckq1 = (float4 *)(base + offs[i].ckq1);
         part.ckq3 = (float4 *)(base + offs[i].ckq3);
@@ -1333,7 +1311,7 @@ int hb_batched_plan_create(const hb_plan *const *plans, const int *nmaps, int np
                 TcGroup &G = bp->hgroups[gi];
                 G.alm_tiles = (const uint4 *)(base + offs[i].tiles_a) + (size_t)k * chunks_a[i] * 16 * N;
                 G.alm_tile_ofs = bp->parts[i].tile_ofs;
-                G.coef = bp->parts[i].coef;
+                G.coef = p->leg32;
                 G.ckh = bp->parts[i].ckh;
                 G.ckq1 = bp->parts[i].ckq1;
                 G.ckq3 = bp->parts[i].ckq3;
@@ -1356,14 +1334,13 @@ int hb_batched_plan_create(const hb_plan *const *plans, const int *nmaps, int np
         (cudaMemcpy(bp->dgroups, bp->hgroups.data(), sizeof(TcGroup) * ngroups, cudaMemcpyHostToDevice) != cudaSuccess ||
          cudaMemset(bp->err, 0, sizeof(int)) != cudaSuccess))
         rc = fail(HB_ERR_CUDA, "hb_batched_plan_create: upload");
-    // recursion coefficient and mid-block tables, then the evanescent skip counts of every plan
+    // mid-block tables, then the evanescent skip counts of every plan
     std::vector<std::vector<int>> syn_skip(nplans), ana_skip(nplans);
     for (int i = 0; i < nplans && rc == HB_OK; ++i) {
         const hb_plan *p = plans[i];
-        coef_table_kernel<<<p->mmax + 1, 256>>>(p->lmax, p->blk_ofs, bp->parts[i].coef);
-        if (cudaGetLastError() != cudaSuccess || launch_ck_mid(p, bp->parts[i].ckh, bp->parts[i].ckq1, bp->parts[i].ckq3) != HB_OK ||
+        if (launch_ck_mid(p, bp->parts[i].ckh, bp->parts[i].ckq1, bp->parts[i].ckq3) != HB_OK ||
             cudaDeviceSynchronize() != cudaSuccess) {
-            rc = fail(HB_ERR_CUDA, "hb_batched_plan_create: coefficient table");
+            rc = fail(HB_ERR_CUDA, "hb_batched_plan_create: checkpoint tables");
             break;
         }
         const int64_t np = p->g->d.npairs, npb = (np + 127) / 128;

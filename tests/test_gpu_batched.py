@@ -175,3 +175,16 @@ def test_bounded_wait_expires_and_context_stays_usable(hb):
     torch.cuda.synchronize()
     assert bp.status() == 0
     assert rel(m, hb.hp_compat.alm2map(a.to(torch.complex128), nside, lmax=lmax)) < TOL
+
+
+def test_plan_shares_the_coefficient_table(hb):
+    """A batched plan reads (A_l, B_l) in the FP32 plan: its own memory is the ring coefficients, both operands' tiles and
+    scales, three checkpoint tables and the unit lists, no second table of 2 KB per 256-l block."""
+    nside, lmax, n = 4, 1023, 2
+    bp = hb.batched.BatchedPlan([(hb.geometry.healpix(nside), lmax, lmax, n)])
+    N = bp.executed_mma_flop()["mma_n"]
+    np_, rows = 2 * nside, lmax + 1
+    blocks = sum((lmax - m) // 256 + 1 for m in range(rows))
+    chunks = sum((lmax - m + 64) // 64 for m in range(rows))
+    need = n * rows * np_ * 16 + chunks * 256 * N + rows * 256 * N + rows * 4 * (N // 2) + 3 * blocks * np_ * 16 + 16 * (rows + blocks) + 8 * rows
+    assert need < bp.nbytes < need + 256 * 2048 < need + blocks * 2048

@@ -364,7 +364,7 @@ def run_msharded(args):
     alm_h = torch.stack([hb.synalm(cl, lmax=lmax, seed=i, device="cpu", dtype=torch.complex64) for i in range(B)])
     alm = alm_h.to(dev)
     ms = D.MShardedSHT(nside, lmax, precision=32)
-    n_fft = ms.lg.fft_launches(32) if ms.lg is not None else 0
+    n_fft = ms.lg.fft_launches(32, B) if ms.lg is not None else 0
 
     def step(a):
         return ms.map2alm(ms.alm2map(a))
@@ -487,7 +487,7 @@ def main():
 
     if args.mode == "plain":
         plan = G.plan(g, lmax, mmax, precision=32)
-        n_launch = 2 + 2 * g.fft_launches(32)
+        n_launch = 2 + 2 * g.fft_launches(32, B)
         ws = torch.empty(plan.workspace_bytes(32, B), dtype=torch.uint8, device=dev)
 
         def step(ev=None):
@@ -534,7 +534,7 @@ def main():
             keys = stage_acc[0].keys()
             return {k: float(np.mean([s[k] for s in stage_acc])) for k in keys}
         groups = (B + (63 if wide else 31)) // (64 if wide else 32)
-        n_launch = 2 * groups + 2 + 2 * g.fft_launches(32)  # operand preps, tensor kernels, ring FFT classes
+        n_launch = 2 * groups + 2 + 2 * g.fft_launches(32, B)  # operand preps, tensor kernels, ring FFT classes
 
         def make_ev():
             return True

@@ -472,13 +472,15 @@ int hb_geom_info(const hb_geom *g, int64_t *nr, int64_t *npix, int64_t *npairs, 
     return HB_OK;
 }
 
-int hb_geom_fft_launches(const hb_geom *g, int precision, int *n) {
-    if (!g || !n || (precision != 32 && precision != 64))
+int hb_geom_fft_launches(const hb_geom *g, int precision, int *n) { return hb_geom_fft_launches_n(g, precision, 1, n); }
+
+int hb_geom_fft_launches_n(const hb_geom *g, int precision, int nmaps, int *n) {
+    if (!g || !n || nmaps < 1 || (precision != 32 && precision != 64))
         return fail(HB_ERR_INVALID, "hb_geom_fft_launches: bad arguments");
     const GeomDev &d = g->d;
     const int ncls = precision == 32 ? d.rest_n_cls : d.n_cls;
     const int nm = precision == 32 ? merged_classes(ncls, d.rest_L, d.rest_first) : merged_classes(ncls, d.cls_L, d.cls_first);
-    *n = (precision == 32 ? pk_launches(d, 1) : 0) + ncls - (nm > 1 ? nm - 1 : 0);
+    *n = (precision == 32 ? pk_launches(d, nmaps) : 0) + ncls - (nm > 1 ? nm - 1 : 0);
     return HB_OK;
 }
 

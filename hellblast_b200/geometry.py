@@ -41,10 +41,11 @@ class Geometry:
             _next_id[0] += 1
             _registry[self.gid] = self
 
-    def fft_launches(self, precision: int = 32) -> int:
-        """Ring-FFT kernel launches per direction for one map (short length classes share launches)."""
+    def fft_launches(self, precision: int = 32, nmaps: int = 1) -> int:
+        """Ring-FFT kernel launches per direction for a call on ``nmaps`` maps (on few maps the short length classes
+        share launches)."""
         n = ctypes.c_int(0)
-        L.call("hb_geom_fft_launches", self.handle, int(precision), ctypes.byref(n))
+        L.call("hb_geom_fft_launches_n", self.handle, int(precision), int(nmaps), ctypes.byref(n))
         return n.value
 
     def __del__(self):  # pragma: no cover - interpreter shutdown order

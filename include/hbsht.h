@@ -102,6 +102,8 @@ HB_API int hb_geom_info(const hb_geom *g, int64_t *nr, int64_t *npix, int64_t *n
  * each; large batches make one per class; no reference counterpart: its FFT is one cuFFT call
  * per ring, sht_raw.py:38-43). */
 HB_API int hb_geom_fft_launches(const hb_geom *g, int precision, int *n);
+/* The same for a call on nmaps maps. */
+HB_API int hb_geom_fft_launches_n(const hb_geom *g, int precision, int nmaps, int *n);
 
 /* Transform plans: a geometry plus (lmax, mmax) plus the FP64-computed checkpoints that
  * re-anchor the FP32 Legendre recursions every 256 l (FP32 transforms need them to stay within

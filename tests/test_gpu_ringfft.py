@@ -176,3 +176,22 @@ def test_fp64_one_map_matches_many(hb, nside, lmax):
         L.call("hb_ring_analysis", p.handle, 64, n, maps[many].data_ptr(), None, F[n].data_ptr(), 0, st)
     assert rel2(maps[1][0].cpu().numpy(), maps[many][0].cpu().numpy()) < 1e-13
     assert rel2(F[1][0].cpu().numpy(), F[many][0].cpu().numpy()) < 1e-13
+
+
+@pytest.mark.parametrize("nside,nmaps,prec", [(64, 1, 32), (256, 3, 32), (256, 300, 32), (128, 2, 64), (512, 40, 32)])
+def test_fft_launches_counts_the_call(hb, nside, nmaps, prec):
+    """Geometry.fft_launches is the number of ring kernels a call on that many maps makes."""
+    from hellblast_b200 import _lib as L
+    from hellblast_b200 import geometry as G
+    g = G.healpix(nside)
+    p = G.plan(g, 20, precision=64)
+    Gm = torch.zeros(nmaps, 21, g.npairs, 2, dtype=torch.complex64 if prec == 32 else torch.complex128, device="cuda")
+    out = torch.empty(nmaps, g.npix, dtype=torch.float32 if prec == 32 else torch.float64, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    L.call("hb_ring_synthesis", p.handle, prec, nmaps, Gm.data_ptr(), out.data_ptr(), 0, st)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        L.call("hb_ring_synthesis", p.handle, prec, nmaps, Gm.data_ptr(), out.data_ptr(), 0, st)
+        torch.cuda.synchronize()
+    seen = sum(e.count for e in prof.key_averages() if "synthesis" in e.key)
+    assert seen == g.fft_launches(prec, nmaps)

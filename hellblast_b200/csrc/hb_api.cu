@@ -174,9 +174,9 @@ __global__ void __launch_bounds__(32 * CL_WARPS) alm2cl_kernel(int lmax, int mma
     }
 }
 
-// Warps per CTA.  Few CTAs: all that find work, since a warp waits on its chain of loads.  CTAs that fill the GPU: 8, as
-// a CTA's start and the sum over its warps cost more than they give; in between 16, longer for complex128, whose
-// loads are twice the bytes.  us with 8 / 16 / 32 warps, complex64 auto spectra: 1 alm of lmax 2047 (64 CTAs) 25.2 /
+// Warps per CTA.  Up to one CTA per SM (148): all that find work, since a warp waits on its chain of loads.  CTAs that
+// fill the GPU: 8, as a CTA's start and the sum over its warps cost more than they give; in between 16, longer for
+// complex128, whose loads are twice the bytes.  us with 8 / 16 / 32 warps, complex64 auto spectra: 1 alm of lmax 2047 (64 CTAs) 25.2 /
 // 18.6 / 14.8, 8 (512 CTAs) 44.5 / 40.7 / 41.4, 64 (4096) 191 / 208 / 246; lmax 300, 8 alm 6.4 / 5.8 / 6.4, 64 (640)
 // 10.4 / 12.2 / 15.3, 512 46 / 62 / 96; lmax 60, 5000 alm 29 / 58 / 139, lmax 10, 5000 alm 15 / 25 / 47 (4 warps 10).
 // complex128: lmax 400, 64 alm crossed (832 CTAs) 36.5 / 32.9 / 32.9, lmax 1300, 16 crossed (656) 83 / 79 / 72.

@@ -8,15 +8,16 @@
 //
 // Synthesis (alm -> G_N/S(m) per ring pair), work unit = (group, m, block of 128 ring pairs):
 //   D_q[pair, n] = sum_{l = m+q mod 2} lambda_l(x_pair) a_l[n],   q = parity of l-m,
-//   MMA M = 128 pairs, N = 2 * maps (Re/Im columns), K = l (32 per parity per stage).
-//   Four producer warps run the recursion (one pair per thread) and write the A tiles (K-major);
-//   a loader warp streams pre-split alm tiles with bulk copies; one thread issues the MMAs.
+//   MMA M = 128 pairs, N = 2 * maps (Re/Im columns), K = l (16 per parity per stage).
+//   Three groups of four producer warps run the recursion (one pair per thread, 128 l at a time from
+//   a checkpoint) and write the A tiles (K-major); a loader warp streams pre-split alm tiles with
+//   bulk copies; one thread issues the MMAs.
 //   Epilogue: G_N = D_0 + D_1, G_S = D_0 - D_1.
 // Analysis (F -> alm), work unit = (group, m, block of 256 consecutive l):
 //   D_q[l, n] = sum_pairs lambda_l(x_pair) (E|O)_pair[n],  E = F_N + F_S, O = F_N - F_S,
-//   MMA M = 128 l of one parity, N = 2 * maps, K = ring pairs (32 per stage).  The recursion
-//   restarts at the block from the plan's FP64-computed checkpoint; three producer warps each
-//   own one pipeline stage (one pair per thread, 256 steps) and write MN-major A tiles.
+//   MMA M = 128 l of one parity, N = 2 * maps, K = ring pairs (16 per stage).  The recursion
+//   restarts from FP64-computed checkpoints every 64 l; twelve producer warps, two per pipeline
+//   stage (one pair and quarter of the block per thread), write MN-major A tiles.
 //
 // Every mbarrier wait is bounded (ctl.wait_ns, 2 s unless a plan sets it); on expiry the kernel records an error code in
 // *err and returns after releasing its tensor memory.

@@ -27,10 +27,6 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-// halves whose exponent is negative become zero
-__device__ __forceinline__ f32x2 live_mask(int e0, int e1) {
-    return (e0 < 0 ? 0ull : 0xffffffffull) | (e1 < 0 ? 0ull : 0xffffffff00000000ull);
-}
 // OR of bit patterns, and whether any of the ORed values can be past 2^32 in magnitude (no false
 // negatives: the OR's exponent field is at least every value's)
 __device__ __forceinline__ unsigned bits_or(unsigned acc, f32x2 v) { return acc | (unsigned)v | (unsigned)(v >> 32); }

@@ -767,7 +767,7 @@ static int ctas_by_smem(size_t bytes) { return (int)((size_t)smem_per_sm() / (by
 // Number of leading classes (ascending L) that share one launch (see the file comment); all of them
 // when their pairs are under two per SM
 int merged_classes(int ncls, const int *L, const int64_t *first) {
-    if (ncls > 0 && first[ncls] <= 2 * 148) return ncls;
+    if (ncls > 0 && first[ncls] <= 2 * sm_count()) return ncls;
     int n = 0;
     while (n < ncls && L[n] <= 1024) ++n;
     return n;

@@ -33,6 +33,16 @@ __device__ __forceinline__ unsigned bits_or(unsigned acc, f32x2 v) { return acc 
 __device__ __forceinline__ bool maybe_big(unsigned acc) { return (acc & 0x7f800000u) >= 0x4f800000u; }
 constexpr float F32_UP = 4294967296.0f;                 // 2^32: a state past this moves to the next exponent
 constexpr float F32_DOWN = 5.42101086242752217e-20f;    // 2^-64: one exponent step
+// (north, south) coefficients of a ring pair, as two 8-byte accesses: F and G are the caller's, complex64, and need
+// no more alignment than that
+__device__ __forceinline__ float4 load_ns(const float2 *p) {
+    const float2 n = p[0], s = p[1];
+    return make_float4(n.x, n.y, s.x, s.y);
+}
+__device__ __forceinline__ void put_ns(float2 *p, float nr, float ni, float sr, float si) {
+    p[0] = make_float2(nr, ni);
+    p[1] = make_float2(sr, si);
+}
 // factor that takes sums in units of 2^(64 e0) to units of 2^(64 e1).  Exponents rise from block to block, but for a
 // first block's e1 < 0 against the 0 of empty sums: one step up is then as good as any, and stays finite.
 __device__ __forceinline__ float sums_to_unit(int e0, int e1) {

@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(NT, MINB) leg_analysis32_kernel(GeomDev g, int
 #pragma unroll
                 for (int b = 0; b < NB; ++b) {
                     float4 f = make_float4(0.f, 0.f, 0.f, 0.f);  // (north, south)
-                    if (p < np) f = *reinterpret_cast<const float4 *>(F + b * fm_stride + 2 * p);
+                    if (p < np) f = load_ns(F + b * fm_stride + 2 * p);
                     fw[((u + i) * NB + b) * NT] = f;
                     set_weights(S, u + i, b, S.e[u + i] < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : f);
                 }
@@ -430,8 +430,7 @@ __global__ void __launch_bounds__(32, MINB) leg_synthesis32_kernel(GeomDev g, in
                 if (p >= np) continue;
                 const float f = S.e[u][h] == 0 ? 1.f : ldexpf(1.f, 64 * S.e[u][h]);
                 float2 *G = Gm + ((int64_t)blockIdx.z * NB + i) * gm_stride + ((int64_t)blockIdx.y * np + p) * 2;
-                *reinterpret_cast<float4 *>(G) = make_float4((er[h] + qr[h]) * f, (ei[h] + qi[h]) * f, (er[h] - qr[h]) * f,
-                                                             (ei[h] - qi[h]) * f);
+                put_ns(G, (er[h] + qr[h]) * f, (ei[h] + qi[h]) * f, (er[h] - qr[h]) * f, (ei[h] - qi[h]) * f);
             }
         }
 }

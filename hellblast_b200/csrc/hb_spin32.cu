@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(NT, MINB) spin_analysis32_kernel(GeomDev g, in
                 neg |= (s.ep < 0) | (s.em < 0);
                 float4 q = make_float4(0.f, 0.f, 0.f, 0.f), u = q;
                 if (p < np) {
-                    q = *reinterpret_cast<const float4 *>(Qf + 2 * p);
-                    u = *reinterpret_cast<const float4 *>(Uf + 2 * p);
+                    q = load_ns(Qf + 2 * p);
+                    u = load_ns(Uf + 2 * p);
                 }
                 fw[(2 * k) * NT] = q;
                 fw[(2 * k + 1) * NT] = u;
@@ -426,9 +426,9 @@ __global__ void __launch_bounds__(32, MINB) spin_synthesis32_kernel(GeomDev g, i
         parts(S.si, true, si);
         const int64_t o = b * gm_stride + ((int64_t)m * np + p) * 2;
         const float h = -0.5f;
-        *reinterpret_cast<float4 *>(QG + o) = make_float4(h * nr.x, h * ni.x, h * sr.x, h * si.x);
+        put_ns(QG + o, h * nr.x, h * ni.x, h * sr.x, h * si.x);
         // -i/2 z = (z.im, -z.re) / 2
-        *reinterpret_cast<float4 *>(UG + o) = make_float4(-h * ni.y, h * nr.y, -h * si.y, h * sr.y);
+        put_ns(UG + o, -h * ni.y, h * nr.y, -h * si.y, h * sr.y);
     }
 }
 

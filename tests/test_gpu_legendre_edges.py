@@ -306,3 +306,28 @@ def test_fp32_analysis_pair_counts(hb, npairs):
             F = torch.zeros_like(full[:1])
             F[:, :, p] = full[:1, :, p]
             assert torch.equal(analysis(th, F), analysis(th[[p, nrings - 1 - p]], full[:1, :, p:p + 1].contiguous())), p
+
+
+@pytest.mark.parametrize("nside,lmax,nmaps", [(16, 40, 1), (64, 130, 2), (512, 300, 2), (1024, 270, 1)])
+def test_stage_buffers_at_8_bytes(hb, nside, lmax, nmaps):
+    """F and G of the FP32 Legendre stages are complex64 and may start at any multiple of 8 bytes."""
+    from hellblast_b200 import _lib as L
+    from hellblast_b200 import geometry as G
+    g = G.healpix(nside)
+    p = G.plan(g, lmax, precision=32)
+    st = torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device="cuda").manual_seed(nside)
+    n = nmaps * (lmax + 1) * g.npairs * 2
+    F = torch.randn(n + 1, dtype=torch.complex64, device="cuda", generator=gen)
+    nalm = L.lib().hb_alm_size(lmax, lmax)
+    alm, out = [], []
+    for f in (F[1:], F[1:].clone()):
+        a = torch.empty(nmaps, nalm, dtype=torch.complex64, device="cuda")
+        L.call("hb_legendre_analysis", p.handle, 32, nmaps, f.data_ptr(), a.data_ptr(), st)
+        alm.append(a)
+    assert torch.equal(alm[0], alm[1])
+    for ofs in (1, 0):
+        buf = torch.zeros(n + 1, dtype=torch.complex64, device="cuda")
+        L.call("hb_legendre_synthesis", p.handle, 32, nmaps, alm[0].data_ptr(), buf[ofs:].data_ptr(), st)
+        out.append(buf[ofs:ofs + n])
+    assert torch.equal(out[0], out[1]) and out[0].abs().sum() > 0

@@ -220,7 +220,11 @@ __device__ __forceinline__ void dif_to_smem(c2_t<T> *buf, int logL, const Tw<T> 
     auto lds = [&](int p) -> V { return buf[ph(p)]; };
     auto sts = [&](int p, V v) { buf[ph(p)] = v; };
     const int P = fft_nstages(logL);
-    fft_stage<false, INV, T>(0, logL, tw, ld_in, sts);
+    if (P == 0) {  // length 1 (a ring of two pixels): the point itself
+        if (threadIdx.x == 0) sts(0, ld_in(0));
+    } else {
+        fft_stage<false, INV, T>(0, logL, tw, ld_in, sts);
+    }
     __syncthreads();
     for (int i = 1; i < P; ++i) {
         fft_stage<false, INV, T>(i, logL, tw, lds, sts);

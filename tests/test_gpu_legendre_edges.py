@@ -331,3 +331,15 @@ def test_stage_buffers_at_8_bytes(hb, nside, lmax, nmaps):
         L.call("hb_legendre_synthesis", p.handle, 32, nmaps, alm[0].data_ptr(), buf[ofs:].data_ptr(), st)
         out.append(buf[ofs:ofs + n])
     assert torch.equal(out[0], out[1]) and out[0].abs().sum() > 0
+
+
+@pytest.mark.parametrize("nphi,lmax", [([2], 3), ([2, 4, 2, 6, 2], 9), ([2, 2, 8, 2, 2, 2], 40)])
+def test_rings_of_two_pixels(hb, oracle, nphi, lmax):
+    """Two pixels are the smallest ring: its FFT has length one."""
+    nphi = np.array(nphi, dtype=np.int32)
+    th = np.linspace(0.3, 2.7, nphi.size)
+    w, phi0 = np.linspace(0.2, 0.4, nphi.size), np.linspace(0, 1, nphi.size)
+    g = oracle.generic_geometry(th, nphi, phi0=phi0, weights=w)
+    _pair(hb, oracle, g, lmax, lmax, 2,
+          lambda a, p: hb.transforms.alm2map(a, hb.geometry.generic(th, nphi, w, phi0), lmax, precision=p),
+          lambda m, p: hb.transforms.map2alm(m, hb.geometry.generic(th, nphi, w, phi0), lmax, precision=p), lmax)

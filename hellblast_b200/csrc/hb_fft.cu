@@ -729,7 +729,7 @@ int build_fft_tables(GeomDev &g, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------------------ launch
-static int max_smem_optin() {
+int max_smem_optin() {
     static int v = -1;
     if (v < 0) {
         int dev = 0;
@@ -842,7 +842,7 @@ static int launch_analysis_t(const GeomDev &g, int nmaps, const T *maps, int64_t
         const int ctas0 = ctas_by_smem(base_smem), ctas1 = ctas_by_smem(base_smem + stage_bytes);
         const bool stage_n = base_smem + stage_bytes <= (size_t)max_smem_optin() && ctas1 >= std::min(2, ctas0);
         const int smem = (int)(base_smem + (stage_n ? stage_bytes : 0));
-        HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin()));
         HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared));
         dim3 grid((unsigned)cnt, (unsigned)nmaps);
@@ -878,7 +878,7 @@ static int launch_synthesis_t(const GeomDev &g, int nmaps, const c2_t<T> *Gm, in
         const int64_t first = c < nmerge ? 0 : clsF[c], cnt = clsF[c + 1] - first;
         const bool stage_t = class_smem_syn<T>(L, mmax, true) <= (size_t)max_smem_optin();
         const int smem = (int)class_smem_syn<T>(L, mmax, stage_t), nt = class_threads(L);
-        HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin()));
         HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          cudaSharedmemCarveoutMaxShared));
         // asynchronous staging when the grid is under two waves of resident CTAs

@@ -216,6 +216,9 @@ int launch_spin_analysis(const hb_plan *p, int precision, int nmaps, const void 
                          cudaStream_t st);
 int launch_spin_synthesis(const hb_plan *p, int precision, int nmaps, const void *E, const void *B, void *QGm, void *UGm,
                           cudaStream_t st);
+// Largest dynamic shared memory of a CTA.  Kernels whose size depends on the call get this as their limit: the limit
+// is the kernel's, and one that followed each call would fail the launch of another thread with a larger size.
+int max_smem_optin();
 // leading ring-FFT classes (ascending L) that share one launch
 int merged_classes(int ncls, const int *L, const int64_t *first);
 // FFT twiddle table and Bluestein chirp spectra of a geometry

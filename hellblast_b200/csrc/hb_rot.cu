@@ -306,7 +306,8 @@ template <int MM, bool TAB>
 int run_rotate(int lmax, int nmaps, const double2 *in, double2 *out, double alpha, const BetaRed &br, double gamma, cudaStream_t st) {
     const size_t smem = rot_smem<MM, TAB>(lmax);
     const int chunks = lmax / ROT_NT + 1;
-    HB_CUDA_TRY(cudaFuncSetAttribute(rotate_alm_kernel<MM, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HB_CUDA_TRY(cudaFuncSetAttribute(rotate_alm_kernel<MM, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     std::max((int)smem, max_smem_optin())));
     if (chunks > 1) HB_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double2) * (size_t)alm_size(lmax, lmax) * nmaps, st));
     rotate_alm_kernel<MM, TAB><<<dim3((unsigned)(lmax / MM + 1), (unsigned)chunks, (unsigned)nmaps), ROT_NT, smem, st>>>(
         lmax, in, out, alpha, br.x, br.lc, br.ls, br.flip ? 1 : 0, gamma, chunks > 1 ? 1 : 0);

@@ -262,3 +262,36 @@ def test_plan_tables_follow_their_use(hb):
         L.call("hb_legendre_analysis", p32.handle, 64, 2, F.data_ptr(), out.data_ptr(), st)
     L.call("hb_legendre_analysis", both.handle, 64, 2, F.data_ptr(), out.data_ptr(), st)
     assert torch.equal(out, a)
+
+
+def test_calls_from_several_threads(hb):
+    """Threads with their own streams and sizes: every call runs and gives what it gives alone (rotations sum by atomics:
+    1e-12)."""
+    import threading
+    cfg = []
+    for i, (nside, lmax) in enumerate([(8, 20), (64, 150), (128, 380), (256, 500), (16, 47), (256, 90), (64, 60), (32, 95)]):
+        gen = torch.Generator(device="cuda").manual_seed(i)
+        m = torch.randn(1, 12 * nside * nside, dtype=torch.float64, device="cuda", generator=gen)
+        a = hb.hp_compat.map2alm(m, lmax=lmax)
+        cfg.append((nside, lmax, m, a, hb.hp_compat.alm2map(a, nside, lmax=lmax), hb.rotate.rotate_alm_euler(a, 0.1, 0.7, 0.3)))
+    torch.cuda.synchronize()
+    failures = []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for i in range(80):
+                    nside, lmax, m, a, back, rot = cfg[(k + 3 * i) % len(cfg)]
+                    got = hb.hp_compat.map2alm(m, lmax=lmax), hb.hp_compat.alm2map(a, nside, lmax=lmax), hb.rotate.rotate_alm_euler(a, 0.1, 0.7, 0.3)
+                    for x, y in zip(got, (a, back, rot)):
+                        if not (x - y).abs().max() <= 1e-12 * y.abs().max():
+                            failures.append((nside, lmax))
+        except Exception as e:
+            failures.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures

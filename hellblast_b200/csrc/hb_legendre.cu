@@ -478,8 +478,8 @@ template <int U, int NB, int MINB> static int run_synthesis(const LegArgs &L, in
 // one after the other (a fixed sum, no atomics), and the 3 or 4 CTAs of an SM fill each other's waits.  That
 // takes enough orders (in_turn) and each of them once, which a list of orders does not promise; else one
 // map's pairs run side by side, 16 warps a CTA.  In us, wide / in turn: nside 1024, one map, lmax 2047
-// 1836 / 1706, 1100 562 / 540, 900 378 / 401.  Two maps in pairs, 8 warps wide / in turn: lmax 2047 4295 / 3077,
-// 700 562 / 439, 500 291 / 280.
+// 1812 / 1680, 1100 553 / 534, 1000 456 / 459, 900 366 / 394.  Two maps, one by one wide / in pairs in turn: lmax 2047
+// 3613 / 3015, 700 468 / 415, 500 242 / 277 (in pairs wide, 8 warps: 4302, 560, 289).
 static bool in_turn(const LegArgs &L, int nb, int64_t nz) {
     return L.np() >= 1024 && !L.mlist && L.rows * nz >= (nb == 1 ? 1024 : 512);
 }

@@ -15,7 +15,7 @@
 // recursion, shared by the NB maps of a CTA).  Two ring pairs share each packed instruction, which
 // leaves half the issue slots to loads and reductions; blocks of 256 l in which a set of pairs stays
 // evanescent are skipped by the plan's flags (a quarter of the work at lmax = 2 nside).
-// One map at nside 1024, lmax 2047: synthesis 1636 -> 890 us (66 % FMA pipe), analysis 2000 -> 1320 us
+// One map at nside 1024, lmax 2047: synthesis 1636 -> 813 us (73 % FMA pipe), analysis 2000 -> 1320 us
 // (51 %; following the pairs that leave e < 0 within a block takes 160 us of it).  The arithmetic and the
 // order of every sum of the analysis are unchanged (same bits).
 #include <cmath>

@@ -372,7 +372,9 @@ template <> __device__ __forceinline__ void store_ns<double2>(double2 *dst, doub
     dst[1] = s;
 }
 
-template <typename T, int MINB>
+// VEC: the maps start at a multiple of two elements (ring offsets are even), and pixels 2p, 2p + 1 move as one vector;
+// other maps by single elements (FP32 162 instead of 160 us at nside 1024; a branch on it in one kernel 166).
+template <typename T, int MINB, bool VEC>
 __global__ void __launch_bounds__(256, MINB)
     ring_analysis_kernel(GeomDev g, const int32_t *__restrict__ pairs, const T *__restrict__ maps, int64_t map_stride,
                          const double *__restrict__ w, c2_t<T> *__restrict__ Fm, int64_t fm_stride, int mmax,
@@ -401,13 +403,14 @@ __global__ void __launch_bounds__(256, MINB)
         const bool direct = bo < 0;
         __syncthreads();  // previous ring done with buf / tables
         const RingTrig<T> R = trig_for_ring<T>(g, tab, pair, side, n, N, mmax);
-        const V *f2 = reinterpret_cast<const V *>(maps + b * map_stride + g.ofs[r]);  // ring offsets: multiples of 4
+        const T *f = maps + b * map_stride + g.ofs[r];
+        const auto f2 = [&](int p) -> V { return VEC ? reinterpret_cast<const V *>(f)[p] : mk2(f[2 * p], f[2 * p + 1]); };
         const V *ch = direct ? nullptr : chirp_table<T>(g, bo, L);
         if (direct) {  // DIF from the ring itself: the spectrum stays in digit order
-            dif_to_smem<false, T>(buf, logL, tw, [&](int p) -> V { return f2[p]; });
+            dif_to_smem<false, T>(buf, logL, tw, f2);
         } else {
             bluestein<T>(buf, logL, tw, blu_table<T>(g) + bo,
-                         [&](int p) -> V { return p < N ? cmul(f2[p], ch[p]) : mk2((T)0, (T)0); }, sts);
+                         [&](int p) -> V { return p < N ? cmul(f2(p), ch[p]) : mk2((T)0, (T)0); }, sts);
             __syncthreads();
         }
         // Z_k, 0 <= k < N
@@ -468,7 +471,7 @@ __global__ void __launch_bounds__(256, MINB)
 }
 
 // ------------------------------------------------------------------------------ synthesis
-template <typename T, int MINB>
+template <typename T, int MINB, bool VEC>
 __global__ void __launch_bounds__(256, MINB)
     ring_synthesis_kernel(GeomDev g, const int32_t *__restrict__ pairs, const c2_t<T> *__restrict__ Gm,
                           int64_t gm_stride, int mmax, T *__restrict__ maps, int64_t map_stride,
@@ -544,7 +547,15 @@ __global__ void __launch_bounds__(256, MINB)
             return mk2(S.x - u.x * D.y + u.y * D.x, S.y + u.x * D.x + u.y * D.y);  // S + i conj(u) D
         };
         const T pscale = apply_w ? (T)(((flags & HB_F_NO2PI) ? 1.0 : twopi) * w[r] / (double)n) : (T)1;
-        V *out2 = reinterpret_cast<V *>(maps + b * map_stride + g.ofs[r]);
+        T *f = maps + b * map_stride + g.ofs[r];
+        const auto store2 = [&](int p, V v) {
+            if (VEC) {
+                reinterpret_cast<V *>(f)[p] = v;
+            } else {
+                f[2 * p] = v.x;
+                f[2 * p + 1] = v.y;
+            }
+        };
         // the spectrum in natural order (its folds loop over aliases, so it gets a pass of its own
         // rather than sitting inside the unrolled first FFT pass); Bluestein: conj(Z_k) chirp_k.
         // One thread takes the bins k and N - k of the Hermitian half-spectrum,
@@ -596,10 +607,10 @@ __global__ void __launch_bounds__(256, MINB)
         auto lds = [&](int p) -> V { return buf[ph(p)]; };
         if (direct) {  // inverse DIF, then a digit-order read for the ring store
             dif_to_smem<true, T>(buf, logL, tw, lds);
-            for (int j = threadIdx.x; j < N; j += blockDim.x) out2[j] = cscale(buf[ph(pos_of_freq(j, logL))], pscale);
+            for (int j = threadIdx.x; j < N; j += blockDim.x) store2(j, cscale(buf[ph(pos_of_freq(j, logL))], pscale));
         } else {  // inverse DFT as conj(DFT(conj Z)) through the chirp-z convolution
             bluestein<T>(buf, logL, tw, blu_table<T>(g) + bo, lds, [&](int p, V v) {
-                if (p < N) out2[p] = cscale(cconj(cmul(v, ch[p])), pscale);
+                if (p < N) store2(p, cscale(cconj(cmul(v, ch[p])), pscale));
             });
         }
     }
@@ -789,18 +800,19 @@ template <typename T> static int min_ctas(int ncls, int nmerge, const int *L, co
         threads = std::max(threads, (first[c + 1] - (c < nmerge ? 0 : first[c])) * nmaps * class_threads(L[c]));
     return threads <= 256 * (int64_t)sm_count() ? 1 : 2;
 }
-template <typename T> static auto analysis_kernel(int minb) {
+template <typename T, bool VEC> static auto analysis_kernel(int minb) {
     if constexpr (sizeof(T) == 4)
-        return ring_analysis_kernel<T, 3>;
+        return ring_analysis_kernel<T, 3, VEC>;
     else
-        return minb == 1 ? ring_analysis_kernel<T, 1> : ring_analysis_kernel<T, 2>;
+        return minb == 1 ? ring_analysis_kernel<T, 1, VEC> : ring_analysis_kernel<T, 2, VEC>;
 }
-template <typename T> static auto synthesis_kernel(int minb) {
+template <typename T, bool VEC> static auto synthesis_kernel(int minb) {
     if constexpr (sizeof(T) == 4)
-        return ring_synthesis_kernel<T, 3>;
+        return ring_synthesis_kernel<T, 3, VEC>;
     else
-        return minb == 1 ? ring_synthesis_kernel<T, 1> : ring_synthesis_kernel<T, 2>;
+        return minb == 1 ? ring_synthesis_kernel<T, 1, VEC> : ring_synthesis_kernel<T, 2, VEC>;
 }
+template <typename T> static bool vec_maps(const T *maps) { return reinterpret_cast<uintptr_t>(maps) % (2 * sizeof(T)) == 0; }
 
 template <typename T>
 static int check_smem(const GeomDev &g, int mmax) {
@@ -833,7 +845,8 @@ static int launch_analysis_t(const GeomDev &g, int nmaps, const T *maps, int64_t
     const int64_t *clsF = f32 ? g.rest_first : g.cls_first;
     const int32_t *clsP = f32 ? g.rest_pairs : g.cls_pairs;
     const int nmerge = merged_classes(ncls, clsL, clsF);
-    const auto kernel = analysis_kernel<T>(min_ctas<T>(ncls, nmerge, clsL, clsF, nmaps));
+    const int minb = min_ctas<T>(ncls, nmerge, clsL, clsF, nmaps);
+    const auto kernel = vec_maps(maps) ? analysis_kernel<T, true>(minb) : analysis_kernel<T, false>(minb);
     for (int c = nmerge ? nmerge - 1 : 0; c < ncls; ++c) {
         const int L = clsL[c];
         const int64_t first = c < nmerge ? 0 : clsF[c], cnt = clsF[c + 1] - first;
@@ -872,7 +885,8 @@ static int launch_synthesis_t(const GeomDev &g, int nmaps, const c2_t<T> *Gm, in
     const int64_t *clsF = f32 ? g.rest_first : g.cls_first;
     const int32_t *clsP = f32 ? g.rest_pairs : g.cls_pairs;
     const int nmerge = merged_classes(ncls, clsL, clsF);
-    const auto kernel = synthesis_kernel<T>(min_ctas<T>(ncls, nmerge, clsL, clsF, nmaps));
+    const int minb = min_ctas<T>(ncls, nmerge, clsL, clsF, nmaps);
+    const auto kernel = vec_maps(maps) ? synthesis_kernel<T, true>(minb) : synthesis_kernel<T, false>(minb);
     for (int c = nmerge ? nmerge - 1 : 0; c < ncls; ++c) {
         const int L = clsL[c];
         const int64_t first = c < nmerge ? 0 : clsF[c], cnt = clsF[c + 1] - first;

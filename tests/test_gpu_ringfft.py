@@ -195,3 +195,39 @@ def test_fft_launches_counts_the_call(hb, nside, nmaps, prec):
         torch.cuda.synchronize()
     seen = sum(e.count for e in prof.key_averages() if "synthesis" in e.key)
     assert seen == g.fft_launches(prec, nmaps)
+
+
+@pytest.mark.parametrize("nside,lmax,nmaps", [(4, 9, 1), (64, 100, 2), (512, 300, 1), (1024, 100, 1)])
+@pytest.mark.parametrize("prec", [32, 64])
+def test_maps_at_any_element(hb, nside, lmax, nmaps, prec):
+    """A map may be a view that starts at an odd element of a larger buffer, in either direction."""
+    from hellblast_b200 import _lib as L
+    from hellblast_b200 import geometry as G
+    dt = torch.float32 if prec == 32 else torch.float64
+    gen = torch.Generator(device="cuda").manual_seed(nside)
+    npix = 12 * nside * nside
+    buf = torch.randn(nmaps * npix + 1, dtype=dt, device="cuda", generator=gen)
+    view = buf[1:].view(nmaps, npix)
+    a = hb.hp_compat.map2alm(view, lmax=lmax)
+    assert torch.equal(a, hb.hp_compat.map2alm(view.clone(), lmax=lmax))
+    if nside <= 64:  # (above 512 ring pairs the FP64 spin-2 analysis adds its chunks by atomics, in no fixed order)
+        q, w = (hb.hp_compat.map2alm_spin(x, x.flip(0), 2, lmax=lmax) for x in (view, view.clone()))
+        assert torch.equal(q[0], w[0]) and torch.equal(q[1], w[1])
+    p = G.plan(G.healpix(nside), lmax, precision=prec)
+    st = torch.cuda.current_stream().cuda_stream
+    Gm = torch.zeros(nmaps, lmax + 1, p.geom.npairs, 2, dtype=a.dtype, device="cuda")
+    L.call("hb_legendre_synthesis", p.handle, prec, nmaps, a.data_ptr(), Gm.data_ptr(), st)
+    out = torch.full_like(buf, float("nan"))
+    L.call("hb_ring_synthesis", p.handle, prec, nmaps, Gm.data_ptr(), out[1:].data_ptr(), 0, st)
+    assert torch.equal(out[1:].view(nmaps, npix), hb.hp_compat.alm2map(a, nside, lmax=lmax)) and torch.isnan(out[0])
+
+
+def test_batched_maps_at_any_element(hb):
+    nside, lmax, n = 64, 100, 3
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    buf = torch.randn(n * 12 * nside * nside + 1, device="cuda", generator=gen)
+    bp = hb.batched.plan(nside, lmax, n)
+    a = bp.map2alm(buf[1:])
+    assert torch.equal(a, bp.map2alm(buf[1:].clone()))
+    out = torch.empty_like(buf)
+    assert torch.equal(bp.alm2map(a, out=out[1:]), bp.alm2map(a))

@@ -835,7 +835,9 @@ static int launch_analysis_t(const GeomDev &g, int nmaps, const T *maps, int64_t
     const int64_t fm_stride = fg_rows(mmax, mblk) * g.npairs * 2;
     // FP32: the pair-packed kernels take the pairs they can (hb_ringpack.cu), this kernel the rest
     const bool f32 = sizeof(T) == 4;
+    const bool fvec = reinterpret_cast<uintptr_t>(Fm) % (2 * sizeof(*Fm)) == 0;  // (north, south) as one vector
     if (f32 && g.pk_n_cls > 0) {
+        if (!fvec) return fail(HB_ERR_INVALID, "ring analysis: F of this grid must start at a multiple of 16 bytes");
         rc = launch_pk_analysis(g, nmaps, reinterpret_cast<const float *>(maps), map_stride, w ? w : g.w,
                                 reinterpret_cast<float2 *>(Fm), mmax, flags, unit_w, mdouble, st, mblk);
         if (rc) return rc;
@@ -853,7 +855,8 @@ static int launch_analysis_t(const GeomDev &g, int nmaps, const T *maps, int64_t
         // stage the north ring's F(m) for joint (north, south) stores unless that costs CTAs per SM
         const size_t base_smem = class_smem<T>(L, mmax), stage_bytes = sizeof(c2_t<T>) * (size_t)(mmax + 1);
         const int ctas0 = ctas_by_smem(base_smem), ctas1 = ctas_by_smem(base_smem + stage_bytes);
-        const bool stage_n = base_smem + stage_bytes <= (size_t)max_smem_optin() && ctas1 >= std::min(2, ctas0);
+        const bool stage_n = base_smem + stage_bytes <= (size_t)max_smem_optin() && ctas1 >= std::min(2, ctas0) &&
+                             (fvec || !f32);
         const int smem = (int)(base_smem + (stage_n ? stage_bytes : 0));
         HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem_optin()));
         HB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -876,6 +879,8 @@ static int launch_synthesis_t(const GeomDev &g, int nmaps, const c2_t<T> *Gm, in
     // FP32: the pair-packed kernels take the pairs they can (hb_ringpack.cu), this kernel the rest
     const bool f32 = sizeof(T) == 4;
     if (f32 && g.pk_n_cls > 0) {
+        if (reinterpret_cast<uintptr_t>(Gm) % (2 * sizeof(*Gm)))
+            return fail(HB_ERR_INVALID, "ring synthesis: G of this grid must start at a multiple of 16 bytes");
         rc = launch_pk_synthesis(g, nmaps, reinterpret_cast<const float2 *>(Gm), mmax, reinterpret_cast<float *>(maps),
                                  map_stride, w ? w : g.w, apply_w, mdouble, flags, st);
         if (rc) return rc;

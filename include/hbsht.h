@@ -262,6 +262,9 @@ HB_API int hb_batched_stage_ms(hb_batched_plan *bp, float *ms);
 /* Pipeline stages (what the transforms are made of), for callers that keep the per-ring
  * Fourier coefficients resident or time the stages.  F / G: complex, precision 32 or 64,
  * layout [nmaps][mmax+1][npairs][2] (north, south ring of each pair), npairs from hb_geom_info.
+ * Buffers are aligned to their elements (maps to one real number, alm, F and G to one complex
+ * number), and F and G of the FP32 ring stages to 16 bytes: with rings of more than 256 pixels
+ * other ones are refused.
  *   hb_ring_analysis:      maps -> F (weights, phi0 phase, alias fold; flags as map2alm)
  *   hb_legendre_analysis:  F -> alm
  *   hb_legendre_synthesis: alm -> G

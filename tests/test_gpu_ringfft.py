@@ -231,3 +231,32 @@ def test_batched_maps_at_any_element(hb):
     assert torch.equal(a, bp.map2alm(buf[1:].clone()))
     out = torch.empty_like(buf)
     assert torch.equal(bp.alm2map(a, out=out[1:]), bp.alm2map(a))
+
+
+def test_stage_buffers_at_8_bytes(hb):
+    """F and G of the FP32 ring stages that start at an odd complex64: taken on grids of short rings, refused where the
+    pair-packed kernels read 16-byte pairs."""
+    from hellblast_b200 import _lib as L
+    from hellblast_b200 import geometry as G
+    st = torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    lmax = 40
+    for nside in (32, 256):
+        p = G.plan(G.healpix(nside), lmax, precision=32)
+        n = (lmax + 1) * p.geom.npairs * 2
+        m = torch.randn(1, p.npix, device="cuda", generator=gen)
+        F = torch.zeros(n + 1, dtype=torch.complex64, device="cuda")
+        want = torch.zeros(n, dtype=torch.complex64, device="cuda")
+        out, ref = torch.zeros_like(m), torch.zeros_like(m)
+        L.call("hb_ring_analysis", p.handle, 32, 1, m.data_ptr(), None, want.data_ptr(), 0, st)
+        L.call("hb_ring_synthesis", p.handle, 32, 1, want.data_ptr(), ref.data_ptr(), 0, st)
+        if nside == 256:
+            with pytest.raises(ValueError, match="16 bytes"):
+                L.call("hb_ring_analysis", p.handle, 32, 1, m.data_ptr(), None, F[1:].data_ptr(), 0, st)
+            with pytest.raises(ValueError, match="16 bytes"):
+                L.call("hb_ring_synthesis", p.handle, 32, 1, F[1:].data_ptr(), out.data_ptr(), 0, st)
+            continue
+        L.call("hb_ring_analysis", p.handle, 32, 1, m.data_ptr(), None, F[1:].data_ptr(), 0, st)
+        assert torch.equal(F[1:], want)
+        L.call("hb_ring_synthesis", p.handle, 32, 1, F[1:].data_ptr(), out.data_ptr(), 0, st)
+        assert torch.equal(out, ref)
